@@ -5,12 +5,14 @@
 // used at nelson/SolverCholeskySchur.hpp:136-140).  S is stored dense,
 // row-major, lower triangle, n padded to a multiple of NB = 128 (identity on
 // the padding).  Per 128-wide panel k:
-//   potrf_diag_kernel  factor of the diagonal tile and its inverse (one CTA)
-//   trsm_kernel        L_ik = A_ik L_kk^-T as a product with the inverse
+//   potrf_diag_kernel  factor of the diagonal tile (one CTA) and the inverses
+//                      of its 16 x 16 diagonal blocks
+//   trsm_kernel        L_ik = A_ik L_kk^-T by substitution with those
 //   syrk update        A_ij -= L_ik L_jk' on the trailing lower triangle
 //                      (tensor-core kernel in tc_syrk.cu for the mixed path,
 //                      cuBLAS DSYRK for the FP64 comparison path)
-// Solves use the tile inverses: trsv_fwd/bwd_kernel with a ticketed
+// After the last panel inv_tiles_kernel forms the inverses of all diagonal
+// tiles; solves use them: trsv_fwd/bwd_kernel with a ticketed
 // look-back between CTAs of one launch, each wait bounded.
 #pragma once
 
@@ -34,41 +36,49 @@ __device__ inline void chain_release() { asm volatile("griddepcontrol.launch_dep
 // One CTA: factor the NB x NB diagonal tile of panel k in the storage
 // precision T (FP64 for the FP64 path; FP32 for the mixed path, whose
 // trailing updates and off-diagonal solves are FP32-accurate as well and whose
-// factor only preconditions the FP64 refinement) and build its inverse, in
-// registers, as 32 super-steps of 4 columns.
+// factor only preconditions the FP64 refinement) and invert the 16 x 16 blocks
+// on its diagonal (all that the panel solves need; inv_tiles_kernel completes
+// the inverse of every tile at once, off the chain).
 //
-// Owner threads (528): thread t owns 4x4 block (R, C), C <= R, of the lower
-// triangle and one register block for it: A until block column C is factored,
-// afterwards B -> X = inv(L) (right-looking forward substitution of L X = I).
-// Pivot warp (warp 14): does all per-super-step work that is not a bulk update,
-// so that no owner warp runs it for one or two active lanes.  Super-step jb:
-//   (2) pivot warp, lane l < 31: for the row-jb block (jb, C = l) if l < jb,
-//       else for the column-jb block (R = l + 1, jb): out = M Di' with M the
-//       staged B' (row block: X_jb,C = out') or A (column block: L_R,jb =
-//       out); publishes L / X in shared memory and writes them to S / Linv.
-//   (3) owners with jb < R (except the next diagonal block) apply one rank-4
-//       update  t -= L_R,jb Q_jb,C  with Q = L_C,jb' while jb < C (A part) and
-//       Q = X_jb,C once jb >= C (X part) -- the same instructions for both --
-//       then stage their block in shared memory if it just became final:
-//       column-(jb+1) blocks (A), row-(jb+1) blocks (B'), diagonal block jb+2.
-//       Concurrently the pivot warp's lane jb, which holds L_jb+1,jb, factors
-//       the next diagonal block A_jb+1,jb+1 - L_jb+1,jb L_jb+1,jb' and inverts
-//       it (Di of super-step jb+1): the serial 4x4 factor overlaps the updates.
-// Warps are spread over the SM's four schedulers by index mod 4; the pivot
-// warp's scheduler carries three owner warps, the others four or five.
-// Shared 4x4 blocks are 20-word rows (16 used): lanes reading or writing
-// consecutive blocks with 16-byte vectors stay within the minimum wavefronts.
-// Two barriers per super-step.  L_kk is written to S and the blocks of
-// inv(L_kk) on and below the diagonal to Linv (its strictly upper blocks are
-// never written: the caller keeps them zero).
-constexpr int kPivotWarp = 14;
-constexpr int PT = 32 * 18;  // 17 owner warps (528 owners) + the pivot warp
-constexpr int kTiles4 = (NB / 4) * (NB / 4 + 1) / 2;  // 528
-constexpr int kBlk = 20;     // words per shared 4x4 block
-constexpr size_t kPotrfSmem = 0;
+// The tile is bound by its 128 dependent pivots, so the kernel is laid out
+// around that chain, in eight block columns of 16:
+//   pivot warp    the diagonal block, a lane holding one row of 16 columns in
+//       registers (lanes 16 .. 31 repeat lanes 0 .. 15).  With u = the unscaled
+//       column, d its pivot and r = 1 / d, an entry becomes a_c -= (a_j r) u_c.
+//       Every lane carries the next pivot itself (d' = v - u1 (u1 r), u1 and v
+//       fetched by shuffle while r is formed), so a column costs one reciprocal
+//       and a few FMAs of latency; the columns further right are updated one
+//       step late from the column published in shared memory.  It has its
+//       scheduler to itself.
+//   row warps     apply the published columns to the rows below, one per lane,
+//       8 columns at a time behind the pivot warp (named barriers), so the
+//       panel solve runs under the pivot chain; 16 rows of the identity beside
+//       them become the inverse of the diagonal block.
+//   helper warps  complete the block column under way (its last update, which
+//       the row warps wait for) and apply all but the last update to the next
+//       one: left-looking, so that the work is even over the block columns.
+// Between two block columns only the last update of the next diagonal block is
+// left on the chain.  Blocks of 16 keep the unrolled code of the roles that run
+// side by side within the instruction cache (blocks of 32 did not: about 3
+// cycles an instruction).  One tile after another on an idle B200: FP32 14.4 us
+// against 30.0 us, FP64 22.6 against 67.5, for 32 rank-4 super-steps that
+// formed the whole inverse as well (forming it here too: 20.5 and 28.7 us).
+constexpr int PB = 16;
+constexpr int kPBlocks = NB / PB;
+constexpr int kPotLd = NB + 4;     // row stride of `sm` (conflict-free rows and MMA operands)
+constexpr int kPotDld = PB + 4;    // of `dg`
+constexpr int kRowWarps = 4;
+constexpr int PT = 512, kHelpWarps = 8;
+// Warp roles: a scheduler serves the warps of equal index mod 4, and warps 4,
+// 8 and 12 stay off the pivot warp's.  0: pivot, 1 .. 4: row warps, 5 .. 12:
+// helpers, -1: none.
+__device__ __forceinline__ int potrf_role(int w) { return w == 0 ? 0 : (w & 3) == 0 ? -1 : w - (w >> 2); }
+template <typename T>
+constexpr size_t potrf_smem() {
+  return sizeof(T) * ((size_t)NB * (kPotLd + kPotDld) + PB * PB + 2 * PB);
+}
 
-// four consecutive elements (16-byte aligned for float, 32 for double; any
-// address space)
+// four consecutive elements (16-byte aligned; any address space)
 __device__ inline void store_row4(float* p, float a, float b, float c, float d) {
   *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
 }
@@ -84,349 +94,737 @@ __device__ inline void load_row4(const double* p, double v[4]) {
   const double2 x = reinterpret_cast<const double2*>(p)[0], y = reinterpret_cast<const double2*>(p)[1];
   v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
 }
-
-// 1 / sqrt of a pivot, clamped away from zero (a non-positive pivot is
-// flagged separately)
-__device__ inline float pivot_rsqrt(float d) { return rsqrtf(fmaxf(d, 1e-30f)); }
-__device__ inline double pivot_rsqrt(double d) { return rsqrt(fmax(d, 1e-300)); }
-
-// Factor the 4x4 SPD block a (lower part used) of diagonal block jb and invert
-// the factor: L to S (zeros above its diagonal), Di = inv(L) to the shared Di
-// (row-major 4x4) and X block (row i, column c at i * 4 + c) and to Linv.
-// Returns false on a non-positive pivot.
+// Shared memory by 32-bit shared-window address (a pointer picked at run time
+// between two shared arrays would be read through the generic path).
 template <typename T>
-__device__ inline bool factor_pivot_block(T a[4][4], int jb, T* __restrict__ S, size_t base, int ld,
-                                          T* __restrict__ Lout, T* Di, T* Xblk) {
-  bool fail = false;
-  T rs[4];
+struct Sh {
+  uint32_t a;
+  __device__ __forceinline__ Sh operator+(int i) const { return Sh{a + (uint32_t)(i * (int)sizeof(T))}; }
+};
+__device__ __forceinline__ void load_row4(Sh<float> p, float v[4]) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(p.a));
+}
+__device__ __forceinline__ void load_row4(Sh<double> p, double v[4]) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(p.a));
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[2]), "=d"(v[3]) : "r"(p.a + 16));
+}
+__device__ __forceinline__ void store_row4(Sh<float> p, float a, float b, float c, float d) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(p.a), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void store_row4(Sh<double> p, double a, double b, double c, double d) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(p.a), "d"(a), "d"(b) : "memory");
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(p.a + 16), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ void load_two(Sh<float> p, float& x, float& y) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(p.a));
+}
+__device__ __forceinline__ void load_two(Sh<double> p, double& x, double& y) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(p.a));
+}
+__device__ __forceinline__ void store_two(Sh<float> p, float x, float y) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(p.a), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ void store_two(Sh<double> p, double x, double y) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(p.a), "d"(x), "d"(y) : "memory");
+}
+__device__ __forceinline__ void store_one(Sh<float> p, float x) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(p.a), "f"(x) : "memory");
+}
+__device__ __forceinline__ void store_one(Sh<double> p, double x) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(p.a), "d"(x) : "memory");
+}
+__device__ __forceinline__ float load_one(Sh<float> p) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p.a));
+  return v;
+}
+__device__ __forceinline__ double load_one(Sh<double> p) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(p.a));
+  return v;
+}
+// 16-byte global -> shared copies that complete asynchronously: a kernel
+// issues all of its staging before one wait, so the staging costs one L2 /
+// HBM round trip however loaded the memory system is
+__device__ inline void cp_async16(uint32_t sa, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ inline void cp_async16(void* smem, const void* gmem) {
+  cp_async16((uint32_t)__cvta_generic_to_shared(smem), gmem);
+}
+__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ inline void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// 1 / d and 1 / sqrt(d) of a pivot, clamped away from zero (a non-positive
+// pivot is flagged separately)
+__device__ __forceinline__ void pivot_inv(float d, float& ri, float& rs) {
+  d = fmaxf(d, 1e-30f);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(d));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(d));
+}
+__device__ __forceinline__ void pivot_inv(double d, double& ri, double& rs) {
+  rs = rsqrt(fmax(d, 1e-300));
+  ri = rs * rs;
+}
+
+__device__ __forceinline__ void named_sync(int id, int n) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int n) {
+  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory");
+}
+
+// Eliminates the 16 x 16 block whose row lane % 16 is a[] (entries right of the
+// diagonal are ignored), leaving the row of L in a[] and publishing every
+// column in uc, (1 / d, 1 / sqrt(d)) in inv_s.  False on a non-positive pivot.
+template <typename T>
+__device__ __forceinline__ bool pivot_block(T (&a)[PB], Sh<T> uc, Sh<T> inv_s, int lane) {
+  bool ok = true;
+  T d = __shfl_sync(0xffffffffu, a[0], 0);
+  T up[PB];
+  T tp = (T)0;
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    T d = a[j][j];
-#pragma unroll
-    for (int l = 0; l < j; l++) d -= a[j][l] * a[j][l];
-    fail |= !(d > (T)0) || !isfinite(d);
-    rs[j] = pivot_rsqrt(d);
-    a[j][j] = d * rs[j];
-#pragma unroll
-    for (int i = j + 1; i < 4; i++) {
-      T v = a[i][j];
-#pragma unroll
-      for (int l = 0; l < j; l++) v -= a[i][l] * a[j][l];
-      a[i][j] = v * rs[j];
+  for (int j = 0; j < PB; j++) {
+    T ri, rs;
+    pivot_inv(d, ri, rs);
+    T u1 = (T)0, u2 = (T)0, v = (T)0;
+    if (j + 1 < PB) {
+      u1 = __shfl_sync(0xffffffffu, a[j], j + 1);
+      v = __shfl_sync(0xffffffffu, a[j + 1], j + 1);
     }
+    if (j + 2 < PB) u2 = __shfl_sync(0xffffffffu, a[j], j + 2);
+    if (lane < PB) store_one(uc + (j * PB + lane), a[j]);
+    ok &= d > (T)0 && isfinite(d);
+    // column j - 1 applied to the columns that its step left out
+    if (j > 0) {
+#pragma unroll
+      for (int c = j + 2; c < PB; c++) a[c] -= tp * up[c];
+    }
+    if (lane == 0) store_two(inv_s + 2 * j, ri, rs);
+    __syncwarp();
+#pragma unroll
+    for (int c = (j + 3) & ~3; c < PB; c += 4) {
+      T q[4];
+      load_row4(uc + (j * PB + c), q);
+#pragma unroll
+      for (int i = 0; i < 4; i++) up[c + i] = q[i];
+    }
+    const T t = a[j] * ri;
+    if (j + 1 < PB) {
+      d = v - u1 * (u1 * ri);
+      a[j + 1] -= t * u1;
+    }
+    if (j + 2 < PB) a[j + 2] -= t * u2;
+    a[j] *= rs;
+    tp = t;
+    if ((j & 7) == 7) named_arrive(1 + (j >> 3), 32 * (1 + kRowWarps));
   }
-  const int r0 = 4 * jb;
+  return ok;
+}
+
+// The same elimination for a row outside the pivot block.
+template <typename T>
+__device__ __forceinline__ void follow_block(T (&a)[PB], Sh<T> uc, Sh<T> inv_s) {
 #pragma unroll
-  for (int i = 0; i < 4; i++)
-    store_row4(S + base + (size_t)(r0 + i) * ld + r0, a[i][0], i >= 1 ? a[i][1] : (T)0, i >= 2 ? a[i][2] : (T)0,
-               i >= 3 ? a[i][3] : (T)0);
-  // inv(L) one column at a time: multiplications only (the rsqrt is 1 / L_ii)
-  T di[4][4];
+  for (int j = 0; j < PB; j++) {
+    if ((j & 7) == 0) named_sync(1 + (j >> 3), 32 * (1 + kRowWarps));
+    T ri, rs;
+    load_two(inv_s + 2 * j, ri, rs);
+    const T t = a[j] * ri;
 #pragma unroll
-  for (int c = 0; c < 4; c++)
+    for (int c = (j + 1) & ~3; c < PB; c += 4) {
+      T q[4];
+      load_row4(uc + (j * PB + c), q);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if (i < c) {
-        di[i][c] = (T)0;
-      } else if (i == c) {
-        di[i][c] = rs[i];
-      } else {
-        T v = (T)0;
+      for (int i = 0; i < 4; i++)
+        if (c + i > j) a[c + i] -= t * q[i];
+    }
+    a[j] *= rs;
+  }
+}
+
+// 16 x 8 piece of one warp: C -= P Q' over k in [k0, k1) (multiples of 16), P
+// and Q rows of `sm`.
+// FP32: lane (g, t) = (lane / 4, lane % 4) owns rows g, g + 8, columns 2 t, 2 t + 1
+__device__ __forceinline__ void help_block(Sh<float> C, Sh<float> P, Sh<float> Q, int k0, int k1, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  float acc[2][2] = {};
+  P = P + g * kPotLd;
+  Q = Q + 2 * t * kPotLd;
+#pragma unroll 1
+  for (int k = k0; k < k1; k += PB) {
 #pragma unroll
-        for (int l = c; l < i; l++) v -= a[i][l] * di[l][c];
-        di[i][c] = v * rs[i];
+    for (int kk = 0; kk < PB; kk += 4) {
+      float p[2][4], q[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        load_row4(P + (8 * i * kPotLd + k + kk), p[i]);
+        load_row4(Q + (i * kPotLd + k + kk), q[i]);
       }
-    }
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    store_row4(Di + 4 * i, di[i][0], di[i][1], di[i][2], di[i][3]);
-    store_row4(Xblk + 4 * i, di[i][0], di[i][1], di[i][2], di[i][3]);
-    store_row4(Lout + (size_t)(r0 + i) * NB + r0, di[i][0], di[i][1], di[i][2], di[i][3]);
+      for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int j = 0; j < 2; j++) acc[i][j] += p[i][m] * q[j][m];
+    }
   }
-  return !fail;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const Sh<float> c = C + ((g + 8 * i) * kPotLd + 2 * t);
+    float x, y;
+    load_two(c, x, y);
+    store_two(c, x - acc[i][0], y - acc[i][1]);
+  }
+}
+// FP64: mma.m8n8k4 (FP64 in and out, 1.6 times the rate of FMAs), lane = 4 g + t
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void help_block(Sh<double> C, Sh<double> P, Sh<double> Q, int k0, int k1, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  double acc[2][2][2] = {};
+  P = P + (g * kPotLd + t);
+  Q = Q + (g * kPotLd + t);
+#pragma unroll 1
+  for (int k = k0; k < k1; k += PB) {
+#pragma unroll
+    for (int kk = 0; kk < PB; kk += 4) {
+      const double b = load_one(Q + (k + kk));
+#pragma unroll
+      for (int i = 0; i < 2; i++) mma_f64(acc[(kk >> 2) & 1][i], load_one(P + (8 * i * kPotLd + k + kk)), b);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const Sh<double> c = C + ((g + 8 * i) * kPotLd + 2 * t);
+    double x, y;
+    load_two(c, x, y);
+    store_two(c, x - (acc[0][i][0] + acc[1][i][0]), y - (acc[0][i][1] + acc[1][i][1]));
+  }
+}
+
+// 8 x 8 piece of the next diagonal block: C -= P Q' over 16 columns
+__device__ __forceinline__ void diag_piece(Sh<float> C, Sh<float> P, Sh<float> Q, int lane) {
+  const int r = lane >> 2, c = 2 * (lane & 3);
+  float s0[2] = {0.f, 0.f}, s1[2] = {0.f, 0.f};
+#pragma unroll
+  for (int k = 0; k < PB; k += 4) {
+    float x[4], y[4], z[4];
+    load_row4(P + (r * kPotLd + k), x);
+    load_row4(Q + (c * kPotLd + k), y);
+    load_row4(Q + ((c + 1) * kPotLd + k), z);
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      s0[m & 1] += x[m] * y[m];
+      s1[m & 1] += x[m] * z[m];
+    }
+  }
+  const Sh<float> o = C + (r * kPotLd + c);
+  float x, y;
+  load_two(o, x, y);
+  store_two(o, x - (s0[0] + s0[1]), y - (s1[0] + s1[1]));
+}
+__device__ __forceinline__ void diag_piece(Sh<double> C, Sh<double> P, Sh<double> Q, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  double acc[2] = {0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < PB; k += 4) mma_f64(acc, load_one(P + (g * kPotLd + k + t)), load_one(Q + (g * kPotLd + k + t)));
+  const Sh<double> c = C + (g * kPotLd + 2 * t);
+  double x, y;
+  load_two(c, x, y);
+  store_two(c, x - acc[0], y - acc[1]);
+}
+
+// Block column p of L (rows 16 p .., zeros above the diagonal) to the tile, and
+// the inverse of its diagonal block (transposed rows in dg) to X.  Threads id, id + n, ...
+template <typename T>
+__device__ __forceinline__ void potrf_write(Sh<T> sm, Sh<T> dg, int p, T* __restrict__ A, int ld, T* __restrict__ X,
+                                            int id, int n) {
+  const int nl = (NB - p * PB) * 4;
+#pragma unroll 1
+  for (int e = id; e < nl; e += n) {
+    const int r = p * PB + (e >> 2), c = p * PB + 4 * (e & 3);
+    T v[4];
+    load_row4(sm + (r * kPotLd + c), v);
+    store_row4(A + (size_t)r * ld + c, v[0], v[1], v[2], v[3]);
+  }
+  if (id < PB) {  // 4 x 4 pieces
+    const int b = 4 * (id & 3), c = 4 * (id >> 2);
+    T v[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) load_row4(dg + ((p * PB + b + q) * kPotDld + c), v[q]);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      store_row4(X + (size_t)(p * PB + c + q) * NB + p * PB + b, v[0][q], v[1][q], v[2][q], v[3][q]);
+  }
 }
 
 template <typename T>
-static __global__ void __launch_bounds__(PT) potrf_diag_kernel(T* __restrict__ S, int ld, int k,
+__device__ __forceinline__ void load_row16(Sh<T> p, T (&a)[PB]) {
+#pragma unroll
+  for (int c = 0; c < PB; c += 4) {
+    T q[4];
+    load_row4(p + c, q);
+#pragma unroll
+    for (int i = 0; i < 4; i++) a[c + i] = q[i];
+  }
+}
+template <typename T>
+__device__ __forceinline__ void store_row16(Sh<T> p, const T (&a)[PB]) {
+#pragma unroll
+  for (int c = 0; c < PB; c += 4) store_row4(p + c, a[c], a[c + 1], a[c + 2], a[c + 3]);
+}
+
+template <typename T>
+static __global__ void __launch_bounds__(PT, 1) potrf_diag_kernel(T* __restrict__ S, int ld, int k,
                                                                T* __restrict__ Linv, int* __restrict__ status,
                                                                const int* __restrict__ active) {
-  // Published blocks of super-step jb (double-buffered): L_R,jb at Lc[.][R]
-  // (row u, column w at w * 4 + u) and X_jb,C at Xr[.][C] (row w, column v at
-  // w * 4 + v), so that rank-4 step w reads 4 consecutive words of each.
-  // Staged blocks M at Mst[slot] (row u, column w at u * 4 + w; row block C:
-  // slot C, holding B'; column block R: slot R - 1, holding A); staged
-  // diagonal blocks by parity.
-  __shared__ __align__(16) T Lc[2][NB / 4][kBlk];
-  __shared__ __align__(16) T Xr[2][NB / 4][kBlk];
-  __shared__ __align__(16) T Mst[NB / 4][kBlk];
-  __shared__ __align__(16) T Di[2][16];  // inv(L_jb,jb), row-major
-  __shared__ T Dst[2][4][4];
-  __shared__ int bad;
+  constexpr int EPV = 16 / (int)sizeof(T);
+  extern __shared__ float4 smf4[];
+  const Sh<T> sm{(uint32_t)__cvta_generic_to_shared(smf4)};  // L on and below the diagonal 16-blocks
+  const Sh<T> dg = sm + NB * kPotLd;     // inverses of the diagonal blocks, transposed
+  const Sh<T> uc = dg + NB * kPotDld;    // published columns of the pivot block
+  const Sh<T> inv_s = uc + PB * PB;    // (1 / d, 1 / sqrt(d)) per column
   chain_release();
   chain_wait();
   if (active && !*active) return;
-  const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
-  const bool pivot = wi == kPivotWarp;
-  const int oid = wi < kPivotWarp ? tid : tid - 32;  // owner index
-  const size_t base = (size_t)k * NB * ld + (size_t)k * NB;
-  T* Lout = Linv + (size_t)k * NB * NB;
-  if (tid == 0) bad = 0;
-  int R = 0, C = 0;
-  const bool own = !pivot && oid < kTiles4;
-  if (own) {
-    R = (int)((sqrtf(8.0f * oid + 1.0f) - 1.0f) * 0.5f);
-    while ((R + 1) * (R + 2) / 2 <= oid) R++;
-    while (R * (R + 1) / 2 > oid) R--;
-    C = oid - R * (R + 1) / 2;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, role = potrf_role(w);
+  T* A = S + (size_t)k * NB * ld + (size_t)k * NB;
+  T* X = Linv + (size_t)k * NB * NB;
+  // the lower 16-blocks of the tile
+#pragma unroll 4
+  for (int e = tid; e < NB * (NB / EPV); e += PT) {
+    const int r = e / (NB / EPV), c = EPV * (e % (NB / EPV));
+    if (c <= (r | (PB - 1))) cp_async16((sm + (r * kPotLd + c)).a, A + (size_t)r * ld + c);
   }
-  const int r0 = 4 * R, c0 = 4 * C;
-  T t[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; u++)
-#pragma unroll
-    for (int v = 0; v < 4; v++)
-      t[u][v] = (own && c0 + v <= r0 + u) ? S[base + (size_t)(r0 + u) * ld + c0 + v] : (T)0;
-  // stage column 0 and the first two diagonal blocks
-  if (own && C == 0 && R > 0) {
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      store_row4(&Mst[R - 1][4 * u], t[u][0], t[u][1], t[u][2], t[u][3]);
-#pragma unroll
-      for (int w = 0; w < 4; w++) t[u][w] = (T)0;
-    }
-  } else if (own && R == C && R <= 1) {
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) Dst[R][u][v] = t[u][v];
-  }
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
-  if (pivot && lane == 0) {
-    T a[4][4];
+#pragma unroll 1
+  for (int kb = 0; kb < kPBlocks; kb++) {
+    if (role == 0) {
+      const Sh<T> row = sm + ((kb * PB + (lane & (PB - 1))) * kPotLd + kb * PB);
+      T a[PB];
+      load_row16(row, a);
+      if (!pivot_block(a, uc, inv_s, lane) && lane == 0) atomicOr(status, ST_CHOL_FAIL);
+      if (lane < PB) {
 #pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) a[u][v] = Dst[0][u][v];
-    if (!factor_pivot_block(a, 0, S, base, ld, Lout, Di[0], Xr[0][0])) bad = 1;
-  }
-  __syncthreads();
-  T out[4][4];  // pivot warp: this super-step's L (or X') block
-  for (int jb = 0; jb < NB / 4; jb++) {
-    const int buf = jb & 1;
-    // (2) the row-jb and column-jb blocks, one per pivot-warp lane
-    if (pivot && lane < NB / 4 - 1) {
-      T m[4][4], d[4][4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        load_row4(&Mst[lane][4 * u], m[u]);
-        load_row4(&Di[buf][4 * u], d[u]);
+        for (int c = 0; c < PB; c++)
+          if (c > lane) a[c] = (T)0;
+        store_row16(row, a);
       }
+    } else if (role > 0 && role <= kRowWarps) {
+      // A row r below block kb, a row of the identity in it
+      const int r = 32 * (role - 1) + lane;
+      const bool unit = r / PB == kb;
+      if (kb > 0) named_sync(3, 32 * (kHelpWarps + kRowWarps));
+      T a[PB];
+      load_row16(sm + (r * kPotLd + kb * PB), a);
 #pragma unroll
-      for (int u = 0; u < 4; u++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-          T s = (T)0;
-#pragma unroll
-          for (int w = 0; w <= v; w++) s += m[u][w] * d[v][w];
-          out[u][v] = s;
-        }
-      const bool rowb = lane < jb;
-      const int idx = rowb ? lane : lane + 1;  // C of a row block, R of a column block
-      // L_R,jb[u][v] at v * 4 + u; X_jb,C[v][u] = out[u][v] at v * 4 + u
-      T* pub = rowb ? Xr[buf][idx] : Lc[buf][idx];
-#pragma unroll
-      for (int v = 0; v < 4; v++) store_row4(pub + 4 * v, out[0][v], out[1][v], out[2][v], out[3][v]);
-      if (rowb) {
-        // X_jb,C = out': row v of X is column v of out
-#pragma unroll
-        for (int v = 0; v < 4; v++)
-          store_row4(Lout + (size_t)(4 * jb + v) * NB + 4 * idx, out[0][v], out[1][v], out[2][v], out[3][v]);
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-          store_row4(S + base + (size_t)(4 * idx + u) * ld + 4 * jb, out[u][0], out[u][1], out[u][2], out[u][3]);
+      for (int c = 0; c < PB; c++)
+        if (unit) a[c] = c == (r & (PB - 1)) ? (T)1 : (T)0;
+      follow_block(a, uc, inv_s);
+      if (r / PB >= kb) store_row16(unit ? dg + r * kPotDld : sm + (r * kPotLd + kb * PB), a);
+    } else if (role > 0 && kb > 0) {
+      // 16 x 8 pieces: block column kb with block column kb - 1 (rows below its
+      // diagonal block, which is done), then block column kb + 1 with 0 .. kb - 1
+      const int hw = role - 1 - kRowWarps, n = 2 * (kPBlocks - 1 - kb);
+#pragma unroll 1
+      for (int u = hw; u < n; u += kHelpWarps) {
+        const int r = (kb + 1 + (u >> 1)) * PB, c = kb * PB + 8 * (u & 1);
+        help_block(sm + (r * kPotLd + c), sm + r * kPotLd, sm + c * kPotLd, (kb - 1) * PB, kb * PB, lane);
       }
+      named_arrive(3, 32 * (kHelpWarps + kRowWarps));
+      // the warps without a piece above first
+#pragma unroll 1
+      for (int u = (hw + kHelpWarps - n % kHelpWarps) % kHelpWarps; u < n; u += kHelpWarps) {
+        const int r = (kb + 1 + (u >> 1)) * PB, c = (kb + 1) * PB + 8 * (u & 1);
+        help_block(sm + (r * kPotLd + c), sm + r * kPotLd, sm + c * kPotLd, 0, kb * PB, lane);
+      }
+      potrf_write(sm, dg, kb - 1, A, ld, X, hw * 32 + lane, 32 * kHelpWarps);
     }
     __syncthreads();
-    // (3) one rank-4 update per block below row jb, then staging; the next
-    //     step writes the other buffers, so no barrier here
-    if (own && jb < R && !(R == C && R == jb + 1)) {
-      const T* q = (jb < C) ? Lc[buf][C] : Xr[buf][C];  // Q_jb,C row w at 4 w either way
-#pragma unroll
-      for (int w = 0; w < 4; w++) {
-        T pr[4], qc[4];
-        load_row4(&Lc[buf][R][4 * w], pr);
-        load_row4(q + 4 * w, qc);
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-          for (int v = 0; v < 4; v++) t[u][v] -= pr[u] * qc[v];
+    if (kb + 1 < kPBlocks) {
+      // the next diagonal block, 8 x 8 pieces on and below the diagonal
+      if (w < 3) {
+        const int i = w > 0, j = w > 1, b = (kb + 1) * PB;
+        diag_piece(sm + ((b + 8 * i) * kPotLd + b + 8 * j), sm + ((b + 8 * i) * kPotLd + kb * PB),
+                   sm + ((b + 8 * j) * kPotLd + kb * PB), lane);
       }
-      if (C == jb + 1 && R > jb + 1) {  // A_R,jb+1 is final
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          store_row4(&Mst[R - 1][4 * u], t[u][0], t[u][1], t[u][2], t[u][3]);
-#pragma unroll
-          for (int w = 0; w < 4; w++) t[u][w] = (T)0;  // the X block starts from zero below the diagonal
-        }
-      } else if (R == jb + 1) {  // B_jb+1,C is final (C <= jb): stage B'
-#pragma unroll
-        for (int u = 0; u < 4; u++) store_row4(&Mst[C][4 * u], t[0][u], t[1][u], t[2][u], t[3][u]);
-      } else if (R == C && R == jb + 2) {  // all but the last update of A_jb+2,jb+2
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-          for (int v = 0; v < 4; v++) Dst[R & 1][u][v] = t[u][v];
-      }
+      __syncthreads();
     }
-    // look-ahead: the next diagonal block, from its staged value and the
-    // L_jb+1,jb held by lane jb
-    if (pivot && lane == jb && jb + 1 < NB / 4) {
-      const int nb = jb + 1;
-      T a[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int c = 0; c <= i; c++) {
-          T v = Dst[nb & 1][i][c];
-#pragma unroll
-          for (int w = 0; w < 4; w++) v -= out[i][w] * out[c][w];
-          a[i][c] = v;
-        }
-      if (!factor_pivot_block(a, nb, S, base, ld, Lout, Di[nb & 1], Xr[nb & 1][nb])) bad = 1;
-    }
-    __syncthreads();
   }
-  if (tid == 0 && bad) atomicOr(status, ST_CHOL_FAIL);
+  potrf_write(sm, dg, kPBlocks - 1, A, ld, X, tid, PT);
 }
 
 // ---------------------------------------------------------------------------
-// L_ik = A_ik inv(L_kk)' for 64-row slabs of rows [row_begin, row_begin +
-// nrows) below the diagonal tile (absolute row indices), as a
-// register-tiled product: X (64 x 128) = A (64 x 128) Linv' (128 x 128).
-// 256 threads, thread (ty, tx) computes rows ty*4 .. ty*4+3 (ty < 16) and
-// columns tx + 16 j (tx < 16, j < 8); A and Linv are staged in shared memory
-// in the working precision, K-major, and read as broadcasts / strided rows.
-constexpr int TRSM_ROWS = 64;
-template <typename T>
+// Panel solve L_ik = A_ik inv(L_kk)' for rows [row_begin, row_begin + nrows)
+// below the diagonal tile (absolute row indices), by substitution over the
+// eight block columns of 16 with the inverses of L_kk's diagonal blocks: half
+// the products of a multiplication by the whole inverse, and nothing waits for
+// that one.  A CTA owns 16 RT rows; thread (ty, tx) holds rows ty RT .. of
+// columns tx + 16 j, so a row lives in half a warp and the substitution needs
+// no CTA barrier.  Step kb: y = t inv(L_kb,kb)' through shared memory, then
+// the columns to the right (kept one block nearer in every step, so that the
+// loop body is the same code) lose y L_j,kb'.
+// RT = 1 while that leaves SMs idle; more rows a thread share L_kk's reads.
+// 96 CTAs beside the chain: 8.0 us against 15.5 us for the product with the
+// whole inverse by 64-row CTAs.
+constexpr int kTrLd = NB + 4, kTrXld = PB + 4;
+template <typename T, int RT>
 constexpr size_t trsm_smem() {
-  return sizeof(T) * ((size_t)NB * (NB + 1) + (size_t)NB * (TRSM_ROWS + 1));
+  return sizeof(T) * ((size_t)NB * (kTrLd + kTrXld) + (size_t)16 * RT * (kTrLd + kTrXld));
 }
 
-template <typename T>
+template <typename T, int RT>
 static __global__ void __launch_bounds__(256) trsm_kernel(T* __restrict__ S, int ld, int k, int row_begin, int nrows,
                                                           const T* __restrict__ Linv,
                                                           uint8_t* __restrict__ pack,
                                                           const int* __restrict__ active) {
-  extern __shared__ unsigned char smraw[];
-  T* sL = reinterpret_cast<T*>(smraw);      // sL[l][j] = Linv[j][l], (NB + 1) stride
-  T* sA = sL + NB * (NB + 1);               // sA[l][r] = A[r][l], (TRSM_ROWS + 1) stride
+  constexpr int ROWS = 16 * RT, EPV = 16 / (int)sizeof(T);
+  extern __shared__ float4 smf4[];
+  const Sh<T> sl{(uint32_t)__cvta_generic_to_shared(smf4)};  // L_kk, lower 16-blocks
+  const Sh<T> sx = sl + NB * kTrLd;                          // inverses of its diagonal blocks
+  const Sh<T> sy = sx + NB * kTrXld;                         // rows: A, then L
+  const Sh<T> st = sy + ROWS * kTrLd;                        // t of one step
+  chain_release();
+  chain_wait();
   if (active && !*active) return;
   const int tid = threadIdx.x;
-  const int r0 = row_begin + blockIdx.x * TRSM_ROWS;
-  const int nr = min(TRSM_ROWS, row_begin + nrows - r0);
+  const int r0 = row_begin + blockIdx.x * ROWS;
+  const int nr = min(ROWS, row_begin + nrows - r0);
   if (nr <= 0) return;
-  // staging: 16 independent loads in flight per thread before the stores
-  const T* Li = Linv + (size_t)k * NB * NB;
-#pragma unroll 1
-  for (int i0 = tid; i0 < NB * NB; i0 += 256 * 16) {
-    T v[16];
-#pragma unroll
-    for (int u = 0; u < 16; u++) v[u] = __ldg(Li + i0 + 256 * u);
-#pragma unroll
-    for (int u = 0; u < 16; u++) {
-      const int i = i0 + 256 * u, j = i / NB, l = i - j * NB;
-      sL[l * (NB + 1) + j] = v[u];
-    }
+  const T* D = S + (size_t)k * NB * ld + (size_t)k * NB;
+  const T* X = Linv + (size_t)k * NB * NB;
+  T* A = S + (size_t)r0 * ld + (size_t)k * NB;
+#pragma unroll 4
+  for (int e = tid; e < NB * (NB / EPV); e += 256) {
+    const int r = e / (NB / EPV), c = EPV * (e % (NB / EPV));
+    if (c < (r & ~(PB - 1)))
+      cp_async16((sl + (r * kTrLd + c)).a, D + (size_t)r * ld + c);
+    else if (c <= (r | (PB - 1)))
+      cp_async16((sx + (r * kTrXld + (c & (PB - 1)))).a, X + (size_t)r * NB + c);
   }
-#pragma unroll 1
-  for (int i0 = tid; i0 < TRSM_ROWS * NB; i0 += 256 * 16) {
-    T v[16];
+#pragma unroll 4
+  for (int e = tid; e < nr * (NB / EPV); e += 256) {
+    const int r = e / (NB / EPV), c = EPV * (e % (NB / EPV));
+    cp_async16((sy + (r * kTrLd + c)).a, A + (size_t)r * ld + c);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  const Sh<T> y = sy + ty * RT * kTrLd, t = st + ty * RT * kTrXld;
+  T acc[RT][kPBlocks];
 #pragma unroll
-    for (int u = 0; u < 16; u++) {
-      const int i = i0 + 256 * u, r = i / NB, l = i - r * NB;
-      v[u] = r < nr ? S[(size_t)(r0 + r) * ld + (size_t)k * NB + l] : (T)0;
+  for (int r = 0; r < RT; r++)
+#pragma unroll
+    for (int j = 0; j < kPBlocks; j++) acc[r][j] = load_one(y + (r * kTrLd + tx + PB * j));
+#pragma unroll 1
+  for (int kb = 0; kb < kPBlocks; kb++) {
+#pragma unroll
+    for (int r = 0; r < RT; r++) store_one(t + (r * kTrXld + tx), acc[r][0]);
+    __syncwarp();
+    T v[RT];
+#pragma unroll
+    for (int r = 0; r < RT; r++) v[r] = (T)0;
+#pragma unroll
+    for (int c = 0; c < PB; c += 4) {
+      T x[4];
+      load_row4(sx + ((kb * PB + tx) * kTrXld + c), x);
+#pragma unroll
+      for (int r = 0; r < RT; r++) {
+        T q[4];
+        load_row4(t + (r * kTrXld + c), q);
+#pragma unroll
+        for (int m = 0; m < 4; m++) v[r] += q[m] * x[m];
+      }
     }
 #pragma unroll
-    for (int u = 0; u < 16; u++) {
-      const int i = i0 + 256 * u, r = i / NB, l = i - r * NB;
-      sA[l * (TRSM_ROWS + 1) + r] = v[u];
+    for (int r = 0; r < RT; r++) store_one(y + (r * kTrLd + kb * PB + tx), v[r]);
+    __syncwarp();
+    T q[RT][PB];
+#pragma unroll
+    for (int r = 0; r < RT; r++)
+#pragma unroll
+      for (int c = 0; c < PB; c += 4) {
+        T w[4];
+        load_row4(y + (r * kTrLd + kb * PB + c), w);
+#pragma unroll
+        for (int m = 0; m < 4; m++) q[r][c + m] = w[m];
+      }
+#pragma unroll
+    for (int j = 0; j + 1 < kPBlocks; j++) {
+      if (kb + 1 + j < kPBlocks) {
+        const Sh<T> l = sl + (((kb + 1 + j) * PB + tx) * kTrLd + kb * PB);
+        T s[RT];
+#pragma unroll
+        for (int r = 0; r < RT; r++) s[r] = (T)0;
+#pragma unroll
+        for (int c = 0; c < PB; c += 4) {
+          T w[4];
+          load_row4(l + c, w);
+#pragma unroll
+          for (int r = 0; r < RT; r++)
+#pragma unroll
+            for (int m = 0; m < 4; m++) s[r] += q[r][c + m] * w[m];
+        }
+#pragma unroll
+        for (int r = 0; r < RT; r++) acc[r][j] = acc[r][j + 1] - s[r];
+      }
     }
   }
   __syncthreads();
-  const int ty = tid >> 4, tx = tid & 15;
-  T acc[4][8];
-#pragma unroll
-  for (int u = 0; u < 4; u++)
-#pragma unroll
-    for (int v = 0; v < 8; v++) acc[u][v] = (T)0;
-#pragma unroll 4
-  for (int l = 0; l < NB; l++) {
-    T a[4], b[8];
-#pragma unroll
-    for (int u = 0; u < 4; u++) a[u] = sA[l * (TRSM_ROWS + 1) + ty * 4 + u];
-#pragma unroll
-    for (int v = 0; v < 8; v++) b[v] = sL[l * (NB + 1) + tx + 16 * v];
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int v = 0; v < 8; v++) acc[u][v] += a[u] * b[v];
-  }
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    const int rr = ty * 4 + u;
-    if (rr < nr) {
-#pragma unroll
-      for (int v = 0; v < 8; v++) S[(size_t)(r0 + rr) * ld + (size_t)k * NB + tx + 16 * v] = acc[u][v];
-    }
+#pragma unroll 2
+  for (int e = tid; e < nr * (NB / 4); e += 256) {
+    const int r = e / (NB / 4), c = 4 * (e % (NB / 4));
+    T v[4];
+    load_row4(sy + (r * kTrLd + c), v);
+    store_row4(A + (size_t)r * ld + c, v[0], v[1], v[2], v[3]);
   }
   if (sizeof(T) == 4 && pack) {
-    // BF16 hi/lo pack of this slab for the tensor-core update: stage it
-    // row-major over the operand buffer (64 x 130 floats fit in sA), then
-    // each item is 8 consecutive columns of one row
-    constexpr int kSt = NB + 2;
-    static_assert(TRSM_ROWS * kSt <= NB * (TRSM_ROWS + 1), "staging fits the operand buffer");
-    float* st = reinterpret_cast<float*>(sA);
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int v = 0; v < 8; v++) st[(ty * 4 + u) * kSt + tx + 16 * v] = (float)acc[u][v];
-    __syncthreads();
+    // BF16 hi/lo pack of the rows for the tensor-core update, 8 consecutive columns per item
     const int rel0 = r0 - (k + 1) * NB;  // pack rows start below the diagonal tile
-    for (int i = tid; i < TRSM_ROWS * 16; i += 256) {
+    for (int i = tid; i < nr * 16; i += 256) {
       const int rr = i >> 4, h = i & 15;
-      if (rr >= nr) continue;
       float x[8];
 #pragma unroll
-      for (int q = 0; q < 8; q++) x[q] = st[rr * kSt + 8 * h + q];
+      for (int q = 0; q < 8; q += 4) {
+        T v[4];
+        load_row4(sy + (rr * kTrLd + 8 * h + q), v);
+#pragma unroll
+        for (int m = 0; m < 4; m++) x[q + m] = (float)v[m];
+      }
       tc_pack_store8(pack, tc_pack_offset(rel0 + rr, h), x);
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Critical-path kernels of the tensor-core schedule (FP32).  Each runs as
-// 128 / RPC CTAs of 256 threads, CTA c owning an RPC-row slice of one
-// 128 x 128 tile (RPC = kChainRows below):
-//   trsm_tile_kernel    L_(j+1),j = A_(j+1),j inv(L_jj)' for row tile j+1 of
-//                       panel j, and its BF16 pack
-//   diag_update_kernel  A_tt -= sum_p L_t,p L_t,p' on diagonal tile t over
-//                       panels p in [p0, p0 + np)
-// Thread (w, lane) of an RPC x 128 slice computes RPC / 2 row pairs (the
-// lane's pair lane / CG, CG = 64 / RPC) and columns 16 w + lane % CG + CG m
-// (m < 16 / CG).  Both operands stay row-major in shared memory (row stride
+// The same substitution for the row tile below panel j's diagonal tile, on the
+// factorisation's critical path, as 32 CTAs of 4 rows: a row's 8 blocks are
+// spread over four half-warps (half-warp group g holds blocks g and g + 4), so
+// a step is one 16 x 16 product in the group that owns block kb, one barrier
+// and at most two products in every other group.  Writes the rows and their
+// BF16 pack.  6.0 us (8 CTAs of 16 rows through trsm_kernel: 8.0 us); what it
+// adds to the 4 us of a product with the whole inverse is less than the
+// diagonal factor saves by not forming that.
+constexpr int kChainTrsmRows = 4;
+template <typename T>
+constexpr size_t trsm_tile_smem() {
+  return sizeof(T) * ((size_t)NB * (kTrLd + kTrXld) + kChainTrsmRows * (kTrLd + kTrXld));
+}
+template <typename T>
+static __global__ void __launch_bounds__(256) trsm_tile_kernel(T* __restrict__ S, int ld, int j,
+                                                               const T* __restrict__ Linv,
+                                                               uint8_t* __restrict__ pack,
+                                                               const int* __restrict__ active) {
+  constexpr int EPV = 16 / (int)sizeof(T), ROWS = kChainTrsmRows;
+  extern __shared__ float4 smf4[];
+  const Sh<T> sl{(uint32_t)__cvta_generic_to_shared(smf4)};  // L_jj, lower 16-blocks
+  const Sh<T> sx = sl + NB * kTrLd;                          // inverses of its diagonal blocks
+  const Sh<T> sy = sx + NB * kTrXld;                         // rows: A, then L
+  const Sh<T> st = sy + ROWS * kTrLd;
+  chain_release();
+  chain_wait();
+  if (active && !*active) return;
+  const int tid = threadIdx.x, rel0 = blockIdx.x * ROWS;
+  const T* D = S + (size_t)j * NB * ld + (size_t)j * NB;
+  const T* X = Linv + (size_t)j * NB * NB;
+  T* A = S + (size_t)((j + 1) * NB + rel0) * ld + (size_t)j * NB;
+  for (int e = tid; e < ROWS * (NB / EPV); e += 256) {
+    const int r = e / (NB / EPV), c = EPV * (e % (NB / EPV));
+    cp_async16((sy + (r * kTrLd + c)).a, A + (size_t)r * ld + c);
+  }
+#pragma unroll 4
+  for (int e = tid; e < NB * (NB / EPV); e += 256) {
+    const int r = e / (NB / EPV), c = EPV * (e % (NB / EPV));
+    if (c < (r & ~(PB - 1)))
+      cp_async16((sl + (r * kTrLd + c)).a, D + (size_t)r * ld + c);
+    else if (c <= (r | (PB - 1)))
+      cp_async16((sx + (r * kTrXld + (c & (PB - 1)))).a, X + (size_t)r * NB + c);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  // warp w: row w / 2; half-warp (w & 1, lane / 16) is group g
+  const int tx = tid & 15, g = (tid >> 4) & 3, row = tid >> 6;
+  const Sh<T> y = sy + row * kTrLd, t = st + row * kTrXld;
+  T acc[2] = {load_one(y + (g * PB + tx)), load_one(y + ((g + 4) * PB + tx))};
+#pragma unroll
+  for (int kb = 0; kb < kPBlocks; kb++) {
+    if (g == (kb & 3)) {
+      store_one(t + tx, acc[kb >> 2]);
+      __syncwarp(0xffffu << (tid & 16));
+      T v[4] = {(T)0, (T)0, (T)0, (T)0};
+#pragma unroll
+      for (int c = 0; c < PB; c += 4) {
+        T x[4], q[4];
+        load_row4(sx + ((kb * PB + tx) * kTrXld + c), x);
+        load_row4(t + c, q);
+#pragma unroll
+        for (int m = 0; m < 4; m++) v[m] += q[m] * x[m];
+      }
+      store_one(y + (kb * PB + tx), (v[0] + v[1]) + (v[2] + v[3]));
+    }
+    __syncthreads();
+    T q[PB];
+    if (kb + 1 < kPBlocks) load_row16(y + kb * PB, q);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int b = g + 4 * h;
+      if (b > kb) {
+        const Sh<T> l = sl + ((b * PB + tx) * kTrLd + kb * PB);
+        T v[4] = {(T)0, (T)0, (T)0, (T)0};
+#pragma unroll
+        for (int c = 0; c < PB; c += 4) {
+          T w[4];
+          load_row4(l + c, w);
+#pragma unroll
+          for (int m = 0; m < 4; m++) v[m] += q[c + m] * w[m];
+        }
+        acc[h] -= (v[0] + v[1]) + (v[2] + v[3]);
+      }
+    }
+  }
+  for (int e = tid; e < ROWS * (NB / 4); e += 256) {
+    const int r = e / (NB / 4), c = 4 * (e % (NB / 4));
+    T v[4];
+    load_row4(sy + (r * kTrLd + c), v);
+    store_row4(A + (size_t)r * ld + c, v[0], v[1], v[2], v[3]);
+  }
+  if (sizeof(T) == 4 && pack) {
+    for (int e = tid; e < ROWS * 16; e += 256) {
+      const int r = e >> 4, h = e & 15;
+      float x[8];
+#pragma unroll
+      for (int q = 0; q < 8; q += 4) {
+        T v[4];
+        load_row4(sy + (r * kTrLd + 8 * h + q), v);
+#pragma unroll
+        for (int m = 0; m < 4; m++) x[q + m] = (float)v[m];
+      }
+      tc_pack_store8(pack, tc_pack_offset(rel0 + r, h), x);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The inverse of every diagonal tile from the inverses of its diagonal
+// 16-blocks (one CTA per tile, once per factorisation): X_ij = -X_ii sum_k
+// L_ik X_kj for i > j.  Columns are independent: warp w owns 8 of them, from
+// block column j = w / 2 on, and walks down the rows with L and its part of X
+// in shared memory as packed lower 16-blocks.  The blocks of Linv above the
+// diagonal are never written.  Bound by the chain of up to seven block rows:
+// FP64 11.7 us (34.6 us with L read from global memory and FMAs).
+constexpr int kInvBlk = PB * (PB + 4);
+__device__ __forceinline__ int inv_blk(int i, int j) { return (i * (i + 1) / 2 + j) * kInvBlk; }
+template <typename T>
+constexpr size_t inv_tiles_smem() {
+  return sizeof(T) * (size_t)(2 * (kPBlocks * (kPBlocks + 1) / 2) * kInvBlk + 16 * PB * (8 + 4));
+}
+// 16 x 8 product of one warp: C (row stride 12) = A B, A 16 x 16 (row stride 20),
+// B 16 x 8 (row stride ldb), added to acc; out() stores it
+__device__ __forceinline__ void inv_mac(float (&acc)[4], Sh<float> A, Sh<float> B, int ldb, int lane) {
+  const int row = lane >> 1, col = 4 * (lane & 1);
+#pragma unroll
+  for (int c = 0; c < PB; c += 4) {
+    float l[4];
+    load_row4(A + (row * (PB + 4) + c), l);
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      float x[4];
+      load_row4(B + ((c + m) * ldb + col), x);
+#pragma unroll
+      for (int q = 0; q < 4; q++) acc[q] += l[m] * x[q];
+    }
+  }
+}
+__device__ __forceinline__ void inv_out(const float (&acc)[4], float sign, Sh<float> C, int ldc, int lane) {
+  store_row4(C + ((lane >> 1) * ldc + 4 * (lane & 1)), sign * acc[0], sign * acc[1], sign * acc[2], sign * acc[3]);
+}
+// FP64 on mma.m8n8k4: acc = rows (g, g + 8), columns (2 t, 2 t + 1)
+__device__ __forceinline__ void inv_mac(double (&acc)[4], Sh<double> A, Sh<double> B, int ldb, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  double c0[2] = {acc[0], acc[1]}, c1[2] = {acc[2], acc[3]};
+#pragma unroll
+  for (int c = 0; c < PB; c += 4) {
+    const double b = load_one(B + ((c + t) * ldb + g));
+    mma_f64(c0, load_one(A + (g * (PB + 4) + c + t)), b);
+    mma_f64(c1, load_one(A + ((g + 8) * (PB + 4) + c + t)), b);
+  }
+  acc[0] = c0[0]; acc[1] = c0[1]; acc[2] = c1[0]; acc[3] = c1[1];
+}
+__device__ __forceinline__ void inv_out(const double (&acc)[4], double sign, Sh<double> C, int ldc, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  store_two(C + (g * ldc + 2 * t), sign * acc[0], sign * acc[1]);
+  store_two(C + ((g + 8) * ldc + 2 * t), sign * acc[2], sign * acc[3]);
+}
+template <typename T>
+static __global__ void __launch_bounds__(512) inv_tiles_kernel(const T* __restrict__ S, int ld, T* __restrict__ Linv,
+                                                              const int* __restrict__ active) {
+  constexpr int EPV = 16 / (int)sizeof(T);
+  extern __shared__ float4 smf4[];
+  const Sh<T> sl{(uint32_t)__cvta_generic_to_shared(smf4)};
+  const Sh<T> sx = sl + kPBlocks * (kPBlocks + 1) / 2 * kInvBlk;
+  if (active && !*active) return;
+  const int k = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const Sh<T> st = sx + (kPBlocks * (kPBlocks + 1) / 2 * kInvBlk + w * PB * 12);
+  const T* L = S + (size_t)k * NB * ld + (size_t)k * NB;
+  T* X = Linv + (size_t)k * NB * NB;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < NB * (NB / EPV); e += 512) {
+    const int r = e / (NB / EPV), c = EPV * (e % (NB / EPV)), i = r / PB, j = c / PB;
+    const int o = inv_blk(i, j) + (r % PB) * (PB + 4) + c % PB;
+    if (j < i)
+      cp_async16((sl + o).a, L + (size_t)r * ld + c);
+    else if (j == i)
+      cp_async16((sx + o).a, X + (size_t)r * NB + c);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int j = w >> 1, h = 8 * (w & 1);
+#pragma unroll 1
+  for (int i = j + 1; i < kPBlocks; i++) {
+    T a[4] = {(T)0, (T)0, (T)0, (T)0}, b[4] = {(T)0, (T)0, (T)0, (T)0};
+#pragma unroll 1
+    for (int c = j; c < i; c++) inv_mac(a, sl + inv_blk(i, c), sx + (inv_blk(c, j) + h), PB + 4, lane);
+    inv_out(a, (T)1, st, 12, lane);
+    __syncwarp();
+    inv_mac(b, sx + inv_blk(i, i), st, 12, lane);
+    inv_out(b, (T)-1, sx + (inv_blk(i, j) + h), PB + 4, lane);
+    __syncwarp();
+  }
+  __syncthreads();
+#pragma unroll 2
+  for (int e = threadIdx.x; e < NB * (NB / 4); e += 512) {
+    const int r = e / (NB / 4), c = 4 * (e % (NB / 4)), i = r / PB, jj = c / PB;
+    if (jj >= i) continue;
+    T v[4];
+    load_row4(sx + (inv_blk(i, jj) + (r % PB) * (PB + 4) + c % PB), v);
+    store_row4(X + (size_t)r * NB + c, v[0], v[1], v[2], v[3]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The trailing update of the next diagonal tile, on the factorisation's
+// critical path (FP32): A_tt -= sum_p L_t,p L_t,p' over panels p in [p0, p0 +
+// np), by 128 / RPC CTAs of 256 threads, CTA c owning an RPC-row slice (RPC =
+// kChainRows below).  Both operands stay row-major in shared memory (row stride
 // 132 floats) and are read as float4 along K.
-constexpr int kSliceRows = 16;  // rows per CTA of the chain kernels at most (shared-memory sizes)
-// Rows per CTA of the row-tile TRSM and the diagonal-tile update on the
-// factorisation's critical path: 4 (32 CTAs).  Config 2, LM it/s on the
-// B200 with identical results: 16 rows (8 CTAs) 93.1, 8 rows 94.6, 4 rows
-// 95.6 -- every CTA stages the whole panel, so more CTAs cut each one's
-// FMAs, not its copies.
+// Rows per CTA, LM it/s at 1,500 9-parameter cameras with identical results:
+// 16 rows (8 CTAs) 93.1, 8 rows 94.6, 4 rows 95.6 -- every CTA stages the
+// whole panel, so more CTAs cut each one's FMAs, not its copies.
 constexpr int kChainRows = 4;
 static_assert(kChainRows == 16 || kChainRows == 8 || kChainRows == 4, "chain kernels: 4, 8 or 16 rows per CTA");
 constexpr int kSlLd = NB + 4;                // 132
-constexpr size_t kTrsmTileSmem = sizeof(float) * (size_t)(NB + kSliceRows) * kSlLd;  // 76,032 B
 constexpr size_t kDiagUpdSmem = sizeof(float) * (size_t)NB * kSlLd;                 // 67,584 B per panel
 
 // acc[h][m] += sum_l a_h[l] b[16 w + (lane & 3) + 4 m][l], l < NB
@@ -458,71 +856,12 @@ __device__ inline void slice_mma(const float* __restrict__ a0, const float* __re
   }
 }
 
-// 16-byte global -> shared copies that complete asynchronously: a kernel
-// issues all of its staging before one wait, so the staging costs one L2 /
-// HBM round trip however loaded the memory system is
-__device__ inline void cp_async16(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ inline void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 // rows x 128 FP32 columns (row stride ld) into shared memory (stride kSlLd)
 __device__ inline void stage_rows_f32(const float* __restrict__ src, size_t ld, int rows, float* __restrict__ dst,
                                       int tid) {
   for (int e = tid; e < rows * NB / 4; e += 256) {
     const int r = e >> 5, c4 = e & 31;
     cp_async16(dst + r * kSlLd + 4 * c4, src + (size_t)r * ld + 4 * c4);
-  }
-}
-
-template <int RPC>
-static __global__ void __launch_bounds__(256) trsm_tile_kernel(float* __restrict__ S, int ld, int j,
-                                                               const float* __restrict__ Linv,
-                                                               uint8_t* __restrict__ pack,
-                                                               const int* __restrict__ active) {
-  constexpr int P = RPC / 2, CG = 32 / P, M = 16 / CG;
-  extern __shared__ float4 smf4[];
-  float* sb = reinterpret_cast<float*>(smf4);  // inv(L_jj), row i = output column i
-  float* sa = sb + NB * kSlLd;                 // the slice's RPC rows of A_(j+1),j
-  chain_release();
-  chain_wait();
-  if (active && !*active) return;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int rel0 = blockIdx.x * RPC;  // first slice row within the tile
-  float* A = S + (size_t)((j + 1) * NB + rel0) * ld + (size_t)j * NB;
-  stage_rows_f32(Linv + (size_t)j * NB * NB, NB, NB, sb, tid);  // zeros above the diagonal included
-  stage_rows_f32(A, ld, RPC, sa, tid);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  float acc[2][M] = {};
-  const float* a0 = sa + (lane / CG) * kSlLd;
-  slice_mma<RPC>(a0, a0 + P * kSlLd, sb, lane, w, acc);
-  // stage the slice of L row-major over the A rows, then store rows to S
-  // (float4) and the pack (8 consecutive columns per item)
-  __syncthreads();
-#pragma unroll
-  for (int h = 0; h < 2; h++)
-#pragma unroll
-    for (int m = 0; m < M; m++) sa[((lane / CG) + P * h) * kSlLd + 16 * w + (lane % CG) + CG * m] = acc[h][m];
-  __syncthreads();
-  for (int e = tid; e < RPC * NB / 4; e += 256) {
-    const int r = e >> 5, c4 = e & 31;
-    *reinterpret_cast<float4*>(A + (size_t)r * ld + 4 * c4) = *reinterpret_cast<const float4*>(sa + r * kSlLd + 4 * c4);
-  }
-  if (pack) {
-    for (int e = tid; e < RPC * 16; e += 256) {
-      const int r = e >> 4, h = e & 15;
-      float x[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) x[q] = sa[r * kSlLd + 8 * h + q];
-      tc_pack_store8(pack, tc_pack_offset(rel0 + r, h), x);
-    }
   }
 }
 

@@ -148,8 +148,8 @@ class SchurCoreT final : public SchurCore {
     NL_TRY(part_.alloc(sizeof(double) * (size_t)std::max(kSymvChunks * ld_, 4 * kRedCTAs)));
     NL_TRY(Linv_.alloc(sizeof(T) * (size_t)ntiles_ * NB * NB));
     NL_TRY(hop_.alloc(sizeof(T) * 2 * kHopDepth * (size_t)ntiles_ * NB * NB));
-    // the diagonal-tile factor writes only the blocks on and below the
-    // diagonal: the strictly upper blocks of every inverse stay zero
+    // only the blocks on and below the diagonal are ever written: the
+    // strictly upper blocks of every inverse stay zero
     NL_CUDA(cudaMemsetAsync(Linv_.p, 0, Linv_.bytes, st_));
     NL_TRY(env_dev_.alloc(sizeof(int) * 2 * (size_t)ntiles_));
     NL_CUDA(cudaMemcpyAsync(env_dev_.p, env_first_.data(), sizeof(int) * ntiles_, cudaMemcpyHostToDevice, st_));
@@ -212,11 +212,15 @@ class SchurCoreT final : public SchurCore {
     d_.s_pair_ptr = s_ptr_.as<long long>();
     d_.pair_a = pa_.as<int>();
     d_.pair_b = pb_.as<int>();
-    NL_CUDA(cudaFuncSetAttribute(trsm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem<T>()));
+    NL_CUDA(cudaFuncSetAttribute(potrf_diag_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)potrf_smem<T>()));
+    NL_CUDA(cudaFuncSetAttribute(trsm_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem<T, 1>()));
+    NL_CUDA(cudaFuncSetAttribute(trsm_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem<T, 2>()));
+    NL_CUDA(cudaFuncSetAttribute(trsm_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)trsm_tile_smem<T>()));
+    NL_CUDA(cudaFuncSetAttribute(inv_tiles_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)inv_tiles_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(trsv_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(trsv_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
-    NL_CUDA(cudaFuncSetAttribute(trsm_tile_kernel<kChainRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kTrsmTileSmem));
     NL_CUDA(cudaFuncSetAttribute(diag_update_kernel<kChainRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  2 * (int)kDiagUpdSmem));
     if (!ev_[0]) {
@@ -329,14 +333,24 @@ class SchurCoreT final : public SchurCore {
     return NL_OK;
   }
 
+  // Rows [r0, r0 + nrows) of panel k.  One row per thread while that leaves
+  // SMs idle, else two: the staging of L_kk is then shared by twice the rows.
+  void launch_trsm(int k, int r0, int nrows, uint8_t* pack, const int* active, cudaStream_t st) {
+    if (nrows <= 16 * 148)
+      trsm_kernel<T, 1><<<cdiv(nrows, 16), 256, trsm_smem<T, 1>(), st>>>(S_.as<T>(), ld_, k, r0, nrows, Linv_.as<T>(),
+                                                                         pack, active);
+    else
+      trsm_kernel<T, 2><<<cdiv(nrows, 32), 256, trsm_smem<T, 2>(), st>>>(S_.as<T>(), ld_, k, r0, nrows, Linv_.as<T>(),
+                                                                         pack, active);
+    launches++;
+  }
+
   nl_status factor_panel(int k, int* status, const int* active) {
-    potrf_diag_kernel<T><<<1, PT, kPotrfSmem, st_>>>(S_.as<T>(), ld_, k, Linv_.as<T>(), status, active);
+    potrf_diag_kernel<T><<<1, PT, potrf_smem<T>(), st_>>>(S_.as<T>(), ld_, k, Linv_.as<T>(), status, active);
     launches++;
     const int below = std::min(ld_, (env_end(k) + 1) * NB) - (k + 1) * NB;  // rows past the envelope are zero
     if (below > 0) {
-      trsm_kernel<T><<<cdiv(below, TRSM_ROWS), 256, trsm_smem<T>(), st_>>>(S_.as<T>(), ld_, k, (k + 1) * NB, below,
-                                                                            Linv_.as<T>(), nullptr, active);
-      launches++;
+      launch_trsm(k, (k + 1) * NB, below, nullptr, active, st_);
       if (sizeof(T) == 4 && use_tc) {
         NL_CUDA(tc_pack_f32(reinterpret_cast<const float*>(S_.p), ld_, k, 0, below, pack_slot(k), active, st_));
         launches++;
@@ -387,7 +401,7 @@ class SchurCoreT final : public SchurCore {
   //           all G panels; TRSM + pack of the rows below tile k+G+1
   //     side  B: tiles of block columns >= k+2G with all G panels.
   // (The tile updates of the chain are diag_update_kernel, the row-tile TRSMs
-  // trsm_tile_kernel: NB / kChainRows CTAs each, FP32 on CUDA cores.)  Packs live in
+  // trsm_tile_kernel.)  Packs live in
   // kPackSlots = 2 G slots (panel mod 2 G): a group's B is the last reader of
   // its slots, and the group after next repacks them only after waiting for it.
   // With G = 2 this is the pair schedule (one B per two panels); G = 4 halves
@@ -440,17 +454,15 @@ class SchurCoreT final : public SchurCore {
       nrows = std::min(nrows, (env_end(j + G - 1) + 1) * NB - r0);
       if (nrows <= 0) return NL_OK;
       // the TRSM writes the BF16 pack of its rows in its epilogue
-      trsm_kernel<T><<<cdiv(nrows, TRSM_ROWS), 256, trsm_smem<T>(), st>>>(S_.as<T>(), ld_, j, r0, nrows,
-                                                                           Linv_.as<T>(), pack_slot(j), active);
-      launches++;
+      launch_trsm(j, r0, nrows, pack_slot(j), active, st);
       return NL_OK;
     };
     // row tile j+1 of panel j (the critical one) and the diagonal-tile
-    // updates: 32-CTA FP32 kernels on the main stream (kChainRows rows each)
+    // updates: FP32 kernels on the main stream
     auto trsm_first = [&](int j) {
       if (tmc) cudaEventRecord(upd_ev_[10 * nT + 4 * j], st_);
-      trsm_tile_kernel<kChainRows><<<NB / kChainRows, 256, kTrsmTileSmem, st_>>>(
-          S, ld_, j, reinterpret_cast<const float*>(Linv_.p), pack_slot(j), active);
+      trsm_tile_kernel<T><<<NB / kChainTrsmRows, 256, trsm_tile_smem<T>(), st_>>>(S_.as<T>(), ld_, j, Linv_.as<T>(),
+                                                                                  pack_slot(j), active);
       if (tmc) cudaEventRecord(upd_ev_[10 * nT + 4 * j + 1], st_);
       launches++;
     };
@@ -470,7 +482,7 @@ class SchurCoreT final : public SchurCore {
       const int e = 8 * nT + 2 * j;  // timing events after the update events
       if (tmc) cudaEventRecord(upd_ev_[e], st_);
       // a programmatic dependent of the diagonal update before it
-      NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, kPotrfSmem, j > 0 && !tmc, S_.as<T>(), ld_, j,
+      NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, potrf_smem<T>(), j > 0 && !tmc, S_.as<T>(), ld_, j,
                            Linv_.as<T>(), status, active));
       if (tmc) cudaEventRecord(upd_ev_[e + 1], st_);
       npev = j + 1;
@@ -699,7 +711,11 @@ class SchurCoreT final : public SchurCore {
     {
       NvtxRange r("nl:factorize");
       s = enqueue_factor(status, active);
-      // the hop matrices of the solves (M_d,I, Q_d,I)
+      // the tile inverses and the hop matrices of the solves (M_d,I, Q_d,I)
+      if (s == NL_OK) {
+        inv_tiles_kernel<T><<<ntiles_, 512, inv_tiles_smem<T>(), st_>>>(S_.as<T>(), ld_, Linv_.as<T>(), active);
+        launches++;
+      }
       if (s == NL_OK && ntiles_ > 1) {
         hop_mat_kernel<T><<<dim3(ntiles_ - 1, 2 * kHopDepth), 256, 0, st_>>>(S_.as<T>(), ld_, ntiles_, Linv_.as<T>(),
                                                                              hop_.as<T>(), active);
