@@ -10,7 +10,7 @@ namespace {
 constexpr int kNT = 256;
 constexpr int kRedCTAs = 296;  // 2 x 148 SMs for grid-stride reductions
 constexpr int kSymvChunks = 8;
-constexpr int kSchurWarps = 8;
+constexpr int kSchurMinChunk = 48, kSchurMaxChunk = 480;  // pairs of a Schur work item
 
 inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
@@ -107,11 +107,35 @@ class SchurCoreT final : public SchurCore {
       for (int k = env_first_[t]; k < t; k++) env_last_[k] = std::max(env_last_[k], t);
     env_run_.assign(ntiles_, 0);
     for (int k = 0; k < ntiles_; k++) env_run_[k] = std::max(env_last_[k], k > 0 ? env_run_[k - 1] : 0);
-    // Schur work order: output blocks by pair count, heaviest first
-    std::vector<int> s_order(std::max(nS_, 1), 0);
-    for (int b = 0; b < nS_; b++) s_order[b] = b;
-    std::stable_sort(s_order.begin(), s_order.begin() + nS_,
-                     [&](int x, int y) { return s_ptr[x + 1] - s_ptr[x] > s_ptr[y + 1] - s_ptr[y]; });
+    // Schur work items, longest first: a block's pair list in parts of at most
+    // chunk_ pairs.  A part costs its warp a fixed ~2 us (indices, first
+    // copies, the partial), so it has at least kSchurMinChunk pairs, and more
+    // where that still leaves every resident warp a few parts.  (96 and 2,000
+    // instead of 48 and 480 pairs: 111 / 953 us instead of 111 / 936 on the two
+    // scenes of schur_kernel's comment, three stages.)
+    {
+      constexpr int PBS = SchurCfg<T, BC>::PB;
+      const long long per = npairs / (148LL * 24 * 4);
+      chunk_ = (int)std::min<long long>(std::max<long long>(per, kSchurMinChunk), kSchurMaxChunk);
+      chunk_ = cdiv(chunk_, PBS) * PBS;
+    }
+    std::vector<SchurItem> items;
+    std::vector<int> slot(std::max(nS_, 1), -1);
+    int nslots = 0;
+    for (int b = 0; b < nS_; b++) {
+      const int np_parts = std::max(1, cdiv(s_ptr[b + 1] - s_ptr[b], chunk_));
+      if (np_parts > 1) {
+        slot[b] = nslots;
+        nslots += np_parts;
+      }
+      for (int k = 0; k < np_parts; k++) items.push_back({b, k});
+    }
+    nitems_ = (int)items.size();
+    auto item_pairs = [&](const SchurItem& it) {
+      return std::min<long long>(chunk_, s_ptr[it.block + 1] - s_ptr[it.block] - (long long)it.part * chunk_);
+    };
+    std::stable_sort(items.begin(), items.end(),
+                     [&](const SchurItem& x, const SchurItem& y) { return item_pairs(x) > item_pairs(y); });
     std::vector<int> pa(std::max<long long>(npairs, 1)), pb(std::max<long long>(npairs, 1));
     {
       std::vector<long long> fill(s_ptr.begin(), s_ptr.end() - 1);
@@ -175,8 +199,11 @@ class SchurCoreT final : public SchurCore {
     NL_TRY(upload(s_i_, s_i, st_));
     NL_TRY(upload(s_j_, s_j, st_));
     NL_TRY(upload(s_uuid_, s_uuid, st_));
-    NL_TRY(upload(s_order_, s_order, st_));
-    NL_TRY(sched_.alloc(sizeof(int) * 4));
+    NL_TRY(upload(s_items_, items, st_));
+    NL_TRY(upload(s_slot_, slot, st_));
+    NL_TRY(s_part_.alloc(sizeof(T) * (size_t)std::max(nslots, 1) * Layout<T, BC>::U));
+    NL_TRY(sched_.alloc(sizeof(int) * (size_t)(4 + std::max(nS_, 1))));
+    NL_CUDA(cudaMemsetAsync(sched_.p, 0, sched_.bytes, st_));
     NL_TRY(upload(s_ptr_, s_ptr, st_));
     NL_TRY(upload(pa_, pa, st_));
     NL_TRY(upload(pb_, pb, st_));
@@ -212,6 +239,10 @@ class SchurCoreT final : public SchurCore {
     d_.s_pair_ptr = s_ptr_.as<long long>();
     d_.pair_a = pa_.as<int>();
     d_.pair_b = pb_.as<int>();
+    NL_CUDA(cudaFuncSetAttribute(schur_kernel<T, BC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)SchurCfg<T, BC>::kSmem));
+    NL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&schur_occ_, schur_kernel<T, BC>,
+                                                          SchurCfg<T, BC>::kWarps * 32, SchurCfg<T, BC>::kSmem));
     NL_CUDA(cudaFuncSetAttribute(potrf_diag_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)potrf_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(trsm_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem<T, 1>()));
     NL_CUDA(cudaFuncSetAttribute(trsm_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem<T, 2>()));
@@ -695,11 +726,13 @@ class SchurCoreT final : public SchurCore {
       launches++;
     }
     {
-      const int grid = std::max(1, std::min(cdiv(nS_, kSchurWarps), 148 * 8));
+      using Cfg = SchurCfg<T, BC>;
+      const int grid = std::max(1, std::min(cdiv(nitems_, Cfg::kWarps), 148 * schur_occ_));
       NL_CUDA(cudaMemsetAsync(sched_.p, 0, sizeof(int), st_));
-      schur_kernel<T, BC, kSchurWarps><<<grid, kSchurWarps * 32, 0, st_>>>(
+      schur_kernel<T, BC><<<grid, Cfg::kWarps * 32, Cfg::kSmem, st_>>>(
           d_, U_.as<T>(), Y_.as<T>(), W_.as<T>(), lam, S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr,
-          s_order_.as<int>(), sched_.as<int>(), active);
+          s_items_.as<SchurItem>(), nitems_, chunk_, s_slot_.as<int>(), s_part_.as<T>(), sched_.as<int>() + 4,
+          sched_.as<int>(), active);
       if (ld_ > n_)
         pad_identity_kernel<T><<<cdiv(ld_ - n_, 128), 128, 0, st_>>>(S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr, n_,
                                                                      ld_, active);
@@ -873,6 +906,7 @@ class SchurCoreT final : public SchurCore {
   cudaStream_t st_ = nullptr;
   int nci_ = 0, np_ = 0, nU_ = 0, nV_ = 0, nW_ = 0, nS_ = 0, n_ = 0, ld_ = 0, ntiles_ = 0;
   long long npairs_ = 0;
+  int nitems_ = 0, chunk_ = 0, schur_occ_ = 1;  // work items of the Schur formation
   bool need_s0_ = false;
   SchurDev d_{};
   DevBuf U_, V_, W_, Y_, Vinv_, bU_, bV_, bS_, incU_, incV_, y_, r_, dx_, part_, Linv_, hop_, flags_, S_, S0_, tcs_;
@@ -882,8 +916,8 @@ class SchurCoreT final : public SchurCore {
   bool s_cleared_ = false;  // S / S0 have had their one full clear (enqueue_increment)
   // last tile row that panel k's TRSM and updates must cover
   int env_end(int k) const { return envelope ? env_run_[std::min(k, ntiles_ - 1)] : ntiles_ - 1; }
-  DevBuf v_uid_, w_row_ptr_, w_col_, w_row_, w_col_ptr_, w_col_uid_, u_diag_, s_i_, s_j_, s_uuid_, s_ptr_, pa_, pb_, s_order_,
-      sched_;
+  DevBuf v_uid_, w_row_ptr_, w_col_, w_row_, w_col_ptr_, w_col_uid_, u_diag_, s_i_, s_j_, s_uuid_, s_ptr_, pa_, pb_, s_items_,
+      s_slot_, s_part_, sched_;
   cudaEvent_t ev_[7] = {};
   cudaEvent_t ev_panel_ = nullptr, ev_b_ = nullptr;
   cudaStream_t st2_ = nullptr;  // side stream of the look-ahead factorisation

@@ -11,8 +11,8 @@
 //                    Y = W Vinv per W block, and bS = -bU + Y bV per camera
 //                    (= -bU - W xV0 of SolverCholeskySchur.hpp:114).
 //   schur_kernel     MatrixWWtMultiplier::multiply (MatrixWWtMultiplier.hpp:139-152):
-//                    S_ij = U_ij - sum_pairs Y_a W_b', one warp per output block over
-//                    the block's pair list (no atomics), plus the diagonal damping of
+//                    S_ij = U_ij - sum_pairs Y_a W_b', the block's pair list in
+//                    one or more warps (no float atomics), plus the diagonal damping of
 //                    SolverCholeskySchur.hpp:121-124, written to dense lower storage.
 //   backsub_kernel   MatrixWtXMultiplier::rightMultVectorSub + MatrixDiagInv::rightMultVector
 //                    (MatrixWtXMultiplier.hpp:58-62, MatrixDiagInv.hpp:153-156):
@@ -147,162 +147,228 @@ static __global__ void __launch_bounds__(NT) wvinv_bs_kernel(SchurDev d, const T
 }
 
 // ---------------------------------------------------------------------------
-// One warp per output block (i <= j); lanes own the BC*BC outputs round-robin.
-// Batches of PB pairs: lane l < 2 np loads one block UID (Y_a for l < np,
-// W_b above), the operands move as 16-byte vectors (blocks are padded to 16
-// bytes) and are re-laid in shared memory with rows padded to 4, so each
-// 3-term row product reads two vectors.
-template <typename T>
-struct Vec4;
-template <>
-struct Vec4<float> {
-  using type = float4;
-};
-template <>
-struct Vec4<double> {
-  using type = double4;
+// S_ij = U_ij - sum_pairs Y_a W_b'.  A work item is one warp's share of an
+// output block: `chunk` pairs of its list at most, so that the long lists (the
+// diagonal blocks: every observation of a camera) are spread over many warps.
+// Items are taken from a work counter, longest first.  The partial sums of a
+// block of several items are added by whichever of its warps finishes last, in
+// item order, so S does not depend on the schedule and no warp waits.
+//
+// Inside an item the pairs' blocks are copied to shared memory as they are
+// (16-byte asynchronous copies, kStages batches in flight per warp), and a lane
+// owns a TR x TR tile of the result (TR = 3, or 2 for BC = 2) of one pair in
+// flight: (BC / TR)^2 lanes a pair, G pairs side by side, so a lane reads 6 TR
+// values for 3 TR^2 FMAs.  A batch's products are summed before they join the
+// running sum (blocked summation: a diagonal block sums thousands of pairs in
+// the working precision).
+//
+// One warp per block was bound by the longest list on small scenes and by the
+// re-laying of the operands in padded rows (a register round trip and scalar
+// stores) on large ones.  200 cameras, 1.6 M pairs: 100 us against 413 us in
+// FP32, 177 against 578 us in FP64; 1,500 cameras, 16.5 M pairs (3.7 GB of
+// gathered blocks): 0.87 ms against 1.71.  Two stages of 12 pairs (9 x 9 blocks)
+// measured 100 / 871 us; three stages 122 / 936, two of 15 pairs 105 / 883,
+// three of 6 pairs 113 / 910.
+template <typename T, int BC>
+struct SchurCfg {
+  static constexpr int LW = Layout<T, BC>::W;
+  static constexpr int TR = BC % 3 == 0 ? 3 : 2;
+  static constexpr int TD = BC / TR;                // tiles along a block row
+  static constexpr int LP = TD * TD;                // lanes per pair
+  static constexpr int G = 32 / LP;                 // pairs side by side
+  static constexpr int ROUNDS = G >= 32 ? 1 : G >= 8 ? 2 : 4;
+  static constexpr int PB = G * ROUNDS;             // pairs per batch (<= 32)
+  static constexpr int kStages = 2;
+  static constexpr int kWarps = 8;
+  static constexpr int VB = LW * (int)sizeof(T) / 16;  // 16-byte vectors per block
+  static constexpr size_t kSmem = (size_t)kWarps * kStages * 2 * PB * LW * sizeof(T);
 };
 
-// A staged row of a BC x 3 block (padded to 4 elements, 16-byte aligned).
-__device__ __forceinline__ void load_row3(const float* p, float& a, float& b, float& c) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  a = v.x;
-  b = v.y;
-  c = v.z;
-}
-__device__ __forceinline__ void load_row3(const double* p, double& a, double& b, double& c) {
-  const double2 v = *reinterpret_cast<const double2*>(p);
-  a = v.x;
-  b = v.y;
-  c = p[2];
-}
+// one work item: pairs [first, first + chunk) of a block's list
+struct SchurItem {
+  int block, part;
+};
 
-// One warp per output block, blocks taken heaviest-first from a work counter
-// (`order` lists them by pair count, descending), so the long diagonal blocks
-// start early and the tail is short; each block is still summed by one warp
-// in pair order, so S does not depend on the schedule.  Lane l < NSTR owns a
-// 1 x SW strip (row r, columns c0 .. c0 + SW - 1) of the BC x BC block.
-// Per batch of PB pairs the warp stages Y_a and W_b (rows padded to 4) in
-// shared memory and already issues the global loads of the next batch, so
-// their latency overlaps this batch's FMAs.  The batch's products are summed
-// before they are subtracted (blocked summation: a diagonal block sums
-// thousands of pairs in the working precision).
-template <typename T, int BC, int WARPS>
-static __global__ void __launch_bounds__(WARPS * 32, 2) schur_kernel(SchurDev d, const T* __restrict__ U,
-                                                                      const T* __restrict__ Y, const T* __restrict__ W,
-                                                                      const double* __restrict__ lam, T* __restrict__ S,
-                                                                      T* __restrict__ S0, const int* __restrict__ order,
-                                                                      int* __restrict__ counter,
-                                                                      const int* __restrict__ active) {
-  constexpr int LW = Layout<T, BC>::W;
-  constexpr int LU = Layout<T, BC>::U;
-  // pairs per batch: FP32 measured fastest at 10 (against 4, 6, 8, 12, 16 on
-  // config 2); the FP64 comparison path keeps 8
-  constexpr int PB = sizeof(T) == 4 ? 10 : 8;
-  constexpr int SW = (BC % 3 == 0) ? 3 : ((BC % 2 == 0) ? 2 : 1);  // strip width
-  constexpr int NSTR = BC * BC / SW;                               // strips (<= 32)
-  constexpr int EPV = 16 / (int)sizeof(T);                         // elements per 16-byte vector
-  constexpr int VB = LW / EPV;                                     // vectors per block
-  constexpr int NV = (2 * PB * VB + 31) / 32;                      // staged vectors per lane
-  using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  static_assert(NSTR <= 32, "one strip per lane");
-  __shared__ __align__(16) T sh[WARPS][2][PB][BC][4];
+template <typename T, int BC>
+static __global__ void __launch_bounds__(SchurCfg<T, BC>::kWarps * 32)
+    schur_kernel(SchurDev d, const T* __restrict__ U, const T* __restrict__ Y, const T* __restrict__ W,
+                 const double* __restrict__ lam, T* __restrict__ S, T* __restrict__ S0,
+                 const SchurItem* __restrict__ items, int nitems, int chunk, const int* __restrict__ slot,
+                 T* __restrict__ partial, int* __restrict__ arrived, int* __restrict__ counter,
+                 const int* __restrict__ active) {
+  using Cfg = SchurCfg<T, BC>;
+  constexpr int LW = Cfg::LW, LU = Layout<T, BC>::U, TR = Cfg::TR, TD = Cfg::TD, LP = Cfg::LP, G = Cfg::G,
+                ROUNDS = Cfg::ROUNDS, PB = Cfg::PB, kStages = Cfg::kStages, VB = Cfg::VB;
+  extern __shared__ float4 schur_smem[];
   if (active && !*active) return;
   const double rel = lam[0], abs = lam[1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = lane / (BC / SW), c0 = (lane % (BC / SW)) * SW;
-  const bool own = lane < NSTR;
-  T(*sy)[BC][4] = sh[warp][0];
-  T(*sw)[BC][4] = sh[warp][1];
+  T* const sh = reinterpret_cast<T*>(schur_smem) + (size_t)warp * kStages * 2 * PB * LW;
+  const uint32_t sh_a = (uint32_t)__cvta_generic_to_shared(sh);
+  const int q = lane / LP, tile = lane % LP;  // pair slot, tile of the block
+  const int r0 = TR * (tile / TD), c0 = TR * (tile % TD);
+  const bool on = q < G;
   for (;;) {
     int idx = 0;
     if (lane == 0) idx = atomicAdd(counter, 1);
     idx = __shfl_sync(0xffffffffu, idx, 0);
-    if (idx >= d.nS) break;
-    const int b = order[idx];
-    const int bi = d.s_i[b], bj = d.s_j[b], uu = d.s_uuid[b];
-    T acc[SW];
+    if (idx >= nitems) break;
+    const SchurItem item = items[idx];
+    const int b = item.block;
+    const long long pb = d.s_pair_ptr[b], pe = d.s_pair_ptr[b + 1];
+    const long long p0 = pb + (long long)item.part * chunk;
+    const int cnt = (int)min((long long)chunk, pe - p0), nbatch = (cnt + PB - 1) / PB;
+    // UIDs of a batch's blocks: lane l holds pair l's
+    int ua = 0, ub = 0;
+    auto load_uids = [&](int t) {
+      if (lane < PB && t * PB + lane < cnt) {
+        ua = __ldg(d.pair_a + p0 + t * PB + lane);
+        ub = __ldg(d.pair_b + p0 + t * PB + lane);
+      }
+    };
+    // the 2 n blocks of batch t, Y blocks first, into its stage
+    auto copy_batch = [&](int t) {
+      const int n = min(PB, cnt - t * PB);
+      const uint32_t dst = sh_a + (uint32_t)((t % kStages) * 2 * PB * LW * (int)sizeof(T));
 #pragma unroll
-    for (int s2 = 0; s2 < SW; s2++)
-      acc[s2] = (own && uu >= 0) ? U[(size_t)uu * LU + r * BC + c0 + s2] : (T)0;
-    const long long p0 = d.s_pair_ptr[b], p1 = d.s_pair_ptr[b + 1];
-    // batch loader: lanes 0..np-1 fetch pair_a, np..2np-1 pair_b, then the
-    // 2 np blocks are read as VB 16-byte vectors each
-    V16 v[NV];
-    int np = 0;
-    auto load_batch = [&](long long pp) {
-      np = (int)min((long long)PB, p1 - pp);
-      int uid = 0;
-      if (lane < np) uid = __ldg(d.pair_a + pp + lane);
-      else if (lane < 2 * np) uid = __ldg(d.pair_b + pp + lane - np);
-#pragma unroll
-      for (int t = 0; t < NV; t++) {
-        const int u = lane + 32 * t;
-        const int blk = u / VB, part = u - blk * VB;
-        const int src_uid = __shfl_sync(0xffffffffu, uid, blk & 31);
-        if (blk < 2 * np) {
-          const T* base = (blk < np ? Y : W) + (size_t)src_uid * LW;
-          v[t] = __ldg(reinterpret_cast<const V16*>(base + part * EPV));
+      for (int v0 = 0; v0 < 2 * PB * VB; v0 += 32) {
+        const int v = v0 + lane, blk = v / VB, part = v - blk * VB;
+        const int pair = blk < PB ? blk : blk - PB;
+        const int y = __shfl_sync(0xffffffffu, ua, pair & 31), w = __shfl_sync(0xffffffffu, ub, pair & 31);
+        if (blk < 2 * PB && pair < n) {
+          const T* src = (blk < PB ? Y + (size_t)y * LW : W + (size_t)w * LW) + part * (16 / (int)sizeof(T));
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16u * (uint32_t)v), "l"(src) : "memory");
         }
       }
     };
-    if (p0 < p1) load_batch(p0);
-    for (long long pp = p0; pp < p1; pp += PB) {
-      const int cur = np;
-      // registers -> shared memory (rows padded to 4)
+    T acc[TR][TR];
 #pragma unroll
-      for (int t = 0; t < NV; t++) {
-        const int u = lane + 32 * t;
-        const int blk = u / VB, part = u - blk * VB;
-        if (blk < 2 * cur) {
-          T(*dst)[4] = blk < cur ? sy[blk] : sw[blk - cur];
-          const T* e = reinterpret_cast<const T*>(&v[t]);
+    for (int i = 0; i < TR; i++)
 #pragma unroll
-          for (int m = 0; m < EPV; m++) {
-            const int el = part * EPV + m;  // element of the BC x 3 block
-            if (el < BC * 3) dst[el / 3][el % 3] = e[m];
-          }
+      for (int j = 0; j < TR; j++) acc[i][j] = (T)0;
+    load_uids(0);
+#pragma unroll
+    for (int t = 0; t < kStages - 1; t++) {
+      if (t < nbatch) {
+        copy_batch(t);
+        load_uids(t + 1);
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    for (int t = 0; t < nbatch; t++) {
+      if (t + kStages - 1 < nbatch) {
+        copy_batch(t + kStages - 1);
+        load_uids(t + kStages);
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 1) : "memory");
+      __syncwarp();
+      const T* st = sh + (t % kStages) * 2 * PB * LW;
+      T part[TR][TR];
+#pragma unroll
+      for (int i = 0; i < TR; i++)
+#pragma unroll
+        for (int j = 0; j < TR; j++) part[i][j] = (T)0;
+#pragma unroll
+      for (int r = 0; r < ROUNDS; r++) {
+        const int pair = r * G + q;
+        if (on && t * PB + pair < cnt) {
+          const T* y = st + pair * LW + 3 * r0;
+          const T* w = st + (PB + pair) * LW + 3 * c0;
+          T yv[TR][3], wv[TR][3];
+#pragma unroll
+          for (int i = 0; i < TR; i++)
+#pragma unroll
+            for (int m = 0; m < 3; m++) {
+              yv[i][m] = y[3 * i + m];
+              wv[i][m] = w[3 * i + m];
+            }
+#pragma unroll
+          for (int i = 0; i < TR; i++)
+#pragma unroll
+            for (int j = 0; j < TR; j++)
+#pragma unroll
+              for (int m = 0; m < 3; m++) part[i][j] += yv[i][m] * wv[j][m];
         }
       }
-      __syncwarp();
-      if (pp + PB < p1) load_batch(pp + PB);  // in flight during the FMAs below
-      if (own) {
-        T part[SW];
 #pragma unroll
-        for (int s2 = 0; s2 < SW; s2++) part[s2] = (T)0;
-        for (int q = 0; q < cur; q++) {
-          T y0, y1, y2;
-          load_row3(sy[q][r], y0, y1, y2);
+      for (int i = 0; i < TR; i++)
 #pragma unroll
-          for (int s2 = 0; s2 < SW; s2++) {
-            T w0, w1, w2;
-            load_row3(sw[q][c0 + s2], w0, w1, w2);
-            part[s2] += y0 * w0 + y1 * w1 + y2 * w2;
-          }
+        for (int j = 0; j < TR; j++) acc[i][j] += part[i][j];
+      __syncwarp();  // the stage is free for the copy of the next iteration
+    }
+    // the pair slots' sums, onto slot 0 in a fixed order
+    if (G == 3) {
+#pragma unroll
+      for (int i = 0; i < TR; i++)
+#pragma unroll
+        for (int j = 0; j < TR; j++) {
+          const T x = __shfl_down_sync(0xffffffffu, acc[i][j], LP), z = __shfl_down_sync(0xffffffffu, acc[i][j], 2 * LP);
+          acc[i][j] += x + z;
         }
+    } else {
 #pragma unroll
-        for (int s2 = 0; s2 < SW; s2++) acc[s2] -= part[s2];
+      for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < TR; i++)
+#pragma unroll
+          for (int j = 0; j < TR; j++) acc[i][j] += __shfl_down_sync(0xffffffffu, acc[i][j], o * LP);
+    }
+    const int sl = slot[b];  // first partial of a block of several items, -1 otherwise
+    if (sl >= 0) {
+      const int nparts = (int)((pe - pb + chunk - 1) / chunk);
+      T* mine = partial + (size_t)(sl + item.part) * LU;
+      if (lane < LP) {
+#pragma unroll
+        for (int i = 0; i < TR; i++)
+#pragma unroll
+          for (int j = 0; j < TR; j++) mine[(r0 + i) * BC + c0 + j] = acc[i][j];
       }
+      __threadfence();
       __syncwarp();
+      int last = 0;
+      if (lane == 0) {
+        last = atomicAdd(arrived + b, 1) == nparts - 1;
+        if (last) arrived[b] = 0;  // for the next call
+      }
+      if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+      __threadfence();
+      if (lane < LP) {
+#pragma unroll
+        for (int i = 0; i < TR; i++)
+#pragma unroll
+          for (int j = 0; j < TR; j++) acc[i][j] = (T)0;
+        for (int k = 0; k < nparts; k++) {
+          const T* p = partial + (size_t)(sl + k) * LU;
+#pragma unroll
+          for (int i = 0; i < TR; i++)
+#pragma unroll
+            for (int j = 0; j < TR; j++) acc[i][j] += __ldcg(p + (r0 + i) * BC + c0 + j);
+        }
+      }
     }
     // damping on the diagonal of diagonal blocks, then the store (lower storage:
     // S_lower[j*BC + c][i*BC + r] = S_ij[r][c])
-    if (own) {
-      const int ud = (bi == bj) ? d.u_diag_uid[bi] : -1;
+    if (lane < LP) {
+      const int bi = d.s_i[b], bj = d.s_j[b], uu = d.s_uuid[b];
 #pragma unroll
-      for (int s2 = 0; s2 < SW; s2++) {
-        const int cc = c0 + s2;
-        T val = acc[s2];
-        if (bi == bj && r == cc && (rel != 0.0 || abs != 0.0)) {
-          const double udg = ud >= 0 ? (double)U[(size_t)ud * LU + r * BC + r] : 0.0;
-          val = (T)((double)val + rel * udg + abs);
+      for (int i = 0; i < TR; i++)
+#pragma unroll
+        for (int j = 0; j < TR; j++) {
+          const int r = r0 + i, cc = c0 + j;
+          const T u = uu >= 0 ? U[(size_t)uu * LU + r * BC + cc] : (T)0;
+          T val = u - acc[i][j];
+          if (bi == bj && r == cc && (rel != 0.0 || abs != 0.0)) {
+            const int ud = d.u_diag_uid[bi];
+            const double udg = ud >= 0 ? (double)U[(size_t)ud * LU + r * BC + r] : 0.0;
+            val = (T)((double)val + rel * udg + abs);
+          }
+          const size_t o = (size_t)(bj * BC + cc) * d.ld + (size_t)(bi * BC + r);
+          if (bi != bj || cc >= r) {
+            S[o] = val;
+            if (S0) S0[o] = val;
+          }
         }
-        const size_t o = (size_t)(bj * BC + cc) * d.ld + (size_t)(bi * BC + r);
-        if (bi != bj || cc >= r) {
-          S[o] = val;
-          if (S0) S0[o] = val;
-        }
-      }
     }
   }
 }
