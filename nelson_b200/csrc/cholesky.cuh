@@ -180,7 +180,8 @@ __device__ __forceinline__ void named_arrive(int id, int n) {
 // Eliminates the 16 x 16 block whose row lane % 16 is a[] (entries right of the
 // diagonal are ignored), leaving the row of L in a[] and publishing every
 // column in uc, (1 / d, 1 / sqrt(d)) in inv_s.  False on a non-positive pivot.
-template <typename T>
+// kPaced: named barriers pace the row warps of the same CTA behind it.
+template <typename T, bool kPaced = true>
 __device__ __forceinline__ bool pivot_block(T (&a)[PB], Sh<T> uc, Sh<T> inv_s, int lane) {
   bool ok = true;
   T d = __shfl_sync(0xffffffffu, a[0], 0);
@@ -220,17 +221,17 @@ __device__ __forceinline__ bool pivot_block(T (&a)[PB], Sh<T> uc, Sh<T> inv_s, i
     if (j + 2 < PB) a[j + 2] -= t * u2;
     a[j] *= rs;
     tp = t;
-    if ((j & 7) == 7) named_arrive(1 + (j >> 3), 32 * (1 + kRowWarps));
+    if (kPaced && (j & 7) == 7) named_arrive(1 + (j >> 3), 32 * (1 + kRowWarps));
   }
   return ok;
 }
 
 // The same elimination for a row outside the pivot block.
-template <typename T>
+template <typename T, bool kPaced = true>
 __device__ __forceinline__ void follow_block(T (&a)[PB], Sh<T> uc, Sh<T> inv_s) {
 #pragma unroll
   for (int j = 0; j < PB; j++) {
-    if ((j & 7) == 0) named_sync(1 + (j >> 3), 32 * (1 + kRowWarps));
+    if (kPaced && (j & 7) == 0) named_sync(1 + (j >> 3), 32 * (1 + kRowWarps));
     T ri, rs;
     load_two(inv_s + 2 * j, ri, rs);
     const T t = a[j] * ri;
