@@ -6,8 +6,8 @@
 // Hessian block is produced by exactly one thread or one CTA, which sums its
 // edges in a fixed order, so results are bit-reproducible run to run.
 //
-//   cost_kernel      one thread per edge, FP64 residual, chi2 per CTA, then
-//                    cost_finalize sums the CTA partials in index order.
+//   cost_kernel      one thread per edge, FP64 residual, chi2 per CTA; the last
+//                    CTA sums the partials in index order.
 //   cam_pass_kernel  one CTA per (internal) camera: edges in W-UID order,
 //                    writes each W block (J_c' J_p) and reduces U_c, bU_c.
 //   pt_pass_kernel   one thread per point: V_p, bV_p.
@@ -112,8 +112,8 @@ __device__ __forceinline__ void ba_project(const double* __restrict__ cs, const 
 // chi2 = sum_e w_e |r_e|^2 in FP64.  `active` (may be null) skips the launch
 // body when the device-side LM state says so.
 template <int BC, int NT>
-static __global__ void __launch_bounds__(NT) cost_kernel(BaDev d, double* __restrict__ partial,
-                                                  const int* __restrict__ active) {
+static __global__ void __launch_bounds__(NT) cost_kernel(BaDev d, double* __restrict__ partial, int* __restrict__ count,
+                                                  double* __restrict__ out, const int* __restrict__ active) {
   __shared__ double sh[NT / 32];
   if (active && !*active) return;
   double acc = 0.0;
@@ -125,8 +125,15 @@ static __global__ void __launch_bounds__(NT) cost_kernel(BaDev d, double* __rest
                                          d.f_fixed, d.cx, d.cy, r0, r1, nullptr, nullptr);
     acc += __ldg(d.e_w + e) * (r0 * r0 + r1 * r1);
   }
-  const double s = block_sum<NT>(acc, sh);
+  double s = block_sum<NT>(acc, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (!last_block(count)) return;
+  // the last CTA adds the partials, each thread a contiguous chunk
+  const int n = gridDim.x, per = (n + NT - 1) / NT, b = threadIdx.x * per;
+  acc = 0.0;
+  for (int i = b; i < min(n, b + per); i++) acc += __ldcg(partial + i);
+  s = block_sum<NT>(acc, sh);
+  if (threadIdx.x == 0) *out = s;
 }
 
 // Sums the per-CTA partials in index order (deterministic) into *out.
@@ -283,10 +290,17 @@ static __global__ void __launch_bounds__(NT) pt_pass_kernel(BaDev d, T* __restri
 // ---------------------------------------------------------------------------
 // Problem::oplus on the device: cameras R <- exp(dw) R, t += dt (, f/k += d);
 // points += d.  The camera increment is read at its internal position.
+// Blocks [0, cam_blocks) update the cameras, the others the points.
 template <int BC>
-static __global__ void oplus_cam_kernel(double* __restrict__ cam, const int* __restrict__ cam_slot_of_internal,
-                                 int nci, const double* __restrict__ incU, const int* __restrict__ active) {
+static __global__ void oplus_kernel(double* __restrict__ cam, const int* __restrict__ cam_slot_of_internal, int nci,
+                                    const double* __restrict__ incU, int cam_blocks, double* __restrict__ pt,
+                                    int np_var, const double* __restrict__ incV, const int* __restrict__ active) {
   if (active && !*active) return;
+  if ((int)blockIdx.x >= cam_blocks) {
+    const int i = (blockIdx.x - cam_blocks) * blockDim.x + threadIdx.x;
+    if (i < 3 * np_var) pt[i] += incV[i];
+    return;
+  }
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nci) return;
   double* s = cam + (size_t)cam_slot_of_internal[c] * 16;
@@ -305,14 +319,6 @@ static __global__ void oplus_cam_kernel(double* __restrict__ cam, const int* __r
 #pragma unroll
     for (int i = 0; i < 3; i++) s[12 + i] += dlt[6 + i];
   }
-}
-
-static __global__ void oplus_pt_kernel(double* __restrict__ pt, int np_var, const double* __restrict__ incV,
-                                const int* __restrict__ active) {
-  if (active && !*active) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * np_var) return;
-  pt[i] += incV[i];
 }
 
 }  // namespace nl

@@ -1212,13 +1212,16 @@ static __global__ void __launch_bounds__(256) hop_mat_kernel(const T* __restrict
 // tiles J < I - kHopDepth of its row as they are published, forms c_I =
 // Linv_I (b_I - partial) while its neighbours are still being solved, then
 // subtracts M_d,I y_I-d for d = kHopDepth .. 1, each as soon as that tile is
-// published.  Thread (warp w, lane l) holds rows 8 w .. 8 w + 7, columns
+// published.  b = the vector b less, if given, the nch partials `part` of a
+// refinement residual.  Thread (warp w, lane l) holds rows 8 w .. 8 w + 7, columns
 // 4 l .. 4 l + 3 of every 128 x 128 block it applies.
 template <typename T>
 static __global__ void __launch_bounds__(SV) trsv_fwd_kernel(const T* __restrict__ L, int ld, int ntiles,
                                                              const T* __restrict__ Linv,
                                                              const T* __restrict__ hop,
-                                                             const double* __restrict__ b, double* __restrict__ y,
+                                                             const double* __restrict__ b,
+                                                             const double* __restrict__ part, int nch,
+                                                             double* __restrict__ y,
                                                              int* __restrict__ ticket, int* __restrict__ flags,
                                                              int epoch, int* __restrict__ status,
                                                              long long spin_limit,
@@ -1238,11 +1241,13 @@ static __global__ void __launch_bounds__(SV) trsv_fwd_kernel(const T* __restrict
     float4* dst = sLi4;
     for (int i = tid; i < (int)(NB * NB * sizeof(T) / 16); i += SV) dst[i] = src[i];
   }
-  double part[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  double dots[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   const T* Lrow = L + (size_t)(I * NB + warp * 8) * ld + 4 * lane;
   // the right-hand side of the row this lane finishes, loaded now
   const int rsel = warp * 8 + reduce8_row(lane);
-  const double b_own = b[(size_t)I * NB + rsel];
+  double b_own = b[(size_t)I * NB + rsel];
+  if (part)
+    for (int c = 0; c < nch; c++) b_own -= part[(size_t)c * ntiles * NB + (size_t)I * NB + rsel];
   // with an envelope, the tiles of row I before its first nonzero are zero
   const int J0 = env ? env[I] : 0;
   const int Jend = I - kHopDepth;  // tiles [J0, Jend) are streamed, the last kHopDepth go through M_d,I
@@ -1269,7 +1274,7 @@ static __global__ void __launch_bounds__(SV) trsv_fwd_kernel(const T* __restrict
     double yv[4];
     load4_cg(y + (size_t)J * NB + 4 * lane, yv);
 #pragma unroll
-    for (int rr = 0; rr < 8; rr++) part[rr] += cur[rr].dot(yv);
+    for (int rr = 0; rr < 8; rr++) dots[rr] += cur[rr].dot(yv);
     if (kPre) {
 #pragma unroll
       for (int rr = 0; rr < 8; rr++) cur[rr] = nxt[rr];
@@ -1280,7 +1285,7 @@ static __global__ void __launch_bounds__(SV) trsv_fwd_kernel(const T* __restrict
   }
   // c_I = Linv_I (b_I - partial)
   {
-    const double sr = reduce8(part, lane);
+    const double sr = reduce8(dots, lane);
     if ((lane & 3) == 0) acc[rsel] = b_own - sr;
   }
   __syncthreads();
@@ -1318,12 +1323,14 @@ static __global__ void __launch_bounds__(SV) trsv_fwd_kernel(const T* __restrict
 // J > I + kHopDepth of column I (rows of L_J,I) as they are published, forms
 // c'_I = Linv_I' (y_I - partial), then subtracts Q_d,I x_I+d for
 // d = kHopDepth .. 1 (Q_d,I row-major: row c is column c of L_I+d,I Linv_I,
-// so these steps have the forward kernel's row layout).
+// so these steps have the forward kernel's row layout).  `sum`, if given, gets x
+// added (a refinement step).
 template <typename T>
 static __global__ void __launch_bounds__(SV) trsv_bwd_kernel(const T* __restrict__ L, int ld, int ntiles,
                                                              const T* __restrict__ Linv,
                                                              const T* __restrict__ hop,
                                                              const double* __restrict__ yv, double* __restrict__ x,
+                                                             double* __restrict__ sum,
                                                              int* __restrict__ ticket, int* __restrict__ flags,
                                                              int epoch, int* __restrict__ status,
                                                              long long spin_limit,
@@ -1437,7 +1444,10 @@ static __global__ void __launch_bounds__(SV) trsv_bwd_kernel(const T* __restrict
     for (int rr = 0; rr < 8; rr++) q8[rr] = qrow[rr].dot(xv);
     xr -= reduce8(q8, lane);
   }
-  if ((lane & 3) == 0) x[(size_t)I * NB + rsel] = xr;
+  if ((lane & 3) == 0) {
+    x[(size_t)I * NB + rsel] = xr;
+    if (sum) sum[(size_t)I * NB + rsel] += xr;
+  }
   publish_tile(flags + I, epoch, tid);
 }
 
@@ -1447,7 +1457,7 @@ static __global__ void __launch_bounds__(SV) trsv_bwd_kernel(const T* __restrict
 // the tile S0_IJ is read row-wise (y_I += S0_IJ x_J), for J > I the tile
 // S0_JI is read row-wise and applied transposed (y_I += S0_JI' x_J); the
 // diagonal tile uses both halves.  Partials per chunk are summed in a fixed
-// order by resid_finalize_kernel.
+// order by the forward solve that follows.
 template <typename T, int NCH>
 static __global__ void __launch_bounds__(SV) symv_partial_kernel(const T* __restrict__ S0, int ld, int ntiles,
                                                                  const double* __restrict__ x,
@@ -1513,25 +1523,6 @@ static __global__ void __launch_bounds__(SV) symv_partial_kernel(const T* __rest
       part[(size_t)ch * ntiles * NB + (size_t)I * NB + r] = rowsum[rr] + c;
     }
   }
-}
-
-template <int NCH>
-static __global__ void resid_finalize_kernel(const double* __restrict__ part, const double* __restrict__ b, int n_pad,
-                                      double* __restrict__ r, const int* __restrict__ active) {
-  if (active && !*active) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_pad) return;
-  double s = 0.0;
-#pragma unroll
-  for (int c = 0; c < NCH; c++) s += part[(size_t)c * n_pad + i];
-  r[i] = b[i] - s;
-}
-
-static __global__ void axpy_kernel(double* __restrict__ x, const double* __restrict__ d, int n,
-                            const int* __restrict__ active) {
-  if (active && !*active) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] += d[i];
 }
 
 }  // namespace nl

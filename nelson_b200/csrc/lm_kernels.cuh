@@ -5,15 +5,15 @@
 // that read and write an LmDev record in device memory, so one sub-iteration
 // is a fixed launch sequence (capturable in a CUDA graph) whose kernels test
 // flags instead of the host branching:
-//   lm_begin_kernel    active = !done; clears the solver status word
 //   [computeIncrement kernels, predicated on `active`]
-//   lm_inc_kernel      |inc|^2, den = inc'(mu inc - b); SuccessSmallIncrement test;
+//   inc_dot_kernel     |inc|^2, den = inc'(mu inc - b); SuccessSmallIncrement test;
 //                      `apply` = active && solve ok && !done
 //   [oplus + cost kernels, predicated on `apply`]
 //   lm_decide_kernel   rho, accept / reject, mu / v update, termination tests;
 //                      `rollback` and `do_jac` flags
 //   [rollback copies on `rollback`; Jacobian pass on `do_jac`]
-//   lm_after_jac_kernel oldChi2 = chi2, iter++, MaxIterationReached test
+//   lm_after_jac_kernel oldChi2 = chi2, iter++, MaxIterationReached test; the
+//                      next sub-iteration's flags (active = !done, status 0)
 #pragma once
 
 #include "nl_common.cuh"
@@ -28,26 +28,24 @@ struct LmDev {
   // state
   double mu, curV, oldChi2, chi2, chi2_new, rho, incSq, den, maxAbsB, maxAbsHDiag;
   double lam[2];  // (relLambda, absLambda) read by the solver kernels
-  int iter, subiter, nsub, done, reason, solve_ok;
+  int iter, subiter, nsub, done;  // read by the host in one copy
+  int reason, solve_ok;
   int active, apply, rollback, do_jac, accepted;
   int trace_n, trace_cap;
   int status;     // solver status bits of the current sub-iteration
 };
 
-static __global__ void lm_begin_kernel(LmDev* s) {
+// The flags and the damping of the next sub-iteration: set on the host for the
+// first one, at the end of lm_after_jac_kernel for the others.
+__host__ __device__ inline void lm_begin(LmDev* s) {
   s->active = s->done ? 0 : 1;
   s->status = 0;
   s->apply = 0;
   s->rollback = 0;
   s->do_jac = 0;
   if (!s->done) {
-    if (s->gn) {
-      s->lam[0] = s->gnRel;
-      s->lam[1] = s->gnAbs;
-    } else {
-      s->lam[0] = 0.0;
-      s->lam[1] = s->mu;
-    }
+    s->lam[0] = s->gn ? s->gnRel : 0.0;
+    s->lam[1] = s->gn ? s->gnAbs : s->mu;
   }
 }
 
@@ -60,12 +58,15 @@ __device__ inline void lm_trace(LmDev* s, double* trace, double it, double sub, 
   s->trace_n++;
 }
 
-// Partial sums of |inc|^2 and inc'(mu inc - b) over CTAs.
+// |inc|^2 and inc'(mu inc - b), CTA partials added by the last CTA, which then
+// takes the first decisions of the sub-iteration.
+__device__ inline void lm_inc(LmDev* s, double a, double b, double* trace);
 template <typename T, int NT>
 static __global__ void __launch_bounds__(NT) inc_dot_kernel(const double* __restrict__ incU, const T* __restrict__ bU,
                                                      int nu, const double* __restrict__ incV,
-                                                     const T* __restrict__ bV, int nv, const LmDev* __restrict__ s,
-                                                     double* __restrict__ part) {
+                                                     const T* __restrict__ bV, int nv, LmDev* __restrict__ s,
+                                                     double* __restrict__ part, int* __restrict__ count,
+                                                     double* __restrict__ trace) {
   __shared__ double sh[NT / 32];
   if (!s->active) return;
   const double mu = s->gn ? 0.0 : s->mu;
@@ -88,15 +89,18 @@ static __global__ void __launch_bounds__(NT) inc_dot_kernel(const double* __rest
     part[2 * blockIdx.x] = a;
     part[2 * blockIdx.x + 1] = b;
   }
+  if (!last_block(count)) return;
+  a = b = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += NT) {
+    a += __ldcg(part + 2 * i);
+    b += __ldcg(part + 2 * i + 1);
+  }
+  a = block_sum<NT>(a, sh);
+  b = block_sum<NT>(b, sh);
+  if (threadIdx.x == 0) lm_inc(s, a, b, trace);
 }
 
-static __global__ void lm_inc_kernel(LmDev* s, const double* __restrict__ part, int nparts, double* trace) {
-  if (!s->active) return;
-  double a = 0.0, b = 0.0;
-  for (int i = 0; i < nparts; i++) {
-    a += part[2 * i];
-    b += part[2 * i + 1];
-  }
+__device__ inline void lm_inc(LmDev* s, double a, double b, double* trace) {
   s->solve_ok = (s->status & (ST_VINV_FAIL | ST_CHOL_FAIL | ST_SPIN_TIMEOUT)) == 0;
   if (!isfinite(a)) s->solve_ok = 0;
   s->incSq = s->solve_ok ? a : 0.0;
@@ -175,9 +179,10 @@ static __global__ void lm_decide_kernel(LmDev* s, double* trace) {
   if (acc) s->do_jac = 1;
 }
 
-static __global__ void lm_after_jac_kernel(LmDev* s, const double* __restrict__ chi2, double* trace) {
-  if (!s->do_jac) return;
-  s->chi2 = *chi2;
+// The cost of update(true) is the accepted candidate's: the same parameters.
+// chi2_out: the handle's cost.
+__device__ inline void lm_after_jac(LmDev* s, double* chi2_out, double* trace) {
+  s->chi2 = *chi2_out = s->chi2_new;
   s->oldChi2 = s->chi2;
   if (s->gn) {
     // GaussNewton.hpp:104-123
@@ -200,11 +205,40 @@ static __global__ void lm_after_jac_kernel(LmDev* s, const double* __restrict__ 
     s->reason = NL_MAX_ITERATION_REACHED;
   }
 }
+static __global__ void lm_after_jac_kernel(LmDev* s, double* chi2_out, double* trace) {
+  if (!s->active) return;
+  if (s->do_jac) lm_after_jac(s, chi2_out, trace);
+  lm_begin(s);
+}
 
-// max |x| over two arrays (CTA partials).
+// Maximum over the block, then over the CTAs' partials by the last CTA.
+template <int NT>
+__device__ inline void max_out(double m, double* sh, double* __restrict__ part, int* __restrict__ count,
+                               double* __restrict__ out) {
+  auto block_max = [&](double v) {
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double r = 0.0;
+    if (threadIdx.x == 0)
+      for (int i = 0; i < NT / 32; i++) r = fmax(r, sh[i]);
+    __syncthreads();
+    return r;
+  };
+  m = block_max(m);
+  if (threadIdx.x == 0) part[blockIdx.x] = m;
+  if (!last_block(count)) return;
+  m = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += NT) m = fmax(m, __ldcg(part + i));
+  m = block_max(m);
+  if (threadIdx.x == 0) *out = m;
+}
+
+// max |x| over two arrays.
 template <typename T, int NT>
 static __global__ void __launch_bounds__(NT) maxabs_kernel(const T* __restrict__ a, int na, const T* __restrict__ b, int nb,
-                                                    double* __restrict__ part, const int* __restrict__ active) {
+                                                    double* __restrict__ part, int* __restrict__ count,
+                                                    double* __restrict__ out, const int* __restrict__ active) {
   __shared__ double sh[NT / 32];
   if (active && !*active) return;
   double m = 0.0;
@@ -212,33 +246,18 @@ static __global__ void __launch_bounds__(NT) maxabs_kernel(const T* __restrict__
     const double v = fabs((double)(i < na ? a[i] : b[i - na]));
     m = fmax(m, v);
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) sh[w] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int i = 0; i < NT / 32; i++) r = fmax(r, sh[i]);
-    part[blockIdx.x] = r;
-  }
-}
-
-static __global__ void max_finalize_kernel(const double* __restrict__ part, int n, double* __restrict__ out,
-                                    const int* __restrict__ active) {
-  if (active && !*active) return;
-  double m = 0.0;
-  for (int i = 0; i < n; i++) m = fmax(m, part[i]);
-  *out = m;
+  max_out<NT>(m, sh, part, count, out);
 }
 
 // max |diag| over the U diagonal blocks and the V blocks (SolverCholeskySchur::maxAbsHDiag).
-template <typename T, int BC>
-static __global__ void hdiag_kernel(const T* __restrict__ U, const int* __restrict__ u_diag_uid, int nci,
-                             const T* __restrict__ V, const int* __restrict__ v_uid, int np,
-                             double* __restrict__ part) {
-  __shared__ double sh[8];
+template <typename T, int BC, int NT>
+static __global__ void __launch_bounds__(NT) hdiag_kernel(const T* __restrict__ U, const int* __restrict__ u_diag_uid,
+                                                   int nci, const T* __restrict__ V, const int* __restrict__ v_uid,
+                                                   int np, double* __restrict__ part, int* __restrict__ count,
+                                                   double* __restrict__ out) {
+  __shared__ double sh[NT / 32];
   double m = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nci + np; i += gridDim.x * blockDim.x) {
+  for (int i = blockIdx.x * NT + threadIdx.x; i < nci + np; i += gridDim.x * NT) {
     if (i < nci) {
       const int q = u_diag_uid[i];
       if (q >= 0)
@@ -249,30 +268,17 @@ static __global__ void hdiag_kernel(const T* __restrict__ U, const int* __restri
         for (int r = 0; r < 3; r++) m = fmax(m, fabs((double)V[(size_t)q * Layout<T, BC>::V + r * 3 + r]));
     }
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) r = fmax(r, sh[i]);
-    part[blockIdx.x] = r;
-  }
+  max_out<NT>(m, sh, part, count, out);
 }
 
-static __global__ void zero_if_failed_kernel(double* __restrict__ x, int n, const int* __restrict__ status,
-                                      const int* __restrict__ active) {
-  if (active && !*active) return;
-  if ((*status & (ST_VINV_FAIL | ST_CHOL_FAIL | ST_SPIN_TIMEOUT)) == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] = 0.0;
-}
-
-// copy predicated on a device flag (backup / rollback of parameters)
+// copies predicated on a device flag (backup / rollback of parameters)
 static __global__ void copy_if_kernel(double* __restrict__ dst, const double* __restrict__ src, size_t n,
-                               const int* __restrict__ flag) {
+                                      double* __restrict__ dst2, const double* __restrict__ src2, size_t n2,
+                                      const int* __restrict__ flag) {
   if (flag && !*flag) return;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    dst[i] = src[i];
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = t; i < n; i += nt) dst[i] = src[i];
+  for (size_t i = t; i < n2; i += nt) dst2[i] = src2[i];
 }
 
 }  // namespace nl

@@ -58,6 +58,22 @@ __device__ inline double block_sum(double v, double* sh) {
   return s;
 }
 
+// True for all threads of the block of a launch that finishes last (`count`
+// starts at zero and is left at zero): that block can read what the others
+// wrote before the call.  Replaces a second launch for the final reduction.
+__device__ inline bool last_block(int* count) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(count, 1) == (int)gridDim.x - 1;
+    if (last) *count = 0;
+  }
+  __syncthreads();
+  __threadfence();
+  return last != 0;
+}
+
 __device__ inline double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;

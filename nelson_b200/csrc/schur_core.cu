@@ -167,7 +167,6 @@ class SchurCoreT final : public SchurCore {
     NL_TRY(incU_.alloc(sizeof(double) * (size_t)ld_));
     NL_TRY(incV_.alloc(sizeof(double) * (size_t)std::max(3 * np_, 1)));
     NL_TRY(y_.alloc(sizeof(double) * (size_t)ld_));
-    NL_TRY(r_.alloc(sizeof(double) * (size_t)ld_));
     NL_TRY(dx_.alloc(sizeof(double) * (size_t)ld_));
     NL_TRY(part_.alloc(sizeof(double) * (size_t)std::max(kSymvChunks * ld_, 4 * kRedCTAs)));
     NL_TRY(Linv_.alloc(sizeof(T) * (size_t)ntiles_ * NB * NB));
@@ -179,7 +178,7 @@ class SchurCoreT final : public SchurCore {
     NL_CUDA(cudaMemcpyAsync(env_dev_.p, env_first_.data(), sizeof(int) * ntiles_, cudaMemcpyHostToDevice, st_));
     NL_CUDA(cudaMemcpyAsync(env_dev_.as<int>() + ntiles_, env_last_.data(), sizeof(int) * ntiles_,
                             cudaMemcpyHostToDevice, st_));
-    NL_TRY(flags_.alloc(sizeof(int) * (size_t)(ntiles_ + 1)));
+    NL_TRY(flags_.alloc(sizeof(int) * (size_t)solve_flags()));
     NL_TRY(S_.alloc(sizeof(T) * (size_t)ld_ * ld_));
     s_cleared_ = false;
     need_s0_ = refine_sweeps > 0 || keep_schur;
@@ -278,22 +277,39 @@ class SchurCoreT final : public SchurCore {
     return NL_OK;
   }
 
-  // ---- solves with the factor: x = S^-1 b (trsv fwd + bwd) ----
-  nl_status enqueue_solve(const double* b, double* x, int* status, const int* active) {
-    NL_CUDA(cudaMemsetAsync(flags_.p, 0, flags_.bytes, st_));
+  // ---- solves with the factor (trsv fwd + bwd) ----
+  // Solve `k` of a call: 0: incU = S^-1 bS; k > 0: dx = S^-1 (bS - sum of the
+  // residual partials), incU += dx.  The first solve_slots() of a call have flags
+  // of their own (ticket + tile flags, forward and backward), which the call has
+  // cleared; later refinement sweeps clear and use them again.
+  nl_status enqueue_solve(int k, int* status, const int* active) {
     const int* env = envelope ? env_dev_.as<int>() : nullptr;
-    trsv_fwd_kernel<T><<<ntiles_, SV, trsv_smem<T>(), st_>>>(S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), b,
-                                                 y_.as<double>(),
-                                                 flags_.as<int>(), flags_.as<int>() + 1, 1, status, wait_limit, env,
-                                                 active);
-    NL_CUDA(cudaMemsetAsync(flags_.p, 0, flags_.bytes, st_));
-    trsv_bwd_kernel<T><<<ntiles_, SV, trsv_smem<T>(), st_>>>(S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(),
-                                                 y_.as<double>(), x,
-                                                 flags_.as<int>(), flags_.as<int>() + 1, 1, status, wait_limit, env,
-                                                 active);
+    const int nf = 2 * (ntiles_ + 1);
+    int* fl = flags_.as<int>() + (size_t)(k % solve_slots()) * nf;
+    if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(fl, 0, sizeof(int) * nf, st_));
+    trsv_fwd_kernel<T><<<ntiles_, SV, trsv_smem<T>(), st_>>>(
+        S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), k > 0 ? part_.as<double>() : nullptr,
+        kSymvChunks, y_.as<double>(), fl, fl + 1, 1, status, wait_limit, env, active);
+    fl += ntiles_ + 1;
+    trsv_bwd_kernel<T><<<ntiles_, SV, trsv_smem<T>(), st_>>>(
+        S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
+        k > 0 ? incU : nullptr, fl, fl + 1, 1, status, wait_limit, env, active);
     launches += 2;
     return NL_OK;
   }
+  // the solve and its refinement sweeps
+  nl_status enqueue_solves(int* status, const int* active) {
+    nl_status s = enqueue_solve(0, status, active);
+    for (int it = 0; it < refine_sweeps && need_s0_ && s == NL_OK; it++) {
+      symv_partial_kernel<T, kSymvChunks><<<dim3(ntiles_, kSymvChunks), SV, 0, st_>>>(
+          S0_.as<T>(), ld_, ntiles_, incU, part_.as<double>(), active);
+      launches++;
+      s = enqueue_solve(1 + it, status, active);
+    }
+    return s;
+  }
+  int solve_slots() const { return 1 + std::max(0, std::min(refine_sweeps, 3)); }
+  int solve_flags() const { return solve_slots() * 2 * (ntiles_ + 1); }
 
   // The forward solve with tile 0 left out: the ticket counter starts at 1,
   // so the ntiles - 1 CTAs take tiles 1 .. ntiles - 1 and each first waits
@@ -306,7 +322,7 @@ class SchurCoreT final : public SchurCore {
     NL_CUDA(cudaMemsetAsync(flags_.p, 0, flags_.bytes, st_));
     set_int_kernel<<<1, 1, 0, st_>>>(flags_.as<int>(), 1);
     trsv_fwd_kernel<T><<<ntiles_ - 1, SV, trsv_smem<T>(), st_>>>(S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(),
-                                                     bS_.as<double>(),
+                                                     bS_.as<double>(), nullptr, 0,
                                                      y_.as<double>(), flags_.as<int>(), flags_.as<int>() + 1, 1,
                                                      status, wait_limit, nullptr, nullptr);
     launches += 2;
@@ -700,7 +716,9 @@ class SchurCoreT final : public SchurCore {
     NvtxRange rg("nl:computeIncrement");
     if (tm) NL_CUDA(cudaEventRecord(ev_[0], st_));
     nvtxRangePushA("nl:vinv+wvinv_bs");
-    vinv_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, V_.as<T>(), Vinv_.as<T>(), lam, status, active);
+    vinv_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, V_.as<T>(), Vinv_.as<T>(), lam, status,
+                                                                     sched_.as<int>(), flags_.as<int>(), solve_flags(),
+                                                                     active);
     if (tm) NL_CUDA(cudaEventRecord(ev_[1], st_));
     if (nci_ > 0)
       wvinv_bs_kernel<T, BC, 128><<<nci_, 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
@@ -716,28 +734,20 @@ class SchurCoreT final : public SchurCore {
     // overflow that builds up there reaches tiles outside the envelope
     // (0 * inf).  That path clears all of S every time.
     const bool unpredicated_writes = sizeof(T) == 8 && cublas_ != nullptr;
-    if (!s_cleared_ || unpredicated_writes) {
-      NL_CUDA(cudaMemsetAsync(S_.p, 0, S_.bytes, st_));
-      if (need_s0_) NL_CUDA(cudaMemsetAsync(S0_.p, 0, S0_.bytes, st_));
-      s_cleared_ = true;
-    } else {
-      clear_envelope_kernel<T><<<ld_, 128, 0, st_>>>(S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr, ld_, NB,
-                                                     env_dev_.as<int>(), active);
-      launches++;
-    }
+    const bool full = !s_cleared_ || unpredicated_writes;  // not predicated
+    clear_kernel<T><<<ld_, 128, 0, st_>>>(S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr, n_, ld_, NB,
+                                          full ? nullptr : env_dev_.as<int>(), full ? nullptr : active);
+    s_cleared_ = true;
+    launches++;
     {
       using Cfg = SchurCfg<T, BC>;
       const int grid = std::max(1, std::min(cdiv(nitems_, Cfg::kWarps), 148 * schur_occ_));
-      NL_CUDA(cudaMemsetAsync(sched_.p, 0, sizeof(int), st_));
       schur_kernel<T, BC><<<grid, Cfg::kWarps * 32, Cfg::kSmem, st_>>>(
           d_, U_.as<T>(), Y_.as<T>(), W_.as<T>(), lam, S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr,
           s_items_.as<SchurItem>(), nitems_, chunk_, s_slot_.as<int>(), s_part_.as<T>(), sched_.as<int>() + 4,
           sched_.as<int>(), active);
-      if (ld_ > n_)
-        pad_identity_kernel<T><<<cdiv(ld_ - n_, 128), 128, 0, st_>>>(S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr, n_,
-                                                                     ld_, active);
     }
-    launches += 4;
+    launches += 3;
     nvtxRangePop();
     if (tm) NL_CUDA(cudaEventRecord(ev_[3], st_));
     nl_status s;
@@ -758,21 +768,11 @@ class SchurCoreT final : public SchurCore {
     if (s != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[4], st_));
     NvtxRange rs("nl:solve+backsub");
-    if ((s = enqueue_solve(bS_.as<double>(), incU, status, active)) != NL_OK) return s;
-    for (int it = 0; it < refine_sweeps && need_s0_; it++) {
-      symv_partial_kernel<T, kSymvChunks><<<dim3(ntiles_, kSymvChunks), SV, 0, st_>>>(
-          S0_.as<T>(), ld_, ntiles_, incU, part_.as<double>(), active);
-      resid_finalize_kernel<kSymvChunks><<<cdiv(ld_, 256), 256, 0, st_>>>(part_.as<double>(), bS_.as<double>(), ld_,
-                                                                          r_.as<double>(), active);
-      if ((s = enqueue_solve(r_.as<double>(), dx_.as<double>(), status, active)) != NL_OK) return s;
-      axpy_kernel<<<cdiv(ld_, 256), 256, 0, st_>>>(incU, dx_.as<double>(), ld_, active);
-      launches += 3;
-    }
+    if ((s = enqueue_solves(status, active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[5], st_));
-    zero_if_failed_kernel<<<cdiv(ld_, 256), 256, 0, st_>>>(incU, ld_, status, active);
     backsub_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
-                                                                      incU, incV, status, active);
-    launches += 2;
+                                                                      incU, ld_, incV, status, active);
+    launches++;
     if (tm) NL_CUDA(cudaEventRecord(ev_[6], st_));
     NL_CUDA(cudaGetLastError());
     if (tm) {
@@ -795,48 +795,40 @@ class SchurCoreT final : public SchurCore {
       wvinv_bs_kernel<T, BC, 128><<<nci_, 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
                                                          bV_.as<T>(), bS_.as<double>(), nullptr);
     launches++;
-    nl_status s = enqueue_solve(bS_.as<double>(), incU, status, nullptr);
+    NL_CUDA(cudaMemsetAsync(flags_.p, 0, flags_.bytes, st_));
+    nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
-    for (int it = 0; it < refine_sweeps && need_s0_; it++) {
-      symv_partial_kernel<T, kSymvChunks><<<dim3(ntiles_, kSymvChunks), SV, 0, st_>>>(
-          S0_.as<T>(), ld_, ntiles_, incU, part_.as<double>(), nullptr);
-      resid_finalize_kernel<kSymvChunks><<<cdiv(ld_, 256), 256, 0, st_>>>(part_.as<double>(), bS_.as<double>(), ld_,
-                                                                          r_.as<double>(), nullptr);
-      if ((s = enqueue_solve(r_.as<double>(), dx_.as<double>(), status, nullptr)) != NL_OK) return s;
-      axpy_kernel<<<cdiv(ld_, 256), 256, 0, st_>>>(incU, dx_.as<double>(), ld_, nullptr);
-      launches += 3;
-    }
-    zero_if_failed_kernel<<<cdiv(ld_, 256), 256, 0, st_>>>(incU, ld_, status, nullptr);
     backsub_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
-                                                                      incU, incV, status, nullptr);
-    launches += 2;
+                                                                      incU, ld_, incV, status, nullptr);
+    launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
   }
 
+  // sched_: [0] the Schur formation's work counter, [1 .. 3] last_block counts of
+  // the three reductions below, [4 ..] parts arrived per block
   nl_status enqueue_hdiag(double* out) override {
     const int grid = std::max(1, std::min(kRedCTAs, cdiv(nci_ + np_, 256)));
-    hdiag_kernel<T, BC><<<grid, 256, 0, st_>>>(U_.as<T>(), d_.u_diag_uid, nci_, V_.as<T>(), d_.v_uid, np_,
-                                               part_.as<double>());
-    max_finalize_kernel<<<1, 1, 0, st_>>>(part_.as<double>(), grid, out, nullptr);
-    launches += 2;
+    hdiag_kernel<T, BC, 256><<<grid, 256, 0, st_>>>(U_.as<T>(), d_.u_diag_uid, nci_, V_.as<T>(), d_.v_uid, np_,
+                                                    part_.as<double>(), sched_.as<int>() + 1, out);
+    launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
   }
 
   nl_status enqueue_maxabs_b(double* out, const int* active) override {
     const int grid = std::max(1, std::min(kRedCTAs, cdiv(n_ + 3 * np_, kNT)));
-    maxabs_kernel<T, kNT><<<grid, kNT, 0, st_>>>(bU_.as<T>(), n_, bV_.as<T>(), 3 * np_, part_.as<double>(), active);
-    max_finalize_kernel<<<1, 1, 0, st_>>>(part_.as<double>(), grid, out, active);
-    launches += 2;
+    maxabs_kernel<T, kNT><<<grid, kNT, 0, st_>>>(bU_.as<T>(), n_, bV_.as<T>(), 3 * np_, part_.as<double>(),
+                                                 sched_.as<int>() + 2, out, active);
+    launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
   }
 
-  nl_status enqueue_inc_dot(const LmDev* s, double* part, int* nparts) override {
+  nl_status enqueue_inc_dot(LmDev* s, double* part, double* trace) override {
     const int grid = std::max(1, std::min(kRedCTAs, cdiv(n_ + 3 * np_, kNT)));
-    inc_dot_kernel<T, kNT><<<grid, kNT, 0, st_>>>(incU, bU_.as<T>(), n_, incV, bV_.as<T>(), 3 * np_, s, part);
-    *nparts = grid;
+    inc_dot_kernel<T, kNT><<<grid, kNT, 0, st_>>>(incU, bU_.as<T>(), n_, incV, bV_.as<T>(), 3 * np_, s, part,
+                                                  sched_.as<int>() + 3, trace);
     launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
@@ -909,7 +901,7 @@ class SchurCoreT final : public SchurCore {
   int nitems_ = 0, chunk_ = 0, schur_occ_ = 1;  // work items of the Schur formation
   bool need_s0_ = false;
   SchurDev d_{};
-  DevBuf U_, V_, W_, Y_, Vinv_, bU_, bV_, bS_, incU_, incV_, y_, r_, dx_, part_, Linv_, hop_, flags_, S_, S0_, tcs_;
+  DevBuf U_, V_, W_, Y_, Vinv_, bU_, bV_, bS_, incU_, incV_, y_, dx_, part_, Linv_, hop_, flags_, S_, S0_, tcs_;
   // envelope of S (host) and its first / last arrays on the device (solves)
   std::vector<int> env_first_, env_last_, env_run_;
   DevBuf env_dev_;

@@ -88,7 +88,8 @@ class SchurCore {
   virtual nl_status enqueue_solve_withheld(int* status) = 0;
   virtual nl_status enqueue_hdiag(double* out) = 0;
   virtual nl_status enqueue_maxabs_b(double* out, const int* active) = 0;
-  virtual nl_status enqueue_inc_dot(const LmDev* s, double* part, int* nparts) = 0;
+  // |inc|^2, inc'(mu inc - b) and the sub-iteration's first decisions (lm_inc)
+  virtual nl_status enqueue_inc_dot(LmDev* s, double* part, double* trace) = 0;
   virtual int n() const = 0;
   virtual int ld() const = 0;
   virtual nl_status get_hessian(double* U, double* V, double* W, double* bU, double* bV) = 0;

@@ -46,9 +46,15 @@ struct SchurDev {
 // ---------------------------------------------------------------------------
 template <typename T, int BC>
 static __global__ void vinv_kernel(SchurDev d, const T* __restrict__ V, T* __restrict__ Vinv, const double* __restrict__ lam,
-                            int* __restrict__ status, const int* __restrict__ active) {
+                            int* __restrict__ status, int* __restrict__ counter, int* __restrict__ flags, int nflags,
+                            const int* __restrict__ active) {
   constexpr int LV = Layout<T, BC>::V;
   if (active && !*active) return;
+  // first kernel of a call: also clears the Schur work counter and the solves' flags
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) *counter = 0;
+    for (int i = threadIdx.x; i < nflags; i += blockDim.x) flags[i] = 0;
+  }
   const double rel = lam[0], abs = lam[1];
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= d.np) return;
@@ -373,48 +379,43 @@ static __global__ void __launch_bounds__(SchurCfg<T, BC>::kWarps * 32)
   }
 }
 
-// Zero the tiles of S (and S0) that can hold nonzeros: row r of tile row I
-// over columns [env_first[I] NB, (I + 1) NB) -- the Cholesky envelope.  The
-// other tiles are zero after the first full clear and stay exactly zero: the
-// Schur blocks lie inside the envelope, and the factorisation writes only
-// zeros there (TRSM and trailing updates of zero tiles).  One CTA per row.
+// Zero S (and S0), with the identity on the padded rows n .. ld - 1.  With
+// env_first only the tiles that can hold nonzeros: row r of tile row I over
+// columns [env_first[I] NB, (I + 1) NB), the Cholesky envelope.  The other tiles
+// are zero after the first full clear and stay exactly zero: the Schur blocks
+// lie inside the envelope, and the factorisation writes only zeros there (TRSM
+// and trailing updates of zero tiles).  One CTA per row.
 template <typename T>
-static __global__ void clear_envelope_kernel(T* __restrict__ S, T* __restrict__ S0, int ld, int nb,
-                                             const int* __restrict__ env_first, const int* __restrict__ active) {
+static __global__ void clear_kernel(T* __restrict__ S, T* __restrict__ S0, int n, int ld, int nb,
+                                    const int* __restrict__ env_first, const int* __restrict__ active) {
   if (active && !*active) return;
   const int r = blockIdx.x, I = r / nb;
-  const size_t c0 = (size_t)env_first[I] * nb, c1 = (size_t)(I + 1) * nb;
+  const size_t c0 = env_first ? (size_t)env_first[I] * nb : 0, c1 = env_first ? (size_t)(I + 1) * nb : (size_t)ld;
   constexpr int EPV = 16 / (int)sizeof(T);  // elements per 16-byte store
   using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  const V16 z = {};
   for (size_t c = c0 + (size_t)threadIdx.x * EPV; c < c1; c += (size_t)blockDim.x * EPV) {
-    *reinterpret_cast<V16*>(S + (size_t)r * ld + c) = z;
-    if (S0) *reinterpret_cast<V16*>(S0 + (size_t)r * ld + c) = z;
+    __align__(16) T z[EPV];
+#pragma unroll
+    for (int i = 0; i < EPV; i++) z[i] = r >= n && c + i == (size_t)r ? (T)1 : (T)0;
+    *reinterpret_cast<V16*>(S + (size_t)r * ld + c) = *reinterpret_cast<const V16*>(z);
+    if (S0) *reinterpret_cast<V16*>(S0 + (size_t)r * ld + c) = *reinterpret_cast<const V16*>(z);
   }
-}
-
-// Identity on the padded tail of S (rows n .. ld-1).
-template <typename T>
-static __global__ void pad_identity_kernel(T* __restrict__ S, T* __restrict__ S0, int n, int ld,
-                                    const int* __restrict__ active) {
-  if (active && !*active) return;
-  const int i = n + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ld) return;
-  S[(size_t)i * ld + i] = (T)1;
-  if (S0) S0[(size_t)i * ld + i] = (T)1;
 }
 
 // ---------------------------------------------------------------------------
 template <typename T, int BC>
 static __global__ void backsub_kernel(SchurDev d, const T* __restrict__ W, const T* __restrict__ Vinv,
-                               const T* __restrict__ bV, const double* __restrict__ xU, double* __restrict__ xV,
+                               const T* __restrict__ bV, double* xU, int nxu, double* __restrict__ xV,
                                const int* __restrict__ ok_flag, const int* __restrict__ active) {
   constexpr int LW = Layout<T, BC>::W;
   constexpr int LV = Layout<T, BC>::V;
   if (active && !*active) return;
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool failed = ok_flag && *ok_flag != 0;  // zero increment
+  if (failed)
+    for (int i = p; i < nxu; i += gridDim.x * blockDim.x) xU[i] = 0.0;
   if (p >= d.np) return;
-  if (ok_flag && *ok_flag != 0) {  // failed factorisation: zero increment
+  if (failed) {
     xV[3 * (size_t)p] = 0.0;
     xV[3 * (size_t)p + 1] = 0.0;
     xV[3 * (size_t)p + 2] = 0.0;
