@@ -359,11 +359,27 @@ __device__ inline void so3_log_dev(const double* R, double* w) {
   w[2] = f * v2;
 }
 
-static __global__ void cams_in_kernel(const double* __restrict__ in, double* __restrict__ state, int n, int bc,
-                                      double f_fixed) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// User parameters to the device layout: blocks [0, cam_blocks) convert kParamNT
+// cameras each, the others copy points (np3 values).  `in` and `pts_in` may be
+// pinned host memory: all accesses to them are coalesced, through shared memory
+// for the cameras.
+constexpr int kParamNT = 128;
+static __global__ void __launch_bounds__(kParamNT) params_in_kernel(const double* __restrict__ in,
+                                                                    double* __restrict__ state, int n, int bc,
+                                                                    double f_fixed, int cam_blocks,
+                                                                    const double* __restrict__ pts_in,
+                                                                    double* __restrict__ pts, int np3) {
+  if ((int)blockIdx.x >= cam_blocks) {
+    const int i = (blockIdx.x - cam_blocks) * kParamNT + threadIdx.x;
+    if (i < np3) pts[i] = pts_in[i];
+    return;
+  }
+  __shared__ double sh[kParamNT * 9];
+  const int c0 = blockIdx.x * kParamNT, c = c0 + threadIdx.x;
+  for (int i = threadIdx.x; i < min(kParamNT, n - c0) * bc; i += kParamNT) sh[i] = in[(size_t)c0 * bc + i];
+  __syncthreads();
   if (c >= n) return;
-  const double* a = in + (size_t)c * bc;
+  const double* a = sh + threadIdx.x * bc;
   double* s = state + (size_t)c * 16;
   double R[9];
   so3_exp(a, R);
@@ -383,24 +399,37 @@ static __global__ void cams_in_kernel(const double* __restrict__ in, double* __r
   s[15] = 0.0;
 }
 
-static __global__ void cams_out_kernel(const double* __restrict__ state, double* __restrict__ out, int n, int bc) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  const double* s = state + (size_t)c * 16;
-  double* o = out + (size_t)c * bc;
-  double w[3];
-  so3_log_dev(s, w);
-  o[0] = w[0];
-  o[1] = w[1];
-  o[2] = w[2];
-  o[3] = s[9];
-  o[4] = s[10];
-  o[5] = s[11];
-  if (bc == 9) {
-    o[6] = s[12];
-    o[7] = s[13];
-    o[8] = s[14];
+// The way back (params_in_kernel).
+static __global__ void __launch_bounds__(kParamNT) params_out_kernel(const double* __restrict__ state,
+                                                                     double* __restrict__ out, int n, int bc,
+                                                                     int cam_blocks, const double* __restrict__ pts,
+                                                                     double* __restrict__ pts_out, int np3) {
+  if ((int)blockIdx.x >= cam_blocks) {
+    const int i = (blockIdx.x - cam_blocks) * kParamNT + threadIdx.x;
+    if (i < np3) pts_out[i] = pts[i];
+    return;
   }
+  __shared__ double sh[kParamNT * 9];
+  const int c0 = blockIdx.x * kParamNT, c = c0 + threadIdx.x;
+  if (c < n) {
+    const double* s = state + (size_t)c * 16;
+    double* o = sh + threadIdx.x * bc;
+    double w[3];
+    so3_log_dev(s, w);
+    o[0] = w[0];
+    o[1] = w[1];
+    o[2] = w[2];
+    o[3] = s[9];
+    o[4] = s[10];
+    o[5] = s[11];
+    if (bc == 9) {
+      o[6] = s[12];
+      o[7] = s[13];
+      o[8] = s[14];
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < min(kParamNT, n - c0) * bc; i += kParamNT) out[(size_t)c0 * bc + i] = sh[i];
 }
 
 // dst[t] = src[order[t]] for observations (2 doubles) and weights.
