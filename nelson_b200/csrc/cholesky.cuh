@@ -1006,41 +1006,62 @@ __device__ inline void syrk_cc_tile(T* __restrict__ S, int ld, int k, int gI, in
 }
 
 // ---------------------------------------------------------------------------
-// Triangular solves with the tile inverses.  CTAs take tickets in tile order
-// (forward) or reverse order (backward); a CTA only waits on tiles whose
-// owners took earlier tickets, so every wait ends; each wait is also bounded.
-// 512 threads: warp w owns rows 8w..8w+7 of a 128-row tile, lane l owns
-// columns 4l..4l+3; partial dot products stay in registers across tiles and
-// are reduced once.
-// Flags are read with GPU-scope acquire loads and written with release
-// stores: the acquire that sees a tile's flag orders the waiting CTA's later
-// reads of that tile (after its barrier) behind the tile's writes.
-__device__ inline int load_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+// Triangular solves with the tile inverses, a chain of one hop per 128-row tile.
+// kSolveCtas CTAs per tile, 32 rows (backward: columns) each: a hop is bounded by
+// the product with a 128 x 128 matrix, which in FP64 arithmetic on one SM takes
+// 1 us (16 conversions and 38 FMAs per clock), and by the way of the result to
+// the next tile.  CTAs take tickets in tile order (forward) or reverse order
+// (backward); a CTA waits on tiles of earlier tickets and on its own tile's, so
+// with four CTAs on the chip every wait ends; each is also bounded.
+//
+// A value is passed on with the tag of its solve as one 16-byte store and load:
+// the reader that finds the tag has the value, without barrier, release, flag and
+// second load.  A tag is never used twice (a call's number and the solve within
+// it), so the packets are not cleared between calls.
+//
+// Per solve, one CTA per tile with flags -> now: 15 tiles FP32 33 -> 21.5 us, FP64
+// 42 -> 22 us, band of 47 tiles 92 -> 53 us, 106 tiles 240 -> 200 us (1.3 us per
+// hop, of which 0.7 us are the packet's way through L2; three hop matrices instead
+// of two change nothing).
+constexpr int kSolveCtas = 4, SVR = NB / kSolveCtas, SVT = 128;
+static_assert(SVT == NB && SVR == 8 * (SVT / 32), "a thread fetches one row, a warp finishes eight");
+
+__device__ inline void put_packet(ulonglong2* p, double v, unsigned long long tag) {
+  asm volatile("{\n.reg .b128 t;\nmov.b128 t, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 look_packet(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("{\n.reg .b128 t;\nld.relaxed.gpu.global.b128 t, [%2];\nmov.b128 {%0, %1}, t;\n}\n"
+               : "=l"(v.x), "=l"(v.y)
+               : "l"(p)
+               : "memory");
   return v;
 }
-static __device__ inline bool wait_flag(const int* flag, int epoch, int* status, long long limit) {
+
+// Fetches the 128 values at pk into dst (shared), one per thread; every thread of
+// the CTA calls it.  `seen`: what a look at the thread's packet gave earlier.
+// False after a wait that ran out.
+__device__ inline bool fetch_tile(const ulonglong2* __restrict__ pk, ulonglong2 seen, unsigned long long tag,
+                                  double* __restrict__ dst, int* __restrict__ status, long long limit) {
   long long it = 0;
-  while (load_acquire(flag) != epoch) {
-    if (++it > limit) {
-      atomicOr(status, ST_SPIN_TIMEOUT);
-      return false;
-    }
+  while (seen.y != tag && ++it <= limit) {
     if (it > 4096) __nanosleep(100);
+    seen = look_packet(pk + threadIdx.x);
   }
-  return true;
+  const bool bad = seen.y != tag;
+  if (bad) atomicOr(status, ST_SPIN_TIMEOUT);
+  dst[threadIdx.x] = __longlong_as_double(seen.x);
+  return !__syncthreads_or(bad);
 }
 
-// Publish a solved tile: the barrier orders every thread's writes of the
-// tile before thread 0's release store of the flag, which by cumulativity
-// orders them before the flag for every observer (one release per CTA).
-__device__ inline void publish_tile(int* flag, int epoch, int tid) {
-  __syncthreads();
-  if (tid == 0) asm volatile("st.release.gpu.global.b32 [%0], %1;\n" ::"l"(flag), "r"(epoch) : "memory");
+// Start of a call that solves without forming S: clears the solves' tickets (the
+// first forward solve hands out CTAs from `first` on) and numbers the call.
+static __global__ void solve_begin_kernel(int* tickets, int n, int first, unsigned long long* call) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) tickets[i] = i == 0 ? first : 0;
+  if (threadIdx.x == 0) (*call)++;
 }
-
-static __global__ void set_int_kernel(int* p, int v) { *p = v; }
 
 template <typename T>
 __device__ inline void load4(const T* p, double* v) {
@@ -1054,18 +1075,7 @@ __device__ inline void load4(const T* p, double* v) {
   }
 }
 
-__device__ inline void load4_cg(const double* p, double* v) {
-  const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-  const double2 b = __ldcg(reinterpret_cast<const double2*>(p + 2));
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-
 constexpr int SV = 512;
-template <typename T>
-constexpr size_t trsv_smem() {
-  return sizeof(T) * NB * NB;
-}
-
 // Four consecutive entries of an L row in the storage type (kept raw in
 // registers, widened to FP64 at the product).
 template <typename T>
@@ -1120,22 +1130,6 @@ __device__ __forceinline__ double reduce8(const double (&v)[8], int lane) {
   return c;
 }
 
-// The tiles a solve CTA reads before its own are published in ticket order,
-// so one wait is followed by a scan of the next flags: every tile found
-// published joins the confirmed range, which the CTA then streams without
-// further waits or barriers.  Thread 0 waits (bounded) on flag J and scans
-// forward (step +1, up to `end` exclusive) or backward (step -1); the result
-// is the first tile not confirmed, or `fail` after a timed-out wait.  The
-// acquire loads of thread 0 followed by the caller's barrier order every
-// thread's later reads of the confirmed tiles.
-__device__ inline int confirm_tiles(const int* flags, int J, int end, int step, int epoch, int* status,
-                                    long long limit, int fail) {
-  if (!wait_flag(flags + J, epoch, status, limit)) return fail;
-  int r = J + step;
-  while (r != end && load_acquire(flags + r) == epoch) r += step;
-  return r;
-}
-
 // The hop matrices of the solves, formed once per factorisation.  For the
 // d-th neighbour (d = 1 .. kHopDepth):
 //   M_d,I = Linv_I L_I,I-d                 (forward, I >= d)
@@ -1144,311 +1138,384 @@ __device__ inline int confirm_tiles(const int* flags, int J, int end, int step, 
 // backward.  With them y_I = c_I - sum_d M_d,I y_I-d, where c_I = Linv_I (b_I
 // - sum_{J < I - kHopDepth} L_IJ y_J) needs only tiles published kHopDepth
 // hops earlier, and likewise x_I = c'_I - sum_d Q_d,I x_I+d: after the wait
-// for its neighbour a solve CTA applies one register-resident 128 x 128
-// matrix.  Grid (ntiles - 1, 2 kHopDepth); products in T (FP32 for the mixed
-// factor, FP64 for the FP64 one), 8 x 8 outputs per thread.  A tile L outside
-// the envelope is zero, and so is its hop matrix.
+// for its neighbour a solve CTA applies one matrix that it has at hand.  Products
+// in T (FP32 for the mixed factor, FP64 for the FP64 one).  A tile L outside the
+// envelope is zero, and so is its hop matrix.  Grid (ntiles - 1, 2 kHopDepth, 4):
+// a 64 x 64 block per CTA, its operands staged in one go: with one CTA per
+// product the chip was idle (15 tiles: 54 CTAs) and every k step waited for memory
+// (15 tiles FP32 30 -> 11 us, FP64 45 -> 13 us, 106 tiles 78 -> 44 us).
 constexpr int kHopDepth = 2;
+
+// The eight rows x four columns of a matrix that a thread of a solve applies, in
+// shared memory: copied and read by that thread alone (no barrier, no conflict).
+template <typename T>
+struct OwnBlock {
+  static constexpr int kPieces = sizeof(T) / 4, kBytes = 8 * kPieces * SVT * 16;  // 16-byte pieces per row
+  char* p;
+  __device__ OwnBlock(void* smem, int i) : p((char*)smem + i * kBytes + threadIdx.x * 16) {}
+  __device__ __forceinline__ void stage(const T* src, size_t row_step) const {
+#pragma unroll
+    for (int i = 0; i < 8 * kPieces; i++)
+      cp_async16(p + i * SVT * 16, src + (i / kPieces) * row_step + (i % kPieces) * (16 / sizeof(T)));
+  }
+  __device__ __forceinline__ void row(int rr, double* v) const {
+    if (sizeof(T) == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p + rr * SVT * 16);
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+      const double2 a = *reinterpret_cast<const double2*>(p + 2 * rr * SVT * 16);
+      const double2 b = *reinterpret_cast<const double2*>(p + (2 * rr + 1) * SVT * 16);
+      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    }
+  }
+  // rows in the lanes' eight values, summed over the warp: the value of row
+  // reduce8_row(lane)
+  __device__ __forceinline__ double times(const double* x4, int lane) const {
+    double q[8];
+#pragma unroll
+    for (int rr = 0; rr < 8; rr++) {
+      double v[4];
+      row(rr, v);
+      q[rr] = v[0] * x4[0] + v[1] * x4[1] + v[2] * x4[2] + v[3] * x4[3];
+    }
+    return reduce8(q, lane);
+  }
+};
+template <typename T>
+constexpr size_t trsv_smem() {  // Linv_I and the hop matrices
+  return (size_t)(1 + kHopDepth) * OwnBlock<T>::kBytes;
+}
+constexpr int kHopB = 64, kHopLd = kHopB + 4;  // output block, row length of a staged block
+template <typename T>
+constexpr size_t hop_smem() {
+  return 4 * sizeof(T) * kHopB * kHopLd;
+}
 template <typename T>
 static __global__ void __launch_bounds__(256) hop_mat_kernel(const T* __restrict__ S, int ld, int ntiles,
-                                                            const T* __restrict__ Linv, T* __restrict__ hop,
-                                                            const int* __restrict__ active) {
-  constexpr int KC = 16;
-  __shared__ T As[KC][NB + 4];  // As[k][r] = A[r][k0 + k]
-  __shared__ T Bs[KC][NB + 4];  // Bs[k][c] = B[k0 + k][c]
+                                                             const T* __restrict__ Linv, T* __restrict__ hop,
+                                                             const int* __restrict__ active) {
+  extern __shared__ float4 hop_stage[];
+  T* sm = reinterpret_cast<T*>(hop_stage);  // [k half][A, B][kHopB][kHopLd]
   if (active && !*active) return;
   const bool fwd = blockIdx.y < kHopDepth;
   const int d = (int)(blockIdx.y % kHopDepth) + 1;
   // forward: I = d + x, tile (I, I - d); backward: I = x, tile (I + d, I)
   const int I = fwd ? d + (int)blockIdx.x : (int)blockIdx.x;
   if ((fwd && I >= ntiles) || (!fwd && I + d >= ntiles)) return;
+  const int br = (blockIdx.z >> 1) * kHopB, bc = (blockIdx.z & 1) * kHopB;  // first row, column of the product
   const T* Lt = fwd ? S + (size_t)I * NB * ld + (size_t)(I - d) * NB : S + (size_t)(I + d) * NB * ld + (size_t)I * NB;
   const T* A = fwd ? Linv + (size_t)I * NB * NB : Lt;
-  const size_t lda = fwd ? NB : (size_t)ld;
+  const int lda = fwd ? NB : ld;
   const T* B = fwd ? Lt : Linv + (size_t)I * NB * NB;
-  const size_t ldb = fwd ? (size_t)ld : NB;
+  const int ldb = fwd ? ld : NB;
+  // Linv is lower triangular: rows of A below 64 end at k = 64 (forward), columns
+  // of B from 64 on start there (backward)
+  const int h0 = !fwd && bc ? 1 : 0, h1 = fwd && !br ? 1 : 2;
   T* out = hop + ((size_t)blockIdx.y * ntiles + I) * NB * NB;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  T acc[8][8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int V = 16 / (int)sizeof(T), PV = kHopB / V;  // elements per copy, copies per row
 #pragma unroll
-  for (int i = 0; i < 8; i++)
-#pragma unroll
-    for (int j = 0; j < 8; j++) acc[i][j] = (T)0;
-  for (int k0 = 0; k0 < NB; k0 += KC) {
-    for (int e = tid; e < NB * KC; e += 256) {
-      const int r = e / KC, kk = e - r * KC;
-      As[kk][r] = A[(size_t)r * lda + k0 + kk];
-      const int kb = e / NB, c = e - kb * NB;
-      Bs[kb][c] = B[(size_t)(k0 + kb) * ldb + c];
+  for (int h = 0; h < 2; h++) {
+    if (h >= h0 && h < h1) {
+      T* As = sm + (2 * h) * kHopB * kHopLd;
+      T* Bs = As + kHopB * kHopLd;
+      for (int e = tid; e < kHopB * PV; e += 256) {
+        const int r = e / PV, c = (e % PV) * V;
+        cp_async16(As + r * kHopLd + c, A + (size_t)(br + r) * lda + h * kHopB + c);
+        cp_async16(Bs + r * kHopLd + c, B + (size_t)(h * kHopB + r) * ldb + bc + c);
+      }
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < KC; kk++) {
-      T a[8], bb[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 8; j++) bb[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] += a[i] * bb[j];
-    }
-    __syncthreads();
+    cp_async_commit();
   }
+  auto staged = [&](int h) {
+    if (h == 0)
+      cp_async_wait<1>();
+    else
+      cp_async_wait<0>();
+    __syncthreads();
+  };
+  if constexpr (sizeof(T) == 8) {
+    // warp: 32 rows x 16 columns, tensor-core FP64
+    const int wr = (warp >> 2) * 32, wc = (warp & 3) * 16, g = lane >> 2, t = lane & 3;
+    double acc[4][2][2] = {};
+    for (int h = h0; h < h1; h++) {
+      staged(h);
+      const T* As = sm + (2 * h) * kHopB * kHopLd + (wr + g) * kHopLd + t;
+      const T* Bs = sm + (2 * h + 1) * kHopB * kHopLd + t * kHopLd + wc + g;
+#pragma unroll 4
+      for (int k = 0; k < kHopB; k += 4) {
+        double a[4], b[2];
 #pragma unroll
-  for (int i = 0; i < 8; i++)
+        for (int i = 0; i < 4; i++) a[i] = As[8 * i * kHopLd + k];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int r = ty + 16 * i, c = tx + 16 * j;
-      if (fwd)
-        out[(size_t)r * NB + c] = acc[i][j];
-      else
-        out[(size_t)c * NB + r] = acc[i][j];
+        for (int j = 0; j < 2; j++) b[j] = Bs[k * kHopLd + 8 * j];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 2; j++) mma_f64(acc[i][j], a[i], b[j]);
+      }
     }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const int r = wr + 8 * i + g, c = wc + 8 * j + 2 * t + q;
+          sm[fwd ? r * kHopLd + c : c * kHopLd + r] = acc[i][j][q];
+        }
+  } else {
+    // thread: 4 rows x 4 columns
+    const int tx = tid & 15, ty = tid >> 4;
+    float acc[4][4] = {};
+    for (int h = h0; h < h1; h++) {
+      staged(h);
+      const float4* As = reinterpret_cast<const float4*>(sm + (2 * h) * kHopB * kHopLd);
+      const float4* Bs = reinterpret_cast<const float4*>(sm + (2 * h + 1) * kHopB * kHopLd);
+#pragma unroll 4
+      for (int k = 0; k < kHopB; k += 4) {
+        float4 a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) a[i] = As[((ty + 16 * i) * kHopLd + k) / 4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) b[q] = Bs[(k + q) * (kHopLd / 4) + tx];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            acc[i][0] += av[q] * b[q].x;
+            acc[i][1] += av[q] * b[q].y;
+            acc[i][2] += av[q] * b[q].z;
+            acc[i][3] += av[q] * b[q].w;
+          }
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int r = ty + 16 * i, c = 4 * tx + j;
+        sm[fwd ? r * kHopLd + c : c * kHopLd + r] = acc[i][j];
+      }
+  }
+  // rows of the result (backward: transposed), whole lines
+  __syncthreads();
+  out += fwd ? (size_t)br * NB + bc : (size_t)bc * NB + br;
+  for (int e = tid; e < kHopB * PV; e += 256) {
+    const int r = e / PV, c = (e % PV) * V;
+    *reinterpret_cast<float4*>(out + (size_t)r * NB + c) = *reinterpret_cast<const float4*>(sm + r * kHopLd + c);
+  }
 }
 
-// Forward solve L y = b by 128-row tiles.  CTA I (ticket order): streams the
-// tiles J < I - kHopDepth of its row as they are published, forms c_I =
-// Linv_I (b_I - partial) while its neighbours are still being solved, then
-// subtracts M_d,I y_I-d for d = kHopDepth .. 1, each as soon as that tile is
-// published.  b = the vector b less, if given, the nch partials `part` of a
-// refinement residual.  Thread (warp w, lane l) holds rows 8 w .. 8 w + 7, columns
-// 4 l .. 4 l + 3 of every 128 x 128 block it applies.
+// Forward solve L y = b.  A CTA of tile I streams the tiles J < I - kHopDepth of
+// its rows as they are published, passes b_I - partial to the CTAs of its tile,
+// subtracts M_d,I y_I-d for d = kHopDepth .. 2, adds c_I = Linv_I (b_I - partial)
+// and ends with M_1,I y_I-1.  b = the vector b less, if given, the nch partials
+// `part` of a refinement residual.  Warp w, lane l: rows 8 w .. 8 w + 7 of the
+// CTA's, columns 4 l .. 4 l + 3.  pk: 2 x 128 ntiles packets (y, b - partial).
 template <typename T>
-static __global__ void __launch_bounds__(SV) trsv_fwd_kernel(const T* __restrict__ L, int ld, int ntiles,
-                                                             const T* __restrict__ Linv,
-                                                             const T* __restrict__ hop,
-                                                             const double* __restrict__ b,
-                                                             const double* __restrict__ part, int nch,
-                                                             double* __restrict__ y,
-                                                             int* __restrict__ ticket, int* __restrict__ flags,
-                                                             int epoch, int* __restrict__ status,
-                                                             long long spin_limit,
-                                                             const int* __restrict__ env,
-                                                             const int* __restrict__ active) {
-  extern __shared__ float4 sLi4[];
-  T* sLi = reinterpret_cast<T*>(sLi4);  // Linv_I, NB x NB
-  __shared__ double acc[NB];
-  __shared__ int I_s, rdy_s[2];
+static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
+    const T* __restrict__ L, int ld, int ntiles, const T* __restrict__ Linv, const T* __restrict__ hop,
+    const double* __restrict__ b, const double* __restrict__ part, int nch, double* __restrict__ y,
+    int* __restrict__ ticket, ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub,
+    int* __restrict__ status, long long spin_limit, const int* __restrict__ env, const int* __restrict__ active) {
+  extern __shared__ float4 own4[];
+  __shared__ double got[2][NB];
+  __shared__ int t_s;
   if (active && !*active) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) I_s = atomicAdd(ticket, 1);
+  const unsigned long long tag = (*call << 32) | (unsigned)sub;
+  if (tid == 0) t_s = atomicAdd(ticket, 1);
   __syncthreads();
-  const int I = I_s;
-  {
-    const float4* src = reinterpret_cast<const float4*>(Linv + (size_t)I * NB * NB);
-    float4* dst = sLi4;
-    for (int i = tid; i < (int)(NB * NB * sizeof(T) / 16); i += SV) dst[i] = src[i];
-  }
-  double dots[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const T* Lrow = L + (size_t)(I * NB + warp * 8) * ld + 4 * lane;
-  // the right-hand side of the row this lane finishes, loaded now
-  const int rsel = warp * 8 + reduce8_row(lane);
-  double b_own = b[(size_t)I * NB + rsel];
+  const int I = t_s / kSolveCtas, r0 = (t_s % kSolveCtas) * SVR + warp * 8;
+  const size_t own = (size_t)r0 * NB + 4 * lane;
+  OwnBlock<T>(own4, 0).stage(Linv + (size_t)I * NB * NB + own, NB);
+#pragma unroll
+  for (int d = 1; d <= kHopDepth; d++)
+    if (I >= d) OwnBlock<T>(own4, d).stage(hop + ((size_t)(d - 1) * ntiles + I) * NB * NB + own, NB);
+  cp_async_commit();
+  // the right-hand side of the row this lane finishes
+  const size_t row = (size_t)I * NB + r0 + reduce8_row(lane);
+  double b_own = b[row];
   if (part)
-    for (int c = 0; c < nch; c++) b_own -= part[(size_t)c * ntiles * NB + (size_t)I * NB + rsel];
+    for (int c = 0; c < nch; c++) b_own -= part[(size_t)c * ntiles * NB + row];
   // with an envelope, the tiles of row I before its first nonzero are zero
   const int J0 = env ? env[I] : 0;
   const int Jend = I - kHopDepth;  // tiles [J0, Jend) are streamed, the last kHopDepth go through M_d,I
-  constexpr bool kPre = sizeof(T) == 4;  // FP32: the next tile loads while this one is used
-  Row4<T> cur[8], nxt[8];
-  if (J0 < Jend) {
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) cur[rr].load(Lrow + (size_t)rr * ld + (size_t)J0 * NB);
-  }
-  int ready = J0, par = 0;  // tiles [J0, ready) are confirmed published
-  auto catch_up = [&](int J) -> bool {  // uniform: every thread calls it with the same J
-    if (tid == 0) rdy_s[par] = confirm_tiles(flags, J, I, 1, epoch, status, spin_limit, -1);
-    __syncthreads();
-    ready = rdy_s[par];
-    par ^= 1;  // the other slot is written only after the next barrier
-    return ready >= 0;
+  int par = 0;
+  double x4[4];
+  auto fetch = [&](const ulonglong2* p, ulonglong2 seen) -> bool {  // uniform
+    const bool ok = fetch_tile(p, seen, tag, got[par], status, spin_limit);
+    load4(got[par] + 4 * lane, x4);
+    par ^= 1;  // the other buffer is written only after the next barrier
+    return ok;
   };
-  for (int J = J0; J < Jend; J++) {
-    if (kPre && J + 1 < Jend) {
+  const ulonglong2 none = make_ulonglong2(0, 0);  // call numbers start at 1
+  double dots[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (J0 < Jend) {
+    const T* Lrow = L + (size_t)(I * NB + r0) * ld + 4 * lane;
+    Row4<T> cur[8];
+    ulonglong2 seen = none;
+    for (int J = J0; J < Jend; J++) {
 #pragma unroll
-      for (int rr = 0; rr < 8; rr++) nxt[rr].load(Lrow + (size_t)rr * ld + (size_t)(J + 1) * NB);
-    }
-    if (J >= ready && !catch_up(J)) return;
-    double yv[4];
-    load4_cg(y + (size_t)J * NB + 4 * lane, yv);
+      for (int rr = 0; rr < 8; rr++) cur[rr].load(Lrow + (size_t)rr * ld + (size_t)J * NB);
+      const ulonglong2* p = pk + (size_t)J * NB;
+      const ulonglong2 now = seen;
+      if (J + 1 < Jend) seen = look_packet(p + NB + tid);
+      if (!fetch(p, now)) return;
 #pragma unroll
-    for (int rr = 0; rr < 8; rr++) dots[rr] += cur[rr].dot(yv);
-    if (kPre) {
-#pragma unroll
-      for (int rr = 0; rr < 8; rr++) cur[rr] = nxt[rr];
-    } else if (J + 1 < Jend) {
-#pragma unroll
-      for (int rr = 0; rr < 8; rr++) cur[rr].load(Lrow + (size_t)rr * ld + (size_t)(J + 1) * NB);
+      for (int rr = 0; rr < 8; rr++) dots[rr] += cur[rr].dot(x4);
     }
   }
-  // c_I = Linv_I (b_I - partial)
+  ulonglong2* pa = pk + (size_t)(ntiles + I) * NB;
   {
     const double sr = reduce8(dots, lane);
-    if ((lane & 3) == 0) acc[rsel] = b_own - sr;
+    if ((lane & 3) == 0) put_packet(pk + (size_t)ntiles * NB + row, b_own - sr, tag);
   }
-  __syncthreads();
-  const T* Li = sLi + (size_t)(warp * 8) * NB + 4 * lane;
-  double av[4] = {acc[4 * lane], acc[4 * lane + 1], acc[4 * lane + 2], acc[4 * lane + 3]};
-  double q8[8];
-#pragma unroll
-  for (int rr = 0; rr < 8; rr++) {
-    double lv[4];
-    load4(Li + (size_t)rr * NB, lv);
-    q8[rr] = lv[0] * av[0] + lv[1] * av[1] + lv[2] * av[2] + lv[3] * av[3];
-  }
-  double yr = reduce8(q8, lane);
-  // y_I = c_I - sum_d M_d,I y_I-d, nearest tile last
+  cp_async_wait<0>();
+  double yr = 0.0;
 #pragma unroll
   for (int d = kHopDepth; d >= 1; d--) {
+    if (d == 1) {
+      if (!fetch(pa, none)) return;
+      yr = OwnBlock<T>(own4, 0).times(x4, lane) - yr;
+    }
     const int J = I - d;
     if (J < 0 || J < J0) continue;  // outside the matrix or the envelope (uniform)
-    Row4<T> mrow[8];
-    const T* Mr = hop + ((size_t)(d - 1) * ntiles + I) * NB * NB + (size_t)(warp * 8) * NB + 4 * lane;
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) mrow[rr].load(Mr + (size_t)rr * NB);
-    if (J >= ready && !catch_up(J)) return;
-    double yv[4];
-    load4_cg(y + (size_t)J * NB + 4 * lane, yv);
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) q8[rr] = mrow[rr].dot(yv);
-    yr -= reduce8(q8, lane);
+    if (!fetch(pk + (size_t)J * NB, none)) return;
+    const double h = OwnBlock<T>(own4, d).times(x4, lane);
+    yr = d > 1 ? yr + h : yr - h;
   }
-  if ((lane & 3) == 0) y[(size_t)I * NB + rsel] = yr;
-  publish_tile(flags + I, epoch, tid);
+  if ((lane & 3) == 0) {
+    put_packet(pk + row, yr, tag);
+    y[row] = yr;
+  }
 }
 
-// Backward solve L' x = y.  CTA I (reverse ticket order): streams the tiles
-// J > I + kHopDepth of column I (rows of L_J,I) as they are published, forms
-// c'_I = Linv_I' (y_I - partial), then subtracts Q_d,I x_I+d for
-// d = kHopDepth .. 1 (Q_d,I row-major: row c is column c of L_I+d,I Linv_I,
-// so these steps have the forward kernel's row layout).  `sum`, if given, gets x
-// added (a refinement step).
+// Backward solve L' x = y.  A CTA of tile I streams the tiles J > I + kHopDepth of
+// its columns (rows of L_J,I), passes y_I - partial to the CTAs of its tile and
+// goes on as the forward solve with Q_d,I x_I+d (Q_d,I row-major: row c is column
+// c of L_I+d,I Linv_I) and c'_I = Linv_I' (y_I - partial).  For L_J,I and Linv_I a
+// thread holds rows 32 w + (l >> 3) + 4 i, columns 4 (l & 7) .. + 3 of the CTA's.
+// `sum`, if given, gets x added (a refinement step).
 template <typename T>
-static __global__ void __launch_bounds__(SV) trsv_bwd_kernel(const T* __restrict__ L, int ld, int ntiles,
-                                                             const T* __restrict__ Linv,
-                                                             const T* __restrict__ hop,
-                                                             const double* __restrict__ yv, double* __restrict__ x,
-                                                             double* __restrict__ sum,
-                                                             int* __restrict__ ticket, int* __restrict__ flags,
-                                                             int epoch, int* __restrict__ status,
-                                                             long long spin_limit,
-                                                             const int* __restrict__ env,
-                                                             const int* __restrict__ active) {
-  extern __shared__ float4 sLi4[];
-  T* sLi = reinterpret_cast<T*>(sLi4);  // Linv_I, NB x NB
-  __shared__ double red[SV / 32][NB];
-  __shared__ double acc[NB];
-  __shared__ int I_s, rdy_s[2];
+static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
+    const T* __restrict__ L, int ld, int ntiles, const T* __restrict__ Linv, const T* __restrict__ hop,
+    const double* __restrict__ yv, double* __restrict__ x, double* __restrict__ sum, int* __restrict__ ticket,
+    ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub, int* __restrict__ status,
+    long long spin_limit, const int* __restrict__ env, const int* __restrict__ active) {
+  extern __shared__ float4 own4[];
+  __shared__ double got[2][NB], red[SVT / 32][SVR];
+  __shared__ int t_s;
   if (active && !*active) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) I_s = ntiles - 1 - atomicAdd(ticket, 1);
+  const unsigned long long tag = (*call << 32) | (unsigned)sub;
+  if (tid == 0) t_s = atomicAdd(ticket, 1);
   __syncthreads();
-  const int I = I_s;
-  {
-    const float4* src = reinterpret_cast<const float4*>(Linv + (size_t)I * NB * NB);
-    float4* dst = sLi4;
-    for (int i = tid; i < (int)(NB * NB * sizeof(T) / 16); i += SV) dst[i] = src[i];
-  }
-  double part[4] = {0, 0, 0, 0};
-  const double y_own = tid < NB ? yv[(size_t)I * NB + tid] : 0.0;  // loaded off the chain
+  const int I = ntiles - 1 - t_s / kSolveCtas, q0 = (t_s % kSolveCtas) * SVR;
+  const int tr = 32 * warp + (lane >> 3), tc = q0 + 4 * (lane & 7);  // transposed blocks: first row, first column
+  OwnBlock<T>(own4, 0).stage(Linv + (size_t)I * NB * NB + (size_t)tr * NB + tc, 4 * NB);
+#pragma unroll
+  for (int d = 1; d <= kHopDepth; d++)
+    if (I + d < ntiles)
+      OwnBlock<T>(own4, d).stage(
+          hop + ((size_t)(kHopDepth + d - 1) * ntiles + I) * NB * NB + (size_t)(q0 + warp * 8) * NB + 4 * lane, NB);
+  cp_async_commit();
+  const double y_own = tid < SVR ? yv[(size_t)I * NB + q0 + tid] : 0.0;
   // with an envelope, the tiles of column I past its last nonzero are zero
   const int J1 = env ? env[ntiles + I] : ntiles - 1;
   const int Jend = I + kHopDepth;  // tiles (Jend, J1] are streamed, the nearest kHopDepth go through Q_d,I
-  const T* Lcol = L + (size_t)(warp * 8) * ld + (size_t)I * NB + 4 * lane;  // + J NB ld: tile (J, I)
-  constexpr bool kPre = sizeof(T) == 4;
-  Row4<T> cur[8], nxt[8];
-  if (J1 > Jend) {
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) cur[rr].load(Lcol + (size_t)(J1 * NB + rr) * ld);
-  }
-  int lo = J1 + 1, par = 0;  // tiles [lo, J1] are confirmed published
-  auto catch_up = [&](int J) -> bool {  // uniform
-    if (tid == 0) rdy_s[par] = confirm_tiles(flags, J, I, -1, epoch, status, spin_limit, -1) + 1;
-    __syncthreads();
-    lo = rdy_s[par];
+  int par = 0;
+  const double* v = nullptr;
+  auto fetch = [&](const ulonglong2* p, ulonglong2 seen) -> bool {  // uniform
+    const bool ok = fetch_tile(p, seen, tag, got[par], status, spin_limit);
+    v = got[par];
     par ^= 1;
-    return lo > 0;
+    return ok;
   };
-  for (int J = J1; J > Jend; J--) {
-    if (kPre && J - 1 > Jend) {
+  // the sum over a column's rows: the lanes of a column, then the warps (thread < SVR)
+  auto column_sum = [&](double (&p)[4]) -> double {
 #pragma unroll
-      for (int rr = 0; rr < 8; rr++) nxt[rr].load(Lcol + (size_t)((J - 1) * NB + rr) * ld);
+    for (int q = 0; q < 4; q++) {
+      p[q] += __shfl_xor_sync(0xffffffffu, p[q], 8);
+      p[q] += __shfl_xor_sync(0xffffffffu, p[q], 16);
     }
-    if (J < lo && !catch_up(J)) return;
+    if (lane < 8) {
 #pragma unroll
-    for (int rr = 0; rr < 8; rr++) {
-      const double xr = __ldcg(x + (size_t)J * NB + warp * 8 + rr);
-#pragma unroll
-      for (int q = 0; q < 4; q++) part[q] += cur[rr].at(q) * xr;
+      for (int q = 0; q < 4; q++) red[warp][4 * lane + q] = p[q];
     }
-    if (kPre) {
-#pragma unroll
-      for (int rr = 0; rr < 8; rr++) cur[rr] = nxt[rr];
-    } else if (J - 1 > Jend) {
-#pragma unroll
-      for (int rr = 0; rr < 8; rr++) cur[rr].load(Lcol + (size_t)((J - 1) * NB + rr) * ld);
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 4; q++) red[warp][4 * lane + q] = part[q];
-  __syncthreads();
-  if (tid < NB) {
+    __syncthreads();
     double s = 0.0;
+    if (tid < SVR) {
 #pragma unroll
-    for (int w = 0; w < SV / 32; w++) s += red[w][tid];
-    acc[tid] = y_own - s;
+      for (int w = 0; w < SVT / 32; w++) s += red[w][tid];
+    }
+    return s;
+  };
+  const ulonglong2 none = make_ulonglong2(0, 0);  // call numbers start at 1
+  double part[4] = {0, 0, 0, 0};
+  if (J1 > Jend) {
+    const T* Lcol = L + (size_t)tr * ld + (size_t)I * NB + tc;  // + J NB ld: tile (J, I)
+    Row4<T> cur[8];
+    ulonglong2 seen = none;
+    for (int J = J1; J > Jend; J--) {
+#pragma unroll
+      for (int rr = 0; rr < 8; rr++) cur[rr].load(Lcol + (size_t)(J * NB + 4 * rr) * ld);
+      const ulonglong2* p = pk + (size_t)J * NB;
+      const ulonglong2 now = seen;
+      if (J - 1 > Jend) seen = look_packet(p - NB + tid);
+      if (!fetch(p, now)) return;
+#pragma unroll
+      for (int rr = 0; rr < 8; rr++) {
+        const double xr = v[tr + 4 * rr];
+#pragma unroll
+        for (int q = 0; q < 4; q++) part[q] += cur[rr].at(q) * xr;
+      }
+    }
   }
-  __syncthreads();
-  // c'_I = Linv_I' acc : c'[c] = sum_r Linv[r][c] acc[r]
-  const T* Li = sLi + (size_t)(warp * 8) * NB + 4 * lane;
-  double p2[4] = {0, 0, 0, 0};
-#pragma unroll
-  for (int rr = 0; rr < 8; rr++) {
-    const double ar = acc[warp * 8 + rr];
-    double lv[4];
-    load4(Li + (size_t)rr * NB, lv);
-    p2[0] += lv[0] * ar;
-    p2[1] += lv[1] * ar;
-    p2[2] += lv[2] * ar;
-    p2[3] += lv[3] * ar;
+  {
+    const double s = column_sum(part);
+    if (tid < SVR) put_packet(pk + (size_t)(ntiles + I) * NB + q0 + tid, y_own - s, tag);
   }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 4; q++) red[warp][4 * lane + q] = p2[q];
-  __syncthreads();
-  if (tid < NB) {
-    double s = 0.0;
-#pragma unroll
-    for (int w = 0; w < SV / 32; w++) s += red[w][tid];
-    acc[tid] = s;  // c'_I
-  }
-  __syncthreads();
+  cp_async_wait<0>();
   const int rsel = warp * 8 + reduce8_row(lane);
-  double xr = acc[rsel];
-  // x_I = c'_I - sum_d Q_d,I x_I+d, nearest tile last
+  double xr = 0.0;
 #pragma unroll
   for (int d = kHopDepth; d >= 1; d--) {
+    if (d == 1) {
+      if (!fetch(pk + (size_t)(ntiles + I) * NB, none)) return;
+      double p2[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int rr = 0; rr < 8; rr++) {
+        const double ar = v[tr + 4 * rr];
+        double lv[4];
+        OwnBlock<T>(own4, 0).row(rr, lv);
+#pragma unroll
+        for (int q = 0; q < 4; q++) p2[q] += lv[q] * ar;
+      }
+      const double s = column_sum(p2);  // red: every thread has passed fetch's barrier since it was read
+      if (warp == 0) red[0][lane] = s;  // thread i alone reads and writes red[0][i] from here
+      __syncthreads();
+      xr = red[0][rsel] - xr;
+    }
     const int J = I + d;
     if (J >= ntiles || J > J1) continue;  // outside the matrix or the envelope (uniform)
-    Row4<T> qrow[8];
-    const T* Qr = hop + ((size_t)(kHopDepth + d - 1) * ntiles + I) * NB * NB + (size_t)(warp * 8) * NB + 4 * lane;
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) qrow[rr].load(Qr + (size_t)rr * NB);
-    if (J < lo && !catch_up(J)) return;
-    double xv[4];
-    load4_cg(x + (size_t)J * NB + 4 * lane, xv);
-    double q8[8];
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) q8[rr] = qrow[rr].dot(xv);
-    xr -= reduce8(q8, lane);
+    if (!fetch(pk + (size_t)J * NB, none)) return;
+    double x4[4];
+    load4(v + 4 * lane, x4);
+    const double h = OwnBlock<T>(own4, d).times(x4, lane);
+    xr = d > 1 ? xr + h : xr - h;
   }
   if ((lane & 3) == 0) {
-    x[(size_t)I * NB + rsel] = xr;
-    if (sum) sum[(size_t)I * NB + rsel] += xr;
+    const size_t row = (size_t)I * NB + q0 + rsel;
+    put_packet(pk + row, xr, tag);
+    x[row] = xr;
+    if (sum) sum[row] += xr;
   }
-  publish_tile(flags + I, epoch, tid);
 }
 
 // ---------------------------------------------------------------------------
@@ -1456,19 +1523,27 @@ static __global__ void __launch_bounds__(SV) trsv_bwd_kernel(const T* __restrict
 // (row tile I, chunk); a chunk covers a range of column tiles J.  For J < I
 // the tile S0_IJ is read row-wise (y_I += S0_IJ x_J), for J > I the tile
 // S0_JI is read row-wise and applied transposed (y_I += S0_JI' x_J); the
-// diagonal tile uses both halves.  Partials per chunk are summed in a fixed
+// diagonal tile uses both halves.  ENV: only the column tiles env[I] ..
+// env[ntiles + I] of the chunk, the others are zero (band of 47 tiles: 35 -> 14 us);
+// the dense form without these bounds is the faster code (106 tiles: 120 against
+// 144 us).  Partials per chunk are summed in a fixed
 // order by the forward solve that follows.
-template <typename T, int NCH>
+template <typename T, int NCH, bool ENV>
 static __global__ void __launch_bounds__(SV) symv_partial_kernel(const T* __restrict__ S0, int ld, int ntiles,
                                                                  const double* __restrict__ x,
                                                                  double* __restrict__ part,
+                                                                 const int* __restrict__ env,
                                                                  const int* __restrict__ active) {
   __shared__ double red[SV / 32][NB];
   if (active && !*active) return;
   const int I = blockIdx.x, ch = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int per = (ntiles + NCH - 1) / NCH;
-  const int J0 = ch * per, J1 = min(ntiles, J0 + per);
+  int J0 = ch * per, J1 = min(ntiles, J0 + per);
+  if (ENV) {
+    J0 = max(J0, env[I]);
+    J1 = min(J1, env[ntiles + I] + 1);
+  }
   double rp[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // rows 8 warp + rr
   double cp[4] = {0, 0, 0, 0};              // columns 4 lane + q
   for (int J = J0; J < J1; J++) {

@@ -178,7 +178,9 @@ class SchurCoreT final : public SchurCore {
     NL_CUDA(cudaMemcpyAsync(env_dev_.p, env_first_.data(), sizeof(int) * ntiles_, cudaMemcpyHostToDevice, st_));
     NL_CUDA(cudaMemcpyAsync(env_dev_.as<int>() + ntiles_, env_last_.data(), sizeof(int) * ntiles_,
                             cudaMemcpyHostToDevice, st_));
-    NL_TRY(flags_.alloc(sizeof(int) * (size_t)solve_flags()));
+    NL_TRY(tickets_.alloc(sizeof(int) * 2 * (size_t)solve_slots()));
+    NL_TRY(packets_.alloc(16 * (2 * (size_t)ld_ + 1)));
+    NL_CUDA(cudaMemsetAsync(packets_.p, 0, packets_.bytes, st_));
     NL_TRY(S_.alloc(sizeof(T) * (size_t)ld_ * ld_));
     s_cleared_ = false;
     need_s0_ = refine_sweeps > 0 || keep_schur;
@@ -249,6 +251,7 @@ class SchurCoreT final : public SchurCore {
                                  (int)trsm_tile_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(inv_tiles_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)inv_tiles_smem<T>()));
+    NL_CUDA(cudaFuncSetAttribute(hop_mat_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hop_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(trsv_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(trsv_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(diag_update_kernel<kChainRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -279,21 +282,20 @@ class SchurCoreT final : public SchurCore {
 
   // ---- solves with the factor (trsv fwd + bwd) ----
   // Solve `k` of a call: 0: incU = S^-1 bS; k > 0: dx = S^-1 (bS - sum of the
-  // residual partials), incU += dx.  The first solve_slots() of a call have flags
-  // of their own (ticket + tile flags, forward and backward), which the call has
-  // cleared; later refinement sweeps clear and use them again.
+  // residual partials), incU += dx.  The first solve_slots() of a call have
+  // tickets of their own (forward and backward), which the call has cleared;
+  // later refinement sweeps clear and use them again.
   nl_status enqueue_solve(int k, int* status, const int* active) {
     const int* env = envelope ? env_dev_.as<int>() : nullptr;
-    const int nf = 2 * (ntiles_ + 1);
-    int* fl = flags_.as<int>() + (size_t)(k % solve_slots()) * nf;
-    if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(fl, 0, sizeof(int) * nf, st_));
-    trsv_fwd_kernel<T><<<ntiles_, SV, trsv_smem<T>(), st_>>>(
+    int* tk = tickets_.as<int>() + 2 * (k % solve_slots());
+    if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(tk, 0, 2 * sizeof(int), st_));
+    const int grid = kSolveCtas * ntiles_;
+    trsv_fwd_kernel<T><<<grid, SVT, trsv_smem<T>(), st_>>>(
         S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), k > 0 ? part_.as<double>() : nullptr,
-        kSymvChunks, y_.as<double>(), fl, fl + 1, 1, status, wait_limit, env, active);
-    fl += ntiles_ + 1;
-    trsv_bwd_kernel<T><<<ntiles_, SV, trsv_smem<T>(), st_>>>(
+        kSymvChunks, y_.as<double>(), tk, packets(), call(), 2 * k, status, wait_limit, env, active);
+    trsv_bwd_kernel<T><<<grid, SVT, trsv_smem<T>(), st_>>>(
         S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
-        k > 0 ? incU : nullptr, fl, fl + 1, 1, status, wait_limit, env, active);
+        k > 0 ? incU : nullptr, tk + 1, packets(), call(), 2 * k + 1, status, wait_limit, env, active);
     launches += 2;
     return NL_OK;
   }
@@ -301,30 +303,31 @@ class SchurCoreT final : public SchurCore {
   nl_status enqueue_solves(int* status, const int* active) {
     nl_status s = enqueue_solve(0, status, active);
     for (int it = 0; it < refine_sweeps && need_s0_ && s == NL_OK; it++) {
-      symv_partial_kernel<T, kSymvChunks><<<dim3(ntiles_, kSymvChunks), SV, 0, st_>>>(
-          S0_.as<T>(), ld_, ntiles_, incU, part_.as<double>(), active);
+      auto symv = envelope ? symv_partial_kernel<T, kSymvChunks, true> : symv_partial_kernel<T, kSymvChunks, false>;
+      symv<<<dim3(ntiles_, kSymvChunks), SV, 0, st_>>>(S0_.as<T>(), ld_, ntiles_, incU, part_.as<double>(),
+                                                       env_dev_.as<int>(), active);
       launches++;
       s = enqueue_solve(1 + it, status, active);
     }
     return s;
   }
+  // [0] the call's number, then two packets per row
+  unsigned long long* call() const { return packets_.as<unsigned long long>(); }
+  ulonglong2* packets() const { return packets_.as<ulonglong2>() + 1; }
   int solve_slots() const { return 1 + std::max(0, std::min(refine_sweeps, 3)); }
-  int solve_flags() const { return solve_slots() * 2 * (ntiles_ + 1); }
 
-  // The forward solve with tile 0 left out: the ticket counter starts at 1,
-  // so the ntiles - 1 CTAs take tiles 1 .. ntiles - 1 and each first waits
-  // for tile 0's flag, which nothing publishes.  Every CTA's wait runs out
-  // after wait_limit polls, records ST_SPIN_TIMEOUT and returns before it
-  // writes anything; no access leaves the buffers (tiles 1 .. ntiles - 1 of
+  // The forward solve with tile 0 left out: the ticket counter starts at
+  // kSolveCtas, so the CTAs take tiles 1 .. ntiles - 1 and each waits for tile 0's
+  // packets, which nothing publishes.  Every CTA's wait runs out after wait_limit
+  // polls, records ST_SPIN_TIMEOUT and returns before it writes anything but
+  // packets of this call; no access leaves the buffers (tiles 1 .. ntiles - 1 of
   // L and Linv).
   nl_status enqueue_solve_withheld(int* status) override {
     if (ntiles_ < 2) return NL_ERR_STATE;
-    NL_CUDA(cudaMemsetAsync(flags_.p, 0, flags_.bytes, st_));
-    set_int_kernel<<<1, 1, 0, st_>>>(flags_.as<int>(), 1);
-    trsv_fwd_kernel<T><<<ntiles_ - 1, SV, trsv_smem<T>(), st_>>>(S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(),
-                                                     bS_.as<double>(), nullptr, 0,
-                                                     y_.as<double>(), flags_.as<int>(), flags_.as<int>() + 1, 1,
-                                                     status, wait_limit, nullptr, nullptr);
+    solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), 2 * solve_slots(), kSolveCtas, call());
+    trsv_fwd_kernel<T><<<kSolveCtas*(ntiles_ - 1), SVT, trsv_smem<T>(), st_>>>(
+        S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), nullptr, 0, y_.as<double>(),
+        tickets_.as<int>(), packets(), call(), 0, status, wait_limit, nullptr, nullptr);
     launches += 2;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
@@ -717,8 +720,8 @@ class SchurCoreT final : public SchurCore {
     if (tm) NL_CUDA(cudaEventRecord(ev_[0], st_));
     nvtxRangePushA("nl:vinv+wvinv_bs");
     vinv_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, V_.as<T>(), Vinv_.as<T>(), lam, status,
-                                                                     sched_.as<int>(), flags_.as<int>(), solve_flags(),
-                                                                     active);
+                                                                     sched_.as<int>(), tickets_.as<int>(),
+                                                                     2 * solve_slots(), call(), active);
     if (tm) NL_CUDA(cudaEventRecord(ev_[1], st_));
     if (nci_ > 0)
       wvinv_bs_kernel<T, BC, 128><<<nci_, 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
@@ -760,8 +763,8 @@ class SchurCoreT final : public SchurCore {
         launches++;
       }
       if (s == NL_OK && ntiles_ > 1) {
-        hop_mat_kernel<T><<<dim3(ntiles_ - 1, 2 * kHopDepth), 256, 0, st_>>>(S_.as<T>(), ld_, ntiles_, Linv_.as<T>(),
-                                                                             hop_.as<T>(), active);
+        hop_mat_kernel<T><<<dim3(ntiles_ - 1, 2 * kHopDepth, 4), 256, hop_smem<T>(), st_>>>(
+            S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), active);
         launches++;
       }
     }
@@ -795,7 +798,8 @@ class SchurCoreT final : public SchurCore {
       wvinv_bs_kernel<T, BC, 128><<<nci_, 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
                                                          bV_.as<T>(), bS_.as<double>(), nullptr);
     launches++;
-    NL_CUDA(cudaMemsetAsync(flags_.p, 0, flags_.bytes, st_));
+    solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), 2 * solve_slots(), 0, call());
+    launches++;
     nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
     backsub_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
@@ -901,7 +905,7 @@ class SchurCoreT final : public SchurCore {
   int nitems_ = 0, chunk_ = 0, schur_occ_ = 1;  // work items of the Schur formation
   bool need_s0_ = false;
   SchurDev d_{};
-  DevBuf U_, V_, W_, Y_, Vinv_, bU_, bV_, bS_, incU_, incV_, y_, dx_, part_, Linv_, hop_, flags_, S_, S0_, tcs_;
+  DevBuf U_, V_, W_, Y_, Vinv_, bU_, bV_, bS_, incU_, incV_, y_, dx_, part_, Linv_, hop_, tickets_, packets_, S_, S0_, tcs_;
   // envelope of S (host) and its first / last arrays on the device (solves)
   std::vector<int> env_first_, env_last_, env_run_;
   DevBuf env_dev_;

@@ -46,14 +46,18 @@ struct SchurDev {
 // ---------------------------------------------------------------------------
 template <typename T, int BC>
 static __global__ void vinv_kernel(SchurDev d, const T* __restrict__ V, T* __restrict__ Vinv, const double* __restrict__ lam,
-                            int* __restrict__ status, int* __restrict__ counter, int* __restrict__ flags, int nflags,
-                            const int* __restrict__ active) {
+                            int* __restrict__ status, int* __restrict__ counter, int* __restrict__ tickets, int ntickets,
+                            unsigned long long* __restrict__ call, const int* __restrict__ active) {
   constexpr int LV = Layout<T, BC>::V;
   if (active && !*active) return;
-  // first kernel of a call: also clears the Schur work counter and the solves' flags
+  // first kernel of a call: also clears the Schur work counter and the solves'
+  // tickets, and numbers the call
   if (blockIdx.x == 0) {
-    if (threadIdx.x == 0) *counter = 0;
-    for (int i = threadIdx.x; i < nflags; i += blockDim.x) flags[i] = 0;
+    if (threadIdx.x == 0) {
+      *counter = 0;
+      (*call)++;
+    }
+    for (int i = threadIdx.x; i < ntickets; i += blockDim.x) tickets[i] = 0;
   }
   const double rel = lam[0], abs = lam[1];
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
