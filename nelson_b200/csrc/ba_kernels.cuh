@@ -8,9 +8,9 @@
 //
 //   cost_kernel      one thread per edge, FP64 residual, chi2 per CTA; the last
 //                    CTA sums the partials in index order.
-//   cam_pass_kernel  one CTA per (internal) camera: edges in W-UID order,
+//   cam_pass_kernel  one or more CTAs per (internal) camera: edges in W-UID order,
 //                    writes each W block (J_c' J_p) and reduces U_c, bU_c.
-//   pt_pass_kernel   one thread per point: V_p, bV_p.
+//   pt_pass_kernel   four lanes per point: V_p, bV_p.
 #pragma once
 
 #include <type_traits>
@@ -154,16 +154,31 @@ static __global__ void __launch_bounds__(NT) sum_partials_kernel(const double* _
 
 // ---------------------------------------------------------------------------
 // Camera-major pass: U_c = sum w Jc'Jc, bU_c = sum w Jc'r, W_{c,p} = sum w Jc'Jp.
+// gridDim.y CTAs per camera (ctas_per_camera).  Bound by latency at three CTAs per
+// SM (168 registers; FP64 255): the next edge is fetched during this one, W leaves
+// through shared memory as whole lines.  200 cameras, 375k edges 36 -> 32 us, 432
+// cameras 73 -> 62 us, 1,500 cameras 245 -> 205 us; 256 threads were slower (38, 92,
+// 308 us).
+template <typename T, int BC, int NT>
+constexpr size_t cam_pass_smem() {
+  return sizeof(T) * NT * Layout<T, BC>::W;
+}
 template <typename T, int BC, int NT>
 static __global__ void __launch_bounds__(NT) cam_pass_kernel(BaDev d, T* __restrict__ U, T* __restrict__ W,
-                                                      T* __restrict__ bU, const int* __restrict__ active) {
+                                                      T* __restrict__ bU, T* __restrict__ part,
+                                                      int* __restrict__ count, const int* __restrict__ active) {
   constexpr int NU = BC * (BC + 1) / 2;  // upper triangle of U_c
   constexpr int NA = NU + BC;            // + bU_c
   constexpr int LW = Layout<T, BC>::W;
   constexpr int LU = Layout<T, BC>::U;
+  using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+  constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV;
+  extern __shared__ float4 w_out[];  // the warp's 32 W blocks, written as whole lines
   __shared__ double cs[16];
-  __shared__ T red[NT / 32][NA];
+  __shared__ T red[NT / 32][NA], total[NA];
   if (active && !*active) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  V16* st = reinterpret_cast<V16*>(w_out) + warp * 32 * PW;
   const int c = blockIdx.x;
   const int slot = d.cam_slot[c];
   if (threadIdx.x < 16) cs[threadIdx.x] = d.cam[(size_t)slot * 16 + threadIdx.x];
@@ -171,19 +186,45 @@ static __global__ void __launch_bounds__(NT) cam_pass_kernel(BaDev d, T* __restr
   T acc[NA];
 #pragma unroll
   for (int i = 0; i < NA; i++) acc[i] = (T)0;
-  const int g0 = d.cam_grp_ptr[c], g1 = d.cam_grp_ptr[c + 1];
-  for (int g = g0 + threadIdx.x; g < g1; g += NT) {
+  const int first = d.cam_grp_ptr[c], per = ((d.cam_grp_ptr[c + 1] - first + gridDim.y - 1) / gridDim.y + 31) & ~31;
+  const int g0 = first + blockIdx.y * per, g1 = min(d.cam_grp_ptr[c + 1], g0 + per);
+  // the next group's block and edges, and its first edge, are fetched while this
+  // one is evaluated
+  int wuid_n = -1, e_n = 0, e1_n = 0;
+  double X[3] = {0, 0, 1}, z0 = 0, z1 = 0, we = 0;
+  auto next_group = [&](int g) {
+    wuid_n = -1;
+    e_n = e1_n = 0;
+    if (g < g1) {
+      wuid_n = d.grp_wuid[g];
+      e_n = d.grp_edge_ptr[g];
+      e1_n = d.grp_edge_ptr[g + 1];
+    }
+  };
+  auto load_edge = [&](int e) {
+    const double* p = d.pt + (size_t)d.e_pt[e] * 3;
+    const double2 z = __ldg(reinterpret_cast<const double2*>(d.e_obs) + e);
+    X[0] = p[0];
+    X[1] = p[1];
+    X[2] = p[2];
+    z0 = z.x;
+    z1 = z.y;
+    we = d.e_w[e];
+  };
+  next_group(g0 + warp * 32 + lane);
+  if (e_n < e1_n) load_edge(e_n);
+  for (int gw = g0 + warp * 32; gw < g1; gw += NT) {
     T wacc[BC * 3];
 #pragma unroll
     for (int i = 0; i < BC * 3; i++) wacc[i] = (T)0;
-    const int wuid = d.grp_wuid[g];
-    for (int e = d.grp_edge_ptr[g]; e < d.grp_edge_ptr[g + 1]; e++) {
-      const double* X = d.pt + (size_t)d.e_pt[e] * 3;
+    const int wuid = wuid_n, e0 = e_n, e1 = e1_n;
+    next_group(gw + NT + lane);
+    for (int e = e0; e < e1; e++) {
+      if (e > e0) load_edge(e);
       double r0, r1;
       T Jc[2 * BC], Jp[6];
-      ba_project<T, BC, true, true>(cs, X, d.e_obs[2 * e], d.e_obs[2 * e + 1], d.f_fixed, d.cx, d.cy, r0,
-                                    r1, Jc, Jp);
-      const T w = (T)d.e_w[e];
+      ba_project<T, BC, true, true>(cs, X, z0, z1, d.f_fixed, d.cx, d.cy, r0, r1, Jc, Jp);
+      const T w = (T)we;
       const T wr0 = w * (T)r0, wr1 = w * (T)r1;
       int q = 0;
 #pragma unroll
@@ -203,31 +244,40 @@ static __global__ void __launch_bounds__(NT) cam_pass_kernel(BaDev d, T* __restr
         }
       }
     }
-    if (wuid >= 0) {
-      // 16-byte vector stores of the padded block
-      using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-      constexpr int EPV = 16 / (int)sizeof(T);
+    if (e_n < e1_n) load_edge(e_n);
+    {
       __align__(16) T blk[LW];
 #pragma unroll
       for (int i = 0; i < LW; i++) blk[i] = i < BC * 3 ? wacc[i] : (T)0;
 #pragma unroll
-      for (int i = 0; i < LW / EPV; i++)
-        reinterpret_cast<V16*>(W + (size_t)wuid * LW)[i] = reinterpret_cast<const V16*>(blk)[i];
+      for (int i = 0; i < PW; i++) st[lane * PW + i] = reinterpret_cast<const V16*>(blk)[i];
     }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < PW; i++) {
+      const int t = lane + 32 * i, u = __shfl_sync(0xffffffffu, wuid, t / PW);
+      if (u >= 0) reinterpret_cast<V16*>(W + (size_t)u * LW)[t % PW] = st[t];
+    }
+    __syncwarp();
   }
   // deterministic CTA reduction: warp shuffles, then warps in index order
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < NA; i++) {
     T v = warp_sum(acc[i]);
     if (lane == 0) red[warp][i] = v;
   }
   __syncthreads();
-  const int uid = d.cam_uid[c];
   for (int i = threadIdx.x; i < NA; i += NT) {
     T s = (T)0;
 #pragma unroll
     for (int w = 0; w < NT / 32; w++) s += red[w][i];
+    total[i] = s;
+  }
+  __syncthreads();
+  if (!item_total<NA>(total, part, count, c)) return;
+  const int uid = d.cam_uid[c];
+  for (int i = threadIdx.x; i < NA; i += NT) {
+    const T s = total[i];
     if (i < NU) {
       if (uid >= 0) {
         // map packed-upper index i -> (r, cc)
@@ -247,22 +297,35 @@ static __global__ void __launch_bounds__(NT) cam_pass_kernel(BaDev d, T* __restr
 }
 
 // ---------------------------------------------------------------------------
-// Point-major pass: V_p = sum w Jp'Jp, bV_p = sum w Jp'r.
+// Point-major pass: V_p = sum w Jp'Jp, bV_p = sum w Jp'r.  Four lanes per point, a
+// quarter of its edges each (consecutive lanes read consecutive edges); the camera
+// state, another line for every lane, comes in 16-byte loads.  Bound by the L1 lines
+// of that gather.  375k edges 30 -> 20 us, 1,500 cameras 233 -> 138 us.
 template <typename T, int BC, int NT>
 static __global__ void __launch_bounds__(NT) pt_pass_kernel(BaDev d, T* __restrict__ V, T* __restrict__ bV,
                                                      const int* __restrict__ active) {
   constexpr int LV = Layout<T, BC>::V;
   if (active && !*active) return;
-  const int p = blockIdx.x * NT + threadIdx.x;
-  if (p >= d.np_var) return;
+  const int t = blockIdx.x * NT + threadIdx.x, l = threadIdx.x & 3;
+  if ((t & ~31) >> 2 >= d.np_var) return;  // whole warps leave
+  const bool valid = t >> 2 < d.np_var;
+  const int p = valid ? t >> 2 : 0;
   const double X[3] = {d.pt[3 * (size_t)p], d.pt[3 * (size_t)p + 1], d.pt[3 * (size_t)p + 2]};
   T v[6] = {0, 0, 0, 0, 0, 0}, b[3] = {0, 0, 0};
-  for (int e = d.pt_edge_ptr[p]; e < d.pt_edge_ptr[p + 1]; e++) {
-    const double* cs = d.cam + (size_t)__ldg(d.p_cam + e) * 16;
+  const int e1 = valid ? d.pt_edge_ptr[p + 1] : 0;
+  for (int e = valid ? d.pt_edge_ptr[p] + l : 0; e < e1; e += 4) {
+    const double2* cam = reinterpret_cast<const double2*>(d.cam + (size_t)__ldg(d.p_cam + e) * 16);
+    double cs[16];
+#pragma unroll
+    for (int i = 0; i < (BC == 9 ? 8 : 6); i++) {
+      const double2 x = __ldg(cam + i);
+      cs[2 * i] = x.x;
+      cs[2 * i + 1] = x.y;
+    }
+    const double2 z = __ldg(reinterpret_cast<const double2*>(d.p_obs) + e);
     double r0, r1;
     T Jp[6];
-    ba_project<T, BC, false, true>(cs, X, __ldg(d.p_obs + 2 * e), __ldg(d.p_obs + 2 * e + 1), d.f_fixed, d.cx,
-                                   d.cy, r0, r1, nullptr, Jp);
+    ba_project<T, BC, false, true>(cs, X, z.x, z.y, d.f_fixed, d.cx, d.cy, r0, r1, nullptr, Jp);
     const T w = (T)__ldg(d.p_w + e);
     const T wr0 = w * (T)r0, wr1 = w * (T)r1;
     v[0] += w * (Jp[0] * Jp[0] + Jp[3] * Jp[3]);
@@ -275,6 +338,14 @@ static __global__ void __launch_bounds__(NT) pt_pass_kernel(BaDev d, T* __restri
     b[1] += Jp[1] * wr0 + Jp[4] * wr1;
     b[2] += Jp[2] * wr0 + Jp[5] * wr1;
   }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+#pragma unroll
+    for (int i = 0; i < 3; i++) b[i] += __shfl_xor_sync(0xffffffffu, b[i], o);
+  }
+  if (!valid || l != 0) return;
   const int uid = d.pt_vuid[p];
   if (uid >= 0) {
     T* o = V + (size_t)uid * LV;

@@ -50,6 +50,8 @@ struct nl_problem {
   std::vector<int> perm;  // user -> internal
   // structure
   int nU = 0, nV = 0, nW = 0, nci = 0, ngrp = 0;
+  int cam_ctas = 1;  // CTAs per camera of cam_pass_kernel; their sums, those finished
+  DevBuf d_cam_part, d_cam_count;
   std::vector<int> u_rc, v_rc, w_rc, h11, h12, h22;
   std::vector<int> eorder;   // device E-order -> insertion index
   std::vector<int> porder;   // device P-order -> insertion index
@@ -258,6 +260,10 @@ nl_status build_structure(nl_problem* h) {
     ss.w_c.push_back(h->w_rc[i + 1]);
   }
   NL_TRY(h->core->setup(ss, h->st));
+  h->cam_ctas = ctas_per_camera(h->nci, h->ngrp, kCamNT);
+  NL_TRY(h->d_cam_part.alloc(sizeof(double) * (size_t)std::max(h->nci, 1) * h->cam_ctas * (bc * (bc + 1) / 2 + bc)));
+  NL_TRY(h->d_cam_count.alloc(sizeof(int) * (size_t)std::max(h->nci, 1)));
+  NL_CUDA(cudaMemsetAsync(h->d_cam_count.p, 0, h->d_cam_count.bytes, h->st));
   BaDev& d = h->ba;
   d.bc = bc;
   d.nci = ncv;
@@ -301,11 +307,12 @@ nl_status enqueue_eval_t(nl_problem* h, bool hessian, double* chi2_out, double* 
   }
   if (hessian) {
     if (h->nci > 0)
-      cam_pass_kernel<T, BC, kCamNT><<<h->nci, kCamNT, 0, h->st>>>(h->ba, (T*)h->core->dU(), (T*)h->core->dW(),
-                                                                   (T*)h->core->dbU(), active);
+      cam_pass_kernel<T, BC, kCamNT><<<dim3(h->nci, h->cam_ctas), kCamNT, cam_pass_smem<T, BC, kCamNT>(), h->st>>>(
+          h->ba, (T*)h->core->dU(), (T*)h->core->dW(), (T*)h->core->dbU(), h->d_cam_part.as<T>(),
+          h->d_cam_count.as<int>(), active);
     if (h->desc.np_var > 0)
-      pt_pass_kernel<T, BC, 128><<<cdiv(h->desc.np_var, 128), 128, 0, h->st>>>(h->ba, (T*)h->core->dV(),
-                                                                                (T*)h->core->dbV(), active);
+      pt_pass_kernel<T, BC, 128><<<cdiv(4LL * h->desc.np_var, 128), 128, 0, h->st>>>(
+          h->ba, (T*)h->core->dV(), (T*)h->core->dbV(), active);
     h->launches += 2;
     nl_status s = h->core->enqueue_maxabs_b(maxb_out, active);
     if (s != NL_OK) return s;

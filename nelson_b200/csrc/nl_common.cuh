@@ -74,6 +74,42 @@ __device__ inline bool last_block(int* count) {
   return last != 0;
 }
 
+// The N sums (shared memory) of CTA blockIdx.y of the gridDim.y that share item c:
+// true for the CTA that finishes last, with the totals (added in CTA order) in
+// `sum`.  `part`: gridDim.y x N per item; `count`: zero per item, left at zero.
+template <int N, typename T>
+__device__ inline bool item_total(T* sum, T* __restrict__ part, int* __restrict__ count, int c) {
+  __shared__ int last;
+  const int n = gridDim.y;
+  if (n == 1) return true;
+  part += (size_t)c * n * N;
+  for (int i = threadIdx.x; i < N; i += blockDim.x) part[(size_t)blockIdx.y * N + i] = sum[i];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(count + c, 1) == n - 1;
+    if (last) count[c] = 0;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    T s = (T)0;
+    for (int y = 0; y < n; y++) s += __ldcg(part + (size_t)y * N + i);
+    sum[i] = s;
+  }
+  __syncthreads();
+  return true;
+}
+
+// CTAs per camera for a pass over a camera's observations with nt threads: four
+// CTAs per SM over the chip, two rounds of work at least for each.
+inline int ctas_per_camera(int nc, long long observations, int nt) {
+  const long long avg = observations / (nc > 0 ? nc : 1), want = (4 * 148 + nc - 1) / (nc > 0 ? nc : 1);
+  const long long n = want < avg / (2 * nt) ? want : avg / (2 * nt);
+  return (int)(n < 1 ? 1 : n > 8 ? 8 : n);
+}
+
 __device__ inline double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;

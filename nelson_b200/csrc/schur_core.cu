@@ -7,7 +7,7 @@ namespace nl {
 
 namespace {
 
-constexpr int kNT = 256;
+constexpr int kNT = 256, kWvNT = 256;
 constexpr int kRedCTAs = 296;  // 2 x 148 SMs for grid-stride reductions
 constexpr int kSymvChunks = 8;
 constexpr int kSchurMinChunk = 48, kSchurMaxChunk = 480;  // pairs of a Schur work item
@@ -251,6 +251,8 @@ class SchurCoreT final : public SchurCore {
                                  (int)trsm_tile_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(inv_tiles_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)inv_tiles_smem<T>()));
+    NL_CUDA(cudaFuncSetAttribute(wvinv_bs_kernel<T, BC, kWvNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)wvinv_smem<T, BC, kWvNT>()));
     NL_CUDA(cudaFuncSetAttribute(hop_mat_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hop_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(trsv_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
     NL_CUDA(cudaFuncSetAttribute(trsv_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
@@ -724,7 +726,7 @@ class SchurCoreT final : public SchurCore {
                                                                      2 * solve_slots(), call(), active);
     if (tm) NL_CUDA(cudaEventRecord(ev_[1], st_));
     if (nci_ > 0)
-      wvinv_bs_kernel<T, BC, 128><<<nci_, 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
+      wvinv_bs_kernel<T, BC, kWvNT><<<nci_, kWvNT, wvinv_smem<T, BC, kWvNT>(), st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
                                                          bV_.as<T>(), bS_.as<double>(), active);
     if (tm) NL_CUDA(cudaEventRecord(ev_[2], st_));
     nvtxRangePop();
@@ -773,7 +775,7 @@ class SchurCoreT final : public SchurCore {
     NvtxRange rs("nl:solve+backsub");
     if ((s = enqueue_solves(status, active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[5], st_));
-    backsub_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
+    backsub_kernel<T, BC><<<cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
                                                                       incU, ld_, incV, status, active);
     launches++;
     if (tm) NL_CUDA(cudaEventRecord(ev_[6], st_));
@@ -795,14 +797,14 @@ class SchurCoreT final : public SchurCore {
 
   nl_status enqueue_resolve(int* status) override {
     if (nci_ > 0)
-      wvinv_bs_kernel<T, BC, 128><<<nci_, 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
+      wvinv_bs_kernel<T, BC, kWvNT><<<nci_, kWvNT, wvinv_smem<T, BC, kWvNT>(), st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
                                                          bV_.as<T>(), bS_.as<double>(), nullptr);
     launches++;
     solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), 2 * solve_slots(), 0, call());
     launches++;
     nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
-    backsub_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
+    backsub_kernel<T, BC><<<cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
                                                                       incU, ld_, incV, status, nullptr);
     launches++;
     NL_CUDA(cudaGetLastError());

@@ -98,6 +98,16 @@ static __global__ void vinv_kernel(SchurDev d, const T* __restrict__ V, T* __res
 }
 
 // ---------------------------------------------------------------------------
+// One CTA per camera, one W block per lane.  The 32 blocks of a warp are
+// consecutive: they pass through shared memory so that every access to W and Y is
+// to whole lines (a lane reading its own 112 bytes takes 32 lines per access).
+// Bound by the L1 lines of the Vinv / bV gather.  375k blocks of 9x3 FP32 33 -> 24
+// us, FP64 65 -> 50 us, 1,500 cameras 338 -> 179 us; several CTAs per camera were
+// slower (28 us: the sums wait for the stores).
+template <typename T, int BC, int NT>
+constexpr size_t wvinv_smem() {
+  return sizeof(T) * NT * Layout<T, BC>::W;
+}
 template <typename T, int BC, int NT>
 static __global__ void __launch_bounds__(NT) wvinv_bs_kernel(SchurDev d, const T* __restrict__ W,
                                                       const T* __restrict__ Vinv, T* __restrict__ Y,
@@ -105,43 +115,63 @@ static __global__ void __launch_bounds__(NT) wvinv_bs_kernel(SchurDev d, const T
                                                       double* __restrict__ bS, const int* __restrict__ active) {
   constexpr int LW = Layout<T, BC>::W;
   constexpr int LV = Layout<T, BC>::V;
+  using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+  constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV;  // elements per piece, pieces per block
+  extern __shared__ float4 w_stage[];
   __shared__ double red[NT / 32][BC];
   if (active && !*active) return;
   const int c = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  V16* st = reinterpret_cast<V16*>(w_stage) + warp * 32 * PW;
   double acc[BC];
 #pragma unroll
   for (int i = 0; i < BC; i++) acc[i] = 0.0;
-  for (int q = d.w_row_ptr[c] + threadIdx.x; q < d.w_row_ptr[c + 1]; q += NT) {
-    const int p = d.w_col[q];
-    // blocks are padded to 16 bytes: move them as 16-byte vectors
-    using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-    constexpr int EPV = 16 / (int)sizeof(T);
-    __align__(16) T w[LW], v[LV], y[LW];
+  const int end = d.w_row_ptr[c + 1];
+  for (int q0 = d.w_row_ptr[c] + warp * 32; q0 < end; q0 += NT) {
+    const int m = min(32, end - q0);
+    const V16* src = reinterpret_cast<const V16*>(W + (size_t)q0 * LW);
 #pragma unroll
-    for (int i = 0; i < LW / EPV; i++)
-      reinterpret_cast<V16*>(w)[i] = __ldg(reinterpret_cast<const V16*>(W + (size_t)q * LW) + i);
+    for (int i = 0; i < PW; i++)
+      if (lane + 32 * i < m * PW) st[lane + 32 * i] = __ldg(src + lane + 32 * i);
+    __align__(16) T v[LV];
+    T bv0 = 0, bv1 = 0, bv2 = 0;
+    if (lane < m) {
+      const int p = d.w_col[q0 + lane];
 #pragma unroll
-    for (int i = 0; i < LV / EPV; i++)
-      reinterpret_cast<V16*>(v)[i] = __ldg(reinterpret_cast<const V16*>(Vinv + (size_t)p * LV) + i);
-    const T bv0 = bV[3 * (size_t)p], bv1 = bV[3 * (size_t)p + 1], bv2 = bV[3 * (size_t)p + 2];
-#pragma unroll
-    for (int i = 0; i < BC; i++) {
-      const T w0 = w[i * 3], w1 = w[i * 3 + 1], w2 = w[i * 3 + 2];
-      const T y0 = w0 * v[0] + w1 * v[3] + w2 * v[6];
-      const T y1 = w0 * v[1] + w1 * v[4] + w2 * v[7];
-      const T y2 = w0 * v[2] + w1 * v[5] + w2 * v[8];
-      y[i * 3] = y0;
-      y[i * 3 + 1] = y1;
-      y[i * 3 + 2] = y2;
-      acc[i] += (double)y0 * (double)bv0 + (double)y1 * (double)bv1 + (double)y2 * (double)bv2;
+      for (int i = 0; i < LV / EPV; i++)
+        reinterpret_cast<V16*>(v)[i] = __ldg(reinterpret_cast<const V16*>(Vinv + (size_t)p * LV) + i);
+      bv0 = bV[3 * (size_t)p];
+      bv1 = bV[3 * (size_t)p + 1];
+      bv2 = bV[3 * (size_t)p + 2];
     }
+    __syncwarp();
+    if (lane < m) {
+      __align__(16) T w[LW];
 #pragma unroll
-    for (int i = BC * 3; i < LW; i++) y[i] = (T)0;
+      for (int i = 0; i < PW; i++) reinterpret_cast<V16*>(w)[i] = st[lane * PW + i];
 #pragma unroll
-    for (int i = 0; i < LW / EPV; i++)
-      reinterpret_cast<V16*>(Y + (size_t)q * LW)[i] = reinterpret_cast<const V16*>(y)[i];
+      for (int i = 0; i < BC; i++) {
+        const T w0 = w[i * 3], w1 = w[i * 3 + 1], w2 = w[i * 3 + 2];
+        const T y0 = w0 * v[0] + w1 * v[3] + w2 * v[6];
+        const T y1 = w0 * v[1] + w1 * v[4] + w2 * v[7];
+        const T y2 = w0 * v[2] + w1 * v[5] + w2 * v[8];
+        w[i * 3] = y0;
+        w[i * 3 + 1] = y1;
+        w[i * 3 + 2] = y2;
+        acc[i] += (double)y0 * (double)bv0 + (double)y1 * (double)bv1 + (double)y2 * (double)bv2;
+      }
+#pragma unroll
+      for (int i = BC * 3; i < LW; i++) w[i] = (T)0;
+#pragma unroll
+      for (int i = 0; i < PW; i++) st[lane * PW + i] = reinterpret_cast<const V16*>(w)[i];
+    }
+    __syncwarp();
+    V16* dst = reinterpret_cast<V16*>(Y + (size_t)q0 * LW);
+#pragma unroll
+    for (int i = 0; i < PW; i++)
+      if (lane + 32 * i < m * PW) dst[lane + 32 * i] = st[lane + 32 * i];
+    __syncwarp();
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < BC; i++) {
     const double v = warp_sum(acc[i]);
@@ -407,47 +437,88 @@ static __global__ void clear_kernel(T* __restrict__ S, T* __restrict__ S0, int n
 }
 
 // ---------------------------------------------------------------------------
+// Eight lanes per point: lane l holds the 16-byte piece l of each of
+// the point's W blocks, so a block is read as one run.  FP64 sixteen lanes.  Bound
+// by the latency of the index chain (point -> W block -> camera).  375k blocks of
+// 9x3, a lane per point -> now: FP32 30 -> 22 us, FP64 49 -> 35 us; 1,500 cameras,
+// where W exceeds L2, 314 -> 178 us; 432 cameras, where it does not, 51 -> 63 us.
+// Half as many lanes: 33, 58, 190, 71 us.
+template <typename T>
+constexpr int kBackLanes = sizeof(T) == 4 ? 8 : 16;
 template <typename T, int BC>
-static __global__ void backsub_kernel(SchurDev d, const T* __restrict__ W, const T* __restrict__ Vinv,
-                               const T* __restrict__ bV, double* xU, int nxu, double* __restrict__ xV,
-                               const int* __restrict__ ok_flag, const int* __restrict__ active) {
+static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T* __restrict__ W,
+                                                             const T* __restrict__ Vinv, const T* __restrict__ bV,
+                                                             double* xU, int nxu, double* __restrict__ xV,
+                                                             const int* __restrict__ ok_flag,
+                                                             const int* __restrict__ active) {
   constexpr int LW = Layout<T, BC>::W;
   constexpr int LV = Layout<T, BC>::V;
+  using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+  constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV, LP = kBackLanes<T>, NP = (PW + LP - 1) / LP;
   if (active && !*active) return;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, l = threadIdx.x & (LP - 1);
   const bool failed = ok_flag && *ok_flag != 0;  // zero increment
-  if (failed)
-    for (int i = p; i < nxu; i += gridDim.x * blockDim.x) xU[i] = 0.0;
-  if (p >= d.np) return;
   if (failed) {
-    xV[3 * (size_t)p] = 0.0;
-    xV[3 * (size_t)p + 1] = 0.0;
-    xV[3 * (size_t)p + 2] = 0.0;
+    for (int i = t; i < nxu; i += gridDim.x * blockDim.x) xU[i] = 0.0;
+    for (int i = t; i < 3 * d.np; i += gridDim.x * blockDim.x) xV[i] = 0.0;
     return;
   }
-  double t0 = -(double)bV[3 * (size_t)p], t1 = -(double)bV[3 * (size_t)p + 1], t2 = -(double)bV[3 * (size_t)p + 2];
-  for (int s = d.w_col_ptr[p]; s < d.w_col_ptr[p + 1]; s++) {
-    const int q = d.w_col_uid[s];
-    const int c = d.w_row[q];
-    using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-    constexpr int EPV = 16 / (int)sizeof(T);
-    __align__(16) T w[LW];
+  const int p = t / LP;
+  if ((t & ~31) / LP >= d.np) return;  // whole warps leave
+  const bool valid = p < d.np;
+  const int s0 = valid ? d.w_col_ptr[p] : 0, s1 = valid ? d.w_col_ptr[p + 1] : 0;
+  // piece i of this lane: elements m0 = (l + LP i) EPV .., rows from m0 / 3 on; sum[i][r]
+  // collects W' x at component (m0 + r) % 3
+  double sum[NP][3] = {};
+  int most = s1 - s0;  // of the warp's points
 #pragma unroll
-    for (int i = 0; i < LW / EPV; i++)
-      reinterpret_cast<V16*>(w)[i] = __ldg(reinterpret_cast<const V16*>(W + (size_t)q * LW) + i);
-    const double* x = xU + (size_t)c * BC;
+  for (int o = LP; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+  for (int base = 0; base < most; base += LP) {
+    const int s = s0 + base + l;
+    const int ql = s < s1 ? d.w_col_uid[s] : -1;
+    const int cl = ql >= 0 ? d.w_row[ql] : 0;
+    const int cnt = min(LP, most - base);
+#pragma unroll 4
+    for (int e = 0; e < cnt; e++) {
+      const int q = __shfl_sync(0xffffffffu, ql, e, LP), c = __shfl_sync(0xffffffffu, cl, e, LP);
+      if (q < 0) continue;
+      const double* x = xU + (size_t)c * BC;
 #pragma unroll
-    for (int i = 0; i < BC; i++) {
-      const double xi = x[i];
-      t0 -= (double)w[i * 3] * xi;
-      t1 -= (double)w[i * 3 + 1] * xi;
-      t2 -= (double)w[i * 3 + 2] * xi;
+      for (int i = 0; i < NP; i++) {
+        const int pc = l + LP * i;
+        if (pc < PW) {
+          __align__(16) T w[EPV];
+          *reinterpret_cast<V16*>(w) = __ldg(reinterpret_cast<const V16*>(W + (size_t)q * LW) + pc);
+          const int m0 = pc * EPV, i0 = m0 / 3, k0 = m0 - 3 * i0;
+          const double xa = i0 < BC ? x[i0] : 0.0, xb = i0 + 1 < BC ? x[i0 + 1] : 0.0;
+#pragma unroll
+          for (int j = 0; j < EPV; j++)
+            if (m0 + j < 3 * BC) sum[i][j % 3] += (double)w[j] * (k0 + j < 3 ? xa : xb);
+        }
+      }
     }
   }
-  const T* v = Vinv + (size_t)p * LV;
-  xV[3 * (size_t)p] = (double)v[0] * t0 + (double)v[1] * t1 + (double)v[2] * t2;
-  xV[3 * (size_t)p + 1] = (double)v[3] * t0 + (double)v[4] * t1 + (double)v[5] * t2;
-  xV[3 * (size_t)p + 2] = (double)v[6] * t0 + (double)v[7] * t1 + (double)v[8] * t2;
+  double a[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+    const int k0 = (l + LP * i) * EPV % 3;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int r = k >= k0 ? k - k0 : k - k0 + 3;
+      a[k] += r == 0 ? sum[i][0] : r == 1 ? sum[i][1] : sum[i][2];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+#pragma unroll
+    for (int o = 1; o < LP; o <<= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+  }
+  if (valid && l < 3) {
+    const double t0 = -(double)bV[3 * (size_t)p] - a[0], t1 = -(double)bV[3 * (size_t)p + 1] - a[1],
+                 t2 = -(double)bV[3 * (size_t)p + 2] - a[2];
+    const T* v = Vinv + (size_t)p * LV + 3 * l;
+    xV[3 * (size_t)p + l] = (double)v[0] * t0 + (double)v[1] * t1 + (double)v[2] * t2;
+  }
 }
 
 }  // namespace nl
