@@ -115,6 +115,7 @@ template <int BC, int NT>
 static __global__ void __launch_bounds__(NT) cost_kernel(BaDev d, double* __restrict__ partial, int* __restrict__ count,
                                                   double* __restrict__ out, const int* __restrict__ active) {
   __shared__ double sh[NT / 32];
+  chain_start(active);
   if (active && !*active) return;
   double acc = 0.0;
   for (int e = blockIdx.x * NT + threadIdx.x; e < d.ne; e += gridDim.x * NT) {
@@ -176,6 +177,7 @@ static __global__ void __launch_bounds__(NT) cam_pass_kernel(BaDev d, T* __restr
   extern __shared__ float4 w_out[];  // the warp's 32 W blocks, written as whole lines
   __shared__ double cs[16];
   __shared__ T red[NT / 32][NA], total[NA];
+  chain_start(active);
   if (active && !*active) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   V16* st = reinterpret_cast<V16*>(w_out) + warp * 32 * PW;
@@ -305,6 +307,7 @@ template <typename T, int BC, int NT>
 static __global__ void __launch_bounds__(NT) pt_pass_kernel(BaDev d, T* __restrict__ V, T* __restrict__ bV,
                                                      const int* __restrict__ active) {
   constexpr int LV = Layout<T, BC>::V;
+  chain_start(active);
   if (active && !*active) return;
   const int t = blockIdx.x * NT + threadIdx.x, l = threadIdx.x & 3;
   if ((t & ~31) >> 2 >= d.np_var) return;  // whole warps leave
@@ -318,7 +321,7 @@ static __global__ void __launch_bounds__(NT) pt_pass_kernel(BaDev d, T* __restri
     double cs[16];
 #pragma unroll
     for (int i = 0; i < (BC == 9 ? 8 : 6); i++) {
-      const double2 x = __ldg(cam + i);
+      const double2 x = cam[i];
       cs[2 * i] = x.x;
       cs[2 * i + 1] = x.y;
     }
@@ -366,6 +369,7 @@ template <int BC>
 static __global__ void oplus_kernel(double* __restrict__ cam, const int* __restrict__ cam_slot_of_internal, int nci,
                                     const double* __restrict__ incU, int cam_blocks, double* __restrict__ pt,
                                     int np_var, const double* __restrict__ incV, const int* __restrict__ active) {
+  chain_start(incU, incV, active);
   if (active && !*active) return;
   if ((int)blockIdx.x >= cam_blocks) {
     const int i = (blockIdx.x - cam_blocks) * blockDim.x + threadIdx.x;

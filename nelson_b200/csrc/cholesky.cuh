@@ -24,14 +24,6 @@ namespace nl {
 constexpr int NB = 128;
 constexpr long long kSpinLimit = 1LL << 24;  // default bound of the flag waits (~1 s worst case)
 
-// Programmatic dependent launch of the critical-path chain (potrf -> row-tile
-// TRSM -> diagonal-tile update -> potrf ...): each kernel lets the next one in
-// its stream launch at its start, and waits for its predecessor's completion
-// (and memory flush) before touching what that predecessor wrote.  Both are
-// no-ops for a kernel launched without the attribute.
-__device__ inline void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ inline void chain_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-
 // ---------------------------------------------------------------------------
 // One CTA: factor the NB x NB diagonal tile of panel k in the storage
 // precision T (FP64 for the FP64 path; FP32 for the mixed path, whose
@@ -774,6 +766,7 @@ static __global__ void __launch_bounds__(512) inv_tiles_kernel(const T* __restri
   extern __shared__ float4 smf4[];
   const Sh<T> sl{(uint32_t)__cvta_generic_to_shared(smf4)};
   const Sh<T> sx = sl + kPBlocks * (kPBlocks + 1) / 2 * kInvBlk;
+  chain_start(S, active);
   if (active && !*active) return;
   const int k = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const Sh<T> st = sx + (kPBlocks * (kPBlocks + 1) / 2 * kInvBlk + w * PB * 12);
@@ -1196,6 +1189,7 @@ static __global__ void __launch_bounds__(256) hop_mat_kernel(const T* __restrict
                                                              const int* __restrict__ active) {
   extern __shared__ float4 hop_stage[];
   T* sm = reinterpret_cast<T*>(hop_stage);  // [k half][A, B][kHopB][kHopLd]
+  chain_start(S, Linv, active);
   if (active && !*active) return;
   const bool fwd = blockIdx.y < kHopDepth;
   const int d = (int)(blockIdx.y % kHopDepth) + 1;
@@ -1326,6 +1320,7 @@ static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
   extern __shared__ float4 own4[];
   __shared__ double got[2][NB];
   __shared__ int t_s;
+  chain_start(L, Linv, hop, b, part, call, active);
   if (active && !*active) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned long long tag = (*call << 32) | (unsigned)sub;
@@ -1411,6 +1406,7 @@ static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
   extern __shared__ float4 own4[];
   __shared__ double got[2][NB], red[SVT / 32][SVR];
   __shared__ int t_s;
+  chain_start(L, Linv, hop, yv, call, active);
   if (active && !*active) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned long long tag = (*call << 32) | (unsigned)sub;
@@ -1535,6 +1531,7 @@ static __global__ void __launch_bounds__(SV) symv_partial_kernel(const T* __rest
                                                                  const int* __restrict__ env,
                                                                  const int* __restrict__ active) {
   __shared__ double red[SV / 32][NB];
+  chain_start(S0, x, active);
   if (active && !*active) return;
   const int I = blockIdx.x, ch = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -68,6 +68,7 @@ static __global__ void __launch_bounds__(NT) inc_dot_kernel(const double* __rest
                                                      double* __restrict__ part, int* __restrict__ count,
                                                      double* __restrict__ trace) {
   __shared__ double sh[NT / 32];
+  chain_start(incU, bU, incV, bV);
   if (!s->active) return;
   const double mu = s->gn ? 0.0 : s->mu;
   double a = 0.0, b = 0.0;
@@ -134,6 +135,7 @@ __device__ inline void lm_inc(LmDev* s, double a, double b, double* trace) {
 
 // LevenbergMarquardt.hpp:78-129 (LM) / GaussNewton.hpp:89-123 (GN).
 static __global__ void lm_decide_kernel(LmDev* s, double* trace) {
+  chain_start();
   if (!s->active || s->done) return;
   if (s->gn) {
     // oplus + update(true) already ran: chi2_new and maxAbsB are current
@@ -206,6 +208,7 @@ __device__ inline void lm_after_jac(LmDev* s, double* chi2_out, double* trace) {
   }
 }
 static __global__ void lm_after_jac_kernel(LmDev* s, double* chi2_out, double* trace) {
+  chain_start();
   if (!s->active) return;
   if (s->do_jac) lm_after_jac(s, chi2_out, trace);
   lm_begin(s);
@@ -240,6 +243,7 @@ static __global__ void __launch_bounds__(NT) maxabs_kernel(const T* __restrict__
                                                     double* __restrict__ part, int* __restrict__ count,
                                                     double* __restrict__ out, const int* __restrict__ active) {
   __shared__ double sh[NT / 32];
+  chain_start(a, b, active);
   if (active && !*active) return;
   double m = 0.0;
   for (int i = blockIdx.x * NT + threadIdx.x; i < na + nb; i += gridDim.x * NT) {
@@ -275,6 +279,7 @@ static __global__ void __launch_bounds__(NT) hdiag_kernel(const T* __restrict__ 
 static __global__ void copy_if_kernel(double* __restrict__ dst, const double* __restrict__ src, size_t n,
                                       double* __restrict__ dst2, const double* __restrict__ src2, size_t n2,
                                       const int* __restrict__ flag) {
+  chain_start(src, src2, flag);
   if (flag && !*flag) return;
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = t; i < n; i += nt) dst[i] = src[i];

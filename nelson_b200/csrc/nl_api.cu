@@ -301,18 +301,19 @@ nl_status build_structure(nl_problem* h) {
 template <typename T, int BC>
 nl_status enqueue_eval_t(nl_problem* h, bool hessian, double* chi2_out, double* maxb_out, const int* active) {
   if (chi2_out) {
-    cost_kernel<BC, kCostNT><<<std::max(1, std::min(kCostCTAs, cdiv(h->ba.ne, kCostNT))), kCostNT, 0, h->st>>>(
-        h->ba, h->d_part.as<double>(), h->d_cnt.as<int>(), chi2_out, active);
+    NL_CUDA(launch_next(cost_kernel<BC, kCostNT>, dim3(std::max(1, std::min(kCostCTAs, cdiv(h->ba.ne, kCostNT)))),
+                        kCostNT, 0, h->st, h->core->pdl, h->ba, h->d_part.as<double>(), h->d_cnt.as<int>(), chi2_out, active));
     h->launches++;
   }
   if (hessian) {
     if (h->nci > 0)
-      cam_pass_kernel<T, BC, kCamNT><<<dim3(h->nci, h->cam_ctas), kCamNT, cam_pass_smem<T, BC, kCamNT>(), h->st>>>(
-          h->ba, (T*)h->core->dU(), (T*)h->core->dW(), (T*)h->core->dbU(), h->d_cam_part.as<T>(),
-          h->d_cam_count.as<int>(), active);
+      NL_CUDA(launch_next(cam_pass_kernel<T, BC, kCamNT>, dim3(h->nci, h->cam_ctas), kCamNT,
+                          cam_pass_smem<T, BC, kCamNT>(), h->st, h->core->pdl, h->ba, (T*)h->core->dU(), (T*)h->core->dW(),
+                          (T*)h->core->dbU(), h->d_cam_part.as<T>(), h->d_cam_count.as<int>(), active));
     if (h->desc.np_var > 0)
-      pt_pass_kernel<T, BC, 128><<<cdiv(4LL * h->desc.np_var, 128), 128, 0, h->st>>>(
-          h->ba, (T*)h->core->dV(), (T*)h->core->dbV(), active);
+      NL_CUDA(launch_next(pt_pass_kernel<T, BC, 128>, dim3(cdiv(4LL * h->desc.np_var, 128)), 128, 0, h->st,
+                          h->core->pdl,
+                          h->ba, (T*)h->core->dV(), (T*)h->core->dbV(), active));
     h->launches += 2;
     nl_status s = h->core->enqueue_maxabs_b(maxb_out, active);
     if (s != NL_OK) return s;
@@ -335,11 +336,11 @@ nl_status enqueue_oplus(nl_problem* h, const int* active) {
   const int cb = cdiv(h->nci, 256), grid = cb + cdiv(3LL * h->desc.np_var, 256);
   if (grid > 0) {
     if (h->desc.bc == 9)
-      oplus_kernel<9><<<grid, 256, 0, h->st>>>(h->cam.as<double>(), h->ba.cam_slot, h->nci, h->core->incU, cb,
-                                               h->pt.as<double>(), h->desc.np_var, h->core->incV, active);
+      NL_CUDA(launch_next(oplus_kernel<9>, dim3(grid), 256, 0, h->st, h->core->pdl, h->cam.as<double>(), h->ba.cam_slot,
+                          h->nci, h->core->incU, cb, h->pt.as<double>(), h->desc.np_var, h->core->incV, active));
     else
-      oplus_kernel<6><<<grid, 256, 0, h->st>>>(h->cam.as<double>(), h->ba.cam_slot, h->nci, h->core->incU, cb,
-                                               h->pt.as<double>(), h->desc.np_var, h->core->incV, active);
+      NL_CUDA(launch_next(oplus_kernel<6>, dim3(grid), 256, 0, h->st, h->core->pdl, h->cam.as<double>(), h->ba.cam_slot,
+                          h->nci, h->core->incU, cb, h->pt.as<double>(), h->desc.np_var, h->core->incV, active));
   }
   h->launches++;
   NL_CUDA(cudaGetLastError());
@@ -352,8 +353,8 @@ nl_status enqueue_copy_params(nl_problem* h, bool to_backup, const int* flag) {
   const double* c_src = to_backup ? h->cam.as<double>() : h->cam_bck.as<double>();
   double* p_dst = to_backup ? h->pt_bck.as<double>() : h->pt.as<double>();
   const double* p_src = to_backup ? h->pt.as<double>() : h->pt_bck.as<double>();
-  copy_if_kernel<<<std::max(1, std::min(592, cdiv(std::max(nc, np), 256))), 256, 0, h->st>>>(c_dst, c_src, nc, p_dst,
-                                                                                           p_src, np, flag);
+  NL_CUDA(launch_next(copy_if_kernel, dim3(std::max(1, std::min(592, cdiv(std::max(nc, np), 256)))), 256, 0, h->st,
+                      true, c_dst, c_src, nc, p_dst, p_src, np, flag));
   h->launches++;
   NL_CUDA(cudaGetLastError());
   return NL_OK;
@@ -367,12 +368,12 @@ nl_status enqueue_subiteration(nl_problem* h, double* trace) {
   if ((r = h->core->enqueue_inc_dot(s, h->d_part.as<double>() + 4096, trace)) != NL_OK) return r;
   if ((r = enqueue_oplus(h, &s->apply)) != NL_OK) return r;
   if ((r = enqueue_eval(h, false, &s->chi2_new, nullptr, &s->apply)) != NL_OK) return r;
-  lm_decide_kernel<<<1, 1, 0, h->st>>>(s, trace);
+  NL_CUDA(launch_next(lm_decide_kernel, dim3(1), 1, 0, h->st, h->core->pdl, s, trace));
   if ((r = enqueue_copy_params(h, false, &s->rollback)) != NL_OK) return r;
   // update(true) at the accepted point (GN: after every step), then backup
   if ((r = enqueue_eval(h, true, nullptr, &s->maxAbsB, &s->do_jac)) != NL_OK) return r;
   if ((r = enqueue_copy_params(h, true, &s->do_jac)) != NL_OK) return r;
-  lm_after_jac_kernel<<<1, 1, 0, h->st>>>(s, h->scal, trace);
+  NL_CUDA(launch_next(lm_after_jac_kernel, dim3(1), 1, 0, h->st, h->core->pdl, s, h->scal, trace));
   h->launches += 2;
   NL_CUDA(cudaGetLastError());
   return NL_OK;

@@ -8,6 +8,12 @@ namespace nl {
 namespace {
 
 constexpr int kNT = 256, kWvNT = 256;
+// Programmatic dependent launches up to this many W blocks: small systems are bound
+// by the 1.8 us between two kernels (20 cameras, 867 -> 718 us per solve; 64
+// cameras 1,590 -> 1,373 us); on large ones the CTAs that wait on the chip cost the
+// running kernels as much as is saved (200 cameras, 375k blocks: 8.85 / 8.87 ms,
+// FP64 12.8 / 13.0 ms).
+constexpr int kPdlBlocks = 1 << 16;
 constexpr int kRedCTAs = 296;  // 2 x 148 SMs for grid-stride reductions
 constexpr int kSymvChunks = 8;
 constexpr int kSchurMinChunk = 48, kSchurMaxChunk = 480;  // pairs of a Schur work item
@@ -158,6 +164,7 @@ class SchurCoreT final : public SchurCore {
   } while (0)
     NL_TRY(U_.alloc(sizeof(T) * (size_t)std::max(nU_, 1) * Layout<T, BC>::U));
     NL_TRY(V_.alloc(sizeof(T) * (size_t)std::max(nV_, 1) * Layout<T, BC>::V));
+    pdl = nW_ <= kPdlBlocks;
     NL_TRY(W_.alloc(sizeof(T) * (size_t)std::max(nW_, 1) * Layout<T, BC>::W));
     NL_TRY(Y_.alloc(sizeof(T) * (size_t)std::max(nW_, 1) * Layout<T, BC>::W));
     NL_TRY(Vinv_.alloc(sizeof(T) * (size_t)std::max(np_, 1) * Layout<T, BC>::V));
@@ -292,12 +299,15 @@ class SchurCoreT final : public SchurCore {
     int* tk = tickets_.as<int>() + 2 * (k % solve_slots());
     if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(tk, 0, 2 * sizeof(int), st_));
     const int grid = kSolveCtas * ntiles_;
-    trsv_fwd_kernel<T><<<grid, SVT, trsv_smem<T>(), st_>>>(
-        S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), k > 0 ? part_.as<double>() : nullptr,
-        kSymvChunks, y_.as<double>(), tk, packets(), call(), 2 * k, status, wait_limit, env, active);
-    trsv_bwd_kernel<T><<<grid, SVT, trsv_smem<T>(), st_>>>(
-        S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
-        k > 0 ? incU : nullptr, tk + 1, packets(), call(), 2 * k + 1, status, wait_limit, env, active);
+    NL_CUDA(launch_next(trsv_fwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl && !timing, S_.as<T>(), ld_,
+                        ntiles_,
+                        Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), k > 0 ? part_.as<double>() : nullptr,
+                        kSymvChunks, y_.as<double>(), tk, packets(), call(), 2 * k, status, wait_limit, env, active));
+    NL_CUDA(launch_next(trsv_bwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl && !timing, S_.as<T>(), ld_,
+                        ntiles_,
+                        Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
+                        k > 0 ? incU : nullptr, tk + 1, packets(), call(), 2 * k + 1, status, wait_limit, env,
+                        active));
     launches += 2;
     return NL_OK;
   }
@@ -306,8 +316,8 @@ class SchurCoreT final : public SchurCore {
     nl_status s = enqueue_solve(0, status, active);
     for (int it = 0; it < refine_sweeps && need_s0_ && s == NL_OK; it++) {
       auto symv = envelope ? symv_partial_kernel<T, kSymvChunks, true> : symv_partial_kernel<T, kSymvChunks, false>;
-      symv<<<dim3(ntiles_, kSymvChunks), SV, 0, st_>>>(S0_.as<T>(), ld_, ntiles_, incU, part_.as<double>(),
-                                                       env_dev_.as<int>(), active);
+      NL_CUDA(launch_next(symv, dim3(ntiles_, kSymvChunks), SV, 0, st_, pdl && !timing, S0_.as<T>(), ld_, ntiles_, incU,
+                          part_.as<double>(), env_dev_.as<int>(), active));
       launches++;
       s = enqueue_solve(1 + it, status, active);
     }
@@ -411,22 +421,10 @@ class SchurCoreT final : public SchurCore {
     return NL_OK;
   }
 
-  // A kernel on the main stream; with pdl, as a programmatic dependent of the
-  // stream's preceding kernel (it may start before that one ends and waits
-  // for it with griddepcontrol.wait).
+  // A kernel on the main stream (launch_next)
   template <typename... KArgs, typename... Args>
-  cudaError_t launch_chain(void (*kern)(KArgs...), int grid, int block, size_t smem, bool pdl, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st_;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
+  cudaError_t launch_chain(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, bool pdl, Args... args) {
+    return launch_next(kern, grid, block, smem, st_, pdl, args...);
   }
 
   uint8_t* pack_slot(int k) const { return static_cast<uint8_t*>(tcs_.p) + (size_t)(k % kPackSlots) * tcs_half_; }
@@ -533,8 +531,8 @@ class SchurCoreT final : public SchurCore {
     auto potrf = [&](int j) -> nl_status {
       const int e = 8 * nT + 2 * j;  // timing events after the update events
       if (tmc) cudaEventRecord(upd_ev_[e], st_);
-      // a programmatic dependent of the diagonal update before it
-      NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, potrf_smem<T>(), j > 0 && !tmc, S_.as<T>(), ld_, j,
+      // a programmatic dependent of the Schur formation or the diagonal update before it
+      NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, potrf_smem<T>(), (j > 0 || pdl) && !tmc, S_.as<T>(), ld_, j,
                            Linv_.as<T>(), status, active));
       if (tmc) cudaEventRecord(upd_ev_[e + 1], st_);
       npev = j + 1;
@@ -721,13 +719,14 @@ class SchurCoreT final : public SchurCore {
     NvtxRange rg("nl:computeIncrement");
     if (tm) NL_CUDA(cudaEventRecord(ev_[0], st_));
     nvtxRangePushA("nl:vinv+wvinv_bs");
-    vinv_kernel<T, BC><<<cdiv(std::max(np_, 1), 128), 128, 0, st_>>>(d_, V_.as<T>(), Vinv_.as<T>(), lam, status,
-                                                                     sched_.as<int>(), tickets_.as<int>(),
-                                                                     2 * solve_slots(), call(), active);
+    NL_CUDA(launch_next(vinv_kernel<T, BC>, dim3(cdiv(std::max(np_, 1), 128)), 128, 0, st_, pdl && !tm, d_, V_.as<T>(),
+                        Vinv_.as<T>(), lam, status, sched_.as<int>(), tickets_.as<int>(), 2 * solve_slots(), call(),
+                        active));
     if (tm) NL_CUDA(cudaEventRecord(ev_[1], st_));
     if (nci_ > 0)
-      wvinv_bs_kernel<T, BC, kWvNT><<<nci_, kWvNT, wvinv_smem<T, BC, kWvNT>(), st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
-                                                         bV_.as<T>(), bS_.as<double>(), active);
+      NL_CUDA(launch_next(wvinv_bs_kernel<T, BC, kWvNT>, dim3(nci_), kWvNT, wvinv_smem<T, BC, kWvNT>(), st_,
+                          pdl && !tm, d_,
+                          W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(), bV_.as<T>(), bS_.as<double>(), active));
     if (tm) NL_CUDA(cudaEventRecord(ev_[2], st_));
     nvtxRangePop();
     nvtxRangePushA("nl:schur");
@@ -740,17 +739,19 @@ class SchurCoreT final : public SchurCore {
     // (0 * inf).  That path clears all of S every time.
     const bool unpredicated_writes = sizeof(T) == 8 && cublas_ != nullptr;
     const bool full = !s_cleared_ || unpredicated_writes;  // not predicated
-    clear_kernel<T><<<ld_, 128, 0, st_>>>(S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr, n_, ld_, NB,
-                                          full ? nullptr : env_dev_.as<int>(), full ? nullptr : active);
+    NL_CUDA(launch_next(clear_kernel<T>, dim3(ld_), 128, 0, st_, pdl && !tm, S_.as<T>(),
+                        need_s0_ ? S0_.as<T>() : nullptr, n_,
+                        ld_, NB, full ? nullptr : env_dev_.as<int>(), full ? nullptr : active));
     s_cleared_ = true;
     launches++;
     {
       using Cfg = SchurCfg<T, BC>;
       const int grid = std::max(1, std::min(cdiv(nitems_, Cfg::kWarps), 148 * schur_occ_));
-      schur_kernel<T, BC><<<grid, Cfg::kWarps * 32, Cfg::kSmem, st_>>>(
-          d_, U_.as<T>(), Y_.as<T>(), W_.as<T>(), lam, S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr,
-          s_items_.as<SchurItem>(), nitems_, chunk_, s_slot_.as<int>(), s_part_.as<T>(), sched_.as<int>() + 4,
-          sched_.as<int>(), active);
+      NL_CUDA(launch_next(schur_kernel<T, BC>, dim3(grid), Cfg::kWarps * 32, Cfg::kSmem, st_, pdl && !tm, d_,
+                          U_.as<T>(),
+                          Y_.as<T>(), W_.as<T>(), lam, S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr,
+                          s_items_.as<SchurItem>(), nitems_, chunk_, s_slot_.as<int>(), s_part_.as<T>(),
+                          sched_.as<int>() + 4, sched_.as<int>(), active));
     }
     launches += 3;
     nvtxRangePop();
@@ -765,8 +766,8 @@ class SchurCoreT final : public SchurCore {
         launches++;
       }
       if (s == NL_OK && ntiles_ > 1) {
-        hop_mat_kernel<T><<<dim3(ntiles_ - 1, 2 * kHopDepth, 4), 256, hop_smem<T>(), st_>>>(
-            S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), active);
+        NL_CUDA(launch_next(hop_mat_kernel<T>, dim3(ntiles_ - 1, 2 * kHopDepth, 4), 256, hop_smem<T>(), st_, pdl && !tm,
+                            S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), active));
         launches++;
       }
     }
@@ -775,8 +776,8 @@ class SchurCoreT final : public SchurCore {
     NvtxRange rs("nl:solve+backsub");
     if ((s = enqueue_solves(status, active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[5], st_));
-    backsub_kernel<T, BC><<<cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
-                                                                      incU, ld_, incV, status, active);
+    NL_CUDA(launch_next(backsub_kernel<T, BC>, dim3(cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128)), 128, 0,
+                        st_, pdl && !tm, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status, active));
     launches++;
     if (tm) NL_CUDA(cudaEventRecord(ev_[6], st_));
     NL_CUDA(cudaGetLastError());
@@ -797,15 +798,15 @@ class SchurCoreT final : public SchurCore {
 
   nl_status enqueue_resolve(int* status) override {
     if (nci_ > 0)
-      wvinv_bs_kernel<T, BC, kWvNT><<<nci_, kWvNT, wvinv_smem<T, BC, kWvNT>(), st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(),
-                                                         bV_.as<T>(), bS_.as<double>(), nullptr);
+      NL_CUDA(launch_next(wvinv_bs_kernel<T, BC, kWvNT>, dim3(nci_), kWvNT, wvinv_smem<T, BC, kWvNT>(), st_, pdl, d_,
+                          W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(), bV_.as<T>(), bS_.as<double>(), nullptr));
     launches++;
     solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), 2 * solve_slots(), 0, call());
     launches++;
     nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
-    backsub_kernel<T, BC><<<cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128), 128, 0, st_>>>(d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(),
-                                                                      incU, ld_, incV, status, nullptr);
+    NL_CUDA(launch_next(backsub_kernel<T, BC>, dim3(cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128)), 128, 0,
+                        st_, pdl, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status, nullptr));
     launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
@@ -824,8 +825,8 @@ class SchurCoreT final : public SchurCore {
 
   nl_status enqueue_maxabs_b(double* out, const int* active) override {
     const int grid = std::max(1, std::min(kRedCTAs, cdiv(n_ + 3 * np_, kNT)));
-    maxabs_kernel<T, kNT><<<grid, kNT, 0, st_>>>(bU_.as<T>(), n_, bV_.as<T>(), 3 * np_, part_.as<double>(),
-                                                 sched_.as<int>() + 2, out, active);
+    NL_CUDA(launch_next(maxabs_kernel<T, kNT>, dim3(grid), kNT, 0, st_, pdl, bU_.as<T>(), n_, bV_.as<T>(), 3 * np_,
+                        part_.as<double>(), sched_.as<int>() + 2, out, active));
     launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
@@ -833,8 +834,8 @@ class SchurCoreT final : public SchurCore {
 
   nl_status enqueue_inc_dot(LmDev* s, double* part, double* trace) override {
     const int grid = std::max(1, std::min(kRedCTAs, cdiv(n_ + 3 * np_, kNT)));
-    inc_dot_kernel<T, kNT><<<grid, kNT, 0, st_>>>(incU, bU_.as<T>(), n_, incV, bV_.as<T>(), 3 * np_, s, part,
-                                                  sched_.as<int>() + 3, trace);
+    NL_CUDA(launch_next(inc_dot_kernel<T, kNT>, dim3(grid), kNT, 0, st_, pdl, incU, bU_.as<T>(), n_, incV,
+                        bV_.as<T>(), 3 * np_, s, part, sched_.as<int>() + 3, trace));
     launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;

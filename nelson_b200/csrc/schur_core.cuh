@@ -106,6 +106,7 @@ class SchurCore {
   double* incV = nullptr;  // device, 3 np
   int keep_schur = 0;      // keep an undamaged copy of S for nl_get_schur
   int refine_sweeps = 0;
+  bool pdl = false;  // launch_next as programmatic dependents (setup)
   int use_tc = 1;          // tensor-core trailing update (mixed)
   nl_phase_times times{};
   long long launches = 0;

@@ -49,6 +49,7 @@ static __global__ void vinv_kernel(SchurDev d, const T* __restrict__ V, T* __res
                             int* __restrict__ status, int* __restrict__ counter, int* __restrict__ tickets, int ntickets,
                             unsigned long long* __restrict__ call, const int* __restrict__ active) {
   constexpr int LV = Layout<T, BC>::V;
+  chain_start(V, lam, active);
   if (active && !*active) return;
   // first kernel of a call: also clears the Schur work counter and the solves'
   // tickets, and numbers the call
@@ -119,6 +120,7 @@ static __global__ void __launch_bounds__(NT) wvinv_bs_kernel(SchurDev d, const T
   constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV;  // elements per piece, pieces per block
   extern __shared__ float4 w_stage[];
   __shared__ double red[NT / 32][BC];
+  chain_start(W, Vinv, bU, bV, active);
   if (active && !*active) return;
   const int c = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -130,16 +132,20 @@ static __global__ void __launch_bounds__(NT) wvinv_bs_kernel(SchurDev d, const T
   for (int q0 = d.w_row_ptr[c] + warp * 32; q0 < end; q0 += NT) {
     const int m = min(32, end - q0);
     const V16* src = reinterpret_cast<const V16*>(W + (size_t)q0 * LW);
+    V16 in[PW];
 #pragma unroll
     for (int i = 0; i < PW; i++)
-      if (lane + 32 * i < m * PW) st[lane + 32 * i] = __ldg(src + lane + 32 * i);
+      if (lane + 32 * i < m * PW) in[i] = src[lane + 32 * i];
+#pragma unroll
+    for (int i = 0; i < PW; i++)
+      if (lane + 32 * i < m * PW) st[lane + 32 * i] = in[i];
     __align__(16) T v[LV];
     T bv0 = 0, bv1 = 0, bv2 = 0;
     if (lane < m) {
       const int p = d.w_col[q0 + lane];
 #pragma unroll
       for (int i = 0; i < LV / EPV; i++)
-        reinterpret_cast<V16*>(v)[i] = __ldg(reinterpret_cast<const V16*>(Vinv + (size_t)p * LV) + i);
+        reinterpret_cast<V16*>(v)[i] = reinterpret_cast<const V16*>(Vinv + (size_t)p * LV)[i];
       bv0 = bV[3 * (size_t)p];
       bv1 = bV[3 * (size_t)p + 1];
       bv2 = bV[3 * (size_t)p + 2];
@@ -240,6 +246,7 @@ static __global__ void __launch_bounds__(SchurCfg<T, BC>::kWarps * 32)
   constexpr int LW = Cfg::LW, LU = Layout<T, BC>::U, TR = Cfg::TR, TD = Cfg::TD, LP = Cfg::LP, G = Cfg::G,
                 ROUNDS = Cfg::ROUNDS, PB = Cfg::PB, kStages = Cfg::kStages, VB = Cfg::VB;
   extern __shared__ float4 schur_smem[];
+  chain_start(U, Y, W, lam, active);
   if (active && !*active) return;
   const double rel = lam[0], abs = lam[1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -422,6 +429,7 @@ static __global__ void __launch_bounds__(SchurCfg<T, BC>::kWarps * 32)
 template <typename T>
 static __global__ void clear_kernel(T* __restrict__ S, T* __restrict__ S0, int n, int ld, int nb,
                                     const int* __restrict__ env_first, const int* __restrict__ active) {
+  chain_start(active);
   if (active && !*active) return;
   const int r = blockIdx.x, I = r / nb;
   const size_t c0 = env_first ? (size_t)env_first[I] * nb : 0, c1 = env_first ? (size_t)(I + 1) * nb : (size_t)ld;
@@ -455,6 +463,7 @@ static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T
   constexpr int LV = Layout<T, BC>::V;
   using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
   constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV, LP = kBackLanes<T>, NP = (PW + LP - 1) / LP;
+  chain_start(W, Vinv, bV, ok_flag, active);
   if (active && !*active) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x, l = threadIdx.x & (LP - 1);
   const bool failed = ok_flag && *ok_flag != 0;  // zero increment
@@ -488,7 +497,7 @@ static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T
         const int pc = l + LP * i;
         if (pc < PW) {
           __align__(16) T w[EPV];
-          *reinterpret_cast<V16*>(w) = __ldg(reinterpret_cast<const V16*>(W + (size_t)q * LW) + pc);
+          *reinterpret_cast<V16*>(w) = reinterpret_cast<const V16*>(W + (size_t)q * LW)[pc];
           const int m0 = pc * EPV, i0 = m0 / 3, k0 = m0 - 3 * i0;
           const double xa = i0 < BC ? x[i0] : 0.0, xb = i0 + 1 < BC ? x[i0 + 1] : 0.0;
 #pragma unroll
