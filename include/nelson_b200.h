@@ -350,16 +350,16 @@ nl_status nl_set_timing_detail(nl_problem* h, int detail);
  * (nelson/SolverDiagonalBlocksInverseWWtMultSchur.hpp:36-140), without that
  * solver's AMD reordering (nelson/DoubleSection.hpp:30-63). */
 nl_status nl_set_solver_kind(nl_problem* h, int kind);
-/* Bound of the flag waits between the CTAs of the triangular solves: a CTA
- * that has polled a tile's flag `polls` times without seeing it published
+/* Bound of the waits between the CTAs of the triangular solves: a CTA that
+ * has polled a tile's values `polls` times without seeing them published
  * records a timeout, returns, and the call reports NL_ERR_TIMEOUT (the wait
  * ends instead of hanging the GPU).  polls <= 0 restores the default
  * (2^24 polls, about a second).  (No counterpart in the reference: its solves
  * run on the host.) */
 nl_status nl_set_wait_limit(nl_problem* h, long long polls);
 /* Check of that bound: runs the forward triangular solve of the handle's
- * current factor with the flag of the first tile never published (its CTA is
- * not launched), so every other CTA's first wait runs out.  Returns
+ * current factor with the values of the first tile never published (its CTAs
+ * are not launched), so every other CTA's first wait runs out.  Returns
  * NL_ERR_TIMEOUT when the waits gave up as designed, NL_ERR_STATE when the
  * reduced system has fewer than two 128-row tiles.  The handle stays usable:
  * the next nl_compute_increment solves normally.  (No counterpart in the

@@ -22,7 +22,7 @@
 namespace nl {
 
 constexpr int NB = 128;
-constexpr long long kSpinLimit = 1LL << 24;  // default bound of the flag waits (~1 s worst case)
+constexpr long long kSpinLimit = 1LL << 24;  // default bound of the solves' waits (~1 s worst case)
 
 // ---------------------------------------------------------------------------
 // One CTA: factor the NB x NB diagonal tile of panel k in the storage
@@ -996,6 +996,72 @@ __device__ inline void syrk_cc_tile(T* __restrict__ S, int ld, int k, int gI, in
       if (I != J || c <= r) S[(size_t)(rA + r) * ld + rB + c] -= acc[i][j];
     }
   }
+}
+
+// The same for the FP64 factorisation, one panel: A_tt -= L_tp L_tp' on the lower
+// triangle, a CTA per 16 x 16 block (36), its four warps a quarter of K each on
+// the FP64 tensor cores.  Bound by its two copies (L2 latency).  With it and the
+// row-tile TRSM the FP64 chain no longer waits for the rest of the panel: 55 us per
+// panel (factor 21, TRSM of all rows 16, cuBLAS column update 12, gaps) before.
+constexpr int kDiag64Ctas = (NB / 16) * (NB / 16 + 1) / 2;
+static __global__ void __launch_bounds__(128) diag_update64_kernel(double* __restrict__ S, int ld, int t, int p,
+                                                                   const int* __restrict__ active) {
+  constexpr int LDA = NB + 4;
+  __shared__ __align__(16) double sa[2][16 * LDA];
+  chain_release();
+  chain_wait();
+  if (active && !*active) return;
+  int bi = 0, bj = blockIdx.x;  // block row, block column
+  while (bj > bi) bj -= ++bi;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double* L = S + (size_t)t * NB * ld + (size_t)p * NB;
+  for (int e = tid; e < 16 * (NB / 2); e += 128) {
+    const int r = e / (NB / 2), c = 2 * (e % (NB / 2));
+    cp_async16(&sa[0][r * LDA + c], L + (size_t)(16 * bi + r) * ld + c);
+    if (bi != bj) cp_async16(&sa[1][r * LDA + c], L + (size_t)(16 * bj + r) * ld + c);
+  }
+  cp_async_commit();
+  const int r = tid >> 3, c = 2 * (tid & 7);  // this thread's two entries of the block
+  double2* C = reinterpret_cast<double2*>(S + (size_t)(t * NB + 16 * bi + r) * ld + (size_t)t * NB + 16 * bj + c);
+  double2 v = *C;
+  cp_async_wait<0>();
+  __syncthreads();
+  const int g = lane >> 2, q = lane & 3;
+  const double* A = sa[0] + g * LDA + q;
+  const double* B = sa[bi != bj] + g * LDA + q;
+  double acc[2][2][2] = {};
+#pragma unroll
+  for (int k = 0; k < NB / 4; k += 4) {
+    const int kk = warp * (NB / 4) + k;
+    double a[2], b[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      a[i] = A[8 * i * LDA + kk];
+      b[i] = B[8 * i * LDA + kk];
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) mma_f64(acc[i][j], a[i], b[j]);
+  }
+  __syncthreads();
+  double* part = sa[0] + warp * 256;
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int m = 0; m < 2; m++) part[(8 * i + g) * 16 + 8 * j + 2 * q + m] = acc[i][j][m];
+  __syncthreads();
+  double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+  for (int w = 0; w < 4; w++) {
+    s0 += sa[0][w * 256 + r * 16 + c];
+    s1 += sa[0][w * 256 + r * 16 + c + 1];
+  }
+  if (bi != bj || c <= r) v.x -= s0;  // above the diagonal of the tile: as it was
+  if (bi != bj || c + 1 <= r) v.y -= s1;
+  *C = v;
 }
 
 // ---------------------------------------------------------------------------

@@ -356,7 +356,7 @@ class SchurCoreT final : public SchurCore {
   nl_status launch_update(int k, int t0, int nt, bool col_only, cudaStream_t st, int* status, const int* active) {
     nt = std::min(nt, env_end(k) - t0 + 1);  // tile rows past the envelope get zero updates
     if (nt <= 0) return NL_OK;
-    if (sizeof(T) == 8 && precision_ == NL_PREC_FP64 && cublas_) {
+    if (sizeof(T) == 8 && precision_ == NL_PREC_FP64 && cublas_ && !col_only) {
       // Row-major lower storage = column-major upper.  X = rows >= r0 of
       // panel k; the column-major view of S is M(a, b) = S[b][a].
       double* Sd = reinterpret_cast<double*>(S_.p);
@@ -366,16 +366,9 @@ class SchurCoreT final : public SchurCore {
       // each stream has its own handle (and workspace)
       cublasHandle_t hb = (st == st_) ? cublas_ : cublas2_;
       if (cublasSetStream(hb, st) != CUBLAS_STATUS_SUCCESS) return NL_ERR_CUDA;
-      if (col_only) {
-        // M(c0.., r0..) -= Pc' Pr : C (128 x n_rem) with A = M(kc.., c0..), B = M(kc.., r0..)
-        if (cublasDgemm(hb, CUBLAS_OP_T, CUBLAS_OP_N, NB, n_rem, NB, &alpha, Sd + r0 * ld_ + kc, ld_,
-                        Sd + r0 * ld_ + kc, ld_, &beta, Sd + r0 * ld_ + r0, ld_) != CUBLAS_STATUS_SUCCESS)
-          return NL_ERR_CUDA;
-      } else {
-        if (cublasDsyrk(hb, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, n_rem, NB, &alpha, Sd + r0 * ld_ + kc, ld_,
-                        &beta, Sd + r0 * ld_ + r0, ld_) != CUBLAS_STATUS_SUCCESS)
-          return NL_ERR_CUDA;
-      }
+      if (cublasDsyrk(hb, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, n_rem, NB, &alpha, Sd + r0 * ld_ + kc, ld_, &beta,
+                      Sd + r0 * ld_ + r0, ld_) != CUBLAS_STATUS_SUCCESS)
+        return NL_ERR_CUDA;
     } else if (sizeof(T) == 4 && use_tc) {
       TcPacks pk{{pack_slot(k), nullptr, nullptr, nullptr}, 1};
       NL_CUDA(tc_update_f32(reinterpret_cast<float*>(S_.p), ld_, k, t0, nt, col_only ? 1 : 0, 0, pk, active, status,
@@ -645,8 +638,118 @@ class SchurCoreT final : public SchurCore {
     return NL_OK;
   }
 
+  // tiles read and written per panel: block column k+1 and the triangle below it,
+  // both cut at the envelope (launch_update's clipping)
+  double update_bytes() const {
+    double tiles = 0;
+    for (int k = 0; k + 1 < ntiles_; k++) {
+      const int last = env_end(k);
+      const double na = std::max(0, last - k), nb = std::max(0, last - k - 1);
+      tiles += na + nb * (nb + 1) / 2;
+    }
+    return tiles * (double)NB * NB * sizeof(T) * 2;
+  }
+
+  // The FP64 schedule (cuBLAS trailing updates).  Per panel k:
+  //   main  potrf(k); [wait the column update of k] TRSM of row tile k+1; [wait
+  //         B(k-1)] tile (k+1, k+1)
+  //   aux   TRSM of the rows below tile k+1; [wait row tile k+1, B(k-1)] block
+  //         column k+1 below its diagonal tile
+  //   side  B(k): the triangle of tiles >= k+2 [waits for both TRSMs]
+  // The column update of k+1 ends 35 us after potrf(k), just before the chain needs
+  // it.  200 cameras: 55 -> 38 us per panel.
+  nl_status enqueue_factor64(int* status, const int* active) {
+    const bool tm = timing && !active;
+    const int nT = ntiles_;
+    if (tm && (int)upd_ev_.size() < 4 * nT) {
+      for (size_t i = upd_ev_.size(); i < (size_t)4 * nT; i++) {
+        cudaEvent_t e;
+        NL_CUDA(cudaEventCreate(&e));
+        upd_ev_.push_back(e);
+      }
+    }
+    double* S = reinterpret_cast<double*>(S_.p);
+    auto rec = [&](int e, cudaStream_t st) { return cudaEventRecord(dev_[e], st); };
+    auto wait = [&](cudaStream_t st, int e) { return cudaStreamWaitEvent(st, dev_[e], 0); };
+    double upd_flop = 0;
+    std::vector<char> timed(4 * (size_t)nT, 0);
+    bool pending_b = false, pending_col = false, early = pdl;
+    for (int k = 0; k < nT; k++) {
+      NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, potrf_smem<T>(), early && !tm, S_.as<T>(), ld_, k,
+                           Linv_.as<T>(), status, active));
+      launches++;
+      if (k + 1 >= nT) break;
+      const int below = ld_ - (k + 1) * NB, last = std::min(nT - 1, env_end(k));  // last tile row with nonzeros
+      upd_flop += (double)NB * below * (below + 1);
+      early = false;
+      if (last <= k) continue;  // nothing below the diagonal tile
+      NL_CUDA(rec(EV_POTRF, st_));
+      if (pending_col) NL_CUDA(wait(st_, EV_A1R));
+      trsm_tile_kernel<T><<<NB / kChainTrsmRows, 256, trsm_tile_smem<T>(), st_>>>(S_.as<T>(), ld_, k, Linv_.as<T>(),
+                                                                                  nullptr, active);
+      NL_CUDA(rec(EV_PACKF, st_));
+      if (pending_b) NL_CUDA(wait(st_, EV_B));
+      NL_CUDA(launch_chain(diag_update64_kernel, kDiag64Ctas, 128, 0, false, S, ld_, k + 1, k, active));
+      launches += 2;
+      early = true;
+      pending_col = false;
+      if (last < k + 2) continue;
+      const int rows = (last - k - 1) * NB;
+      NL_CUDA(wait(st3_, EV_POTRF));
+      launch_trsm(k, (k + 2) * NB, rows, nullptr, active, st3_);
+      NL_CUDA(rec(EV_PACKR, st3_));
+      NL_CUDA(wait(st3_, EV_PACKF));
+      if (pending_b) NL_CUDA(wait(st3_, EV_B));
+      if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k], st3_));
+      {
+        const double alpha = -1.0, beta = 1.0;
+        const size_t kc = (size_t)k * NB, c0 = (size_t)(k + 1) * NB, r0 = c0 + NB;
+        if (cublasSetStream(cublas_, st3_) != CUBLAS_STATUS_SUCCESS ||
+            cublasDgemm(cublas_, CUBLAS_OP_T, CUBLAS_OP_N, NB, rows, NB, &alpha, S + c0 * ld_ + kc, ld_,
+                        S + r0 * ld_ + kc, ld_, &beta, S + r0 * ld_ + c0, ld_) != CUBLAS_STATUS_SUCCESS)
+          return NL_ERR_CUDA;
+      }
+      if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 1], st3_));
+      timed[4 * k] = tm;
+      NL_CUDA(rec(EV_A1R, st3_));
+      pending_col = true;
+      NL_CUDA(wait(st2_, EV_PACKF));
+      NL_CUDA(wait(st2_, EV_PACKR));
+      if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 2], st2_));
+      nl_status r = launch_update(k, k + 2, nT - k - 2, false, st2_, status, active);
+      if (r != NL_OK) return r;
+      if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 3], st2_));
+      timed[4 * k + 2] = tm;
+      NL_CUDA(rec(EV_B, st2_));
+      pending_b = true;
+    }
+    // join: the solves that follow read every tile and Linv
+    if (pending_b) {  // the auxiliary stream has had work as well
+      NL_CUDA(rec(EV_AUX, st3_));
+      NL_CUDA(wait(st_, EV_AUX));
+      NL_CUDA(wait(st_, EV_B));
+    }
+    cublasSetStream(cublas_, st_);
+    if (tm) {
+      NL_CUDA(cudaStreamSynchronize(st_));
+      float tot = 0;
+      for (int i = 0; i < 4 * nT; i += 2)
+        if (timed[i]) {
+          float ms = 0;
+          cudaEventElapsedTime(&ms, upd_ev_[i], upd_ev_[i + 1]);
+          tot += ms;
+        }
+      times.update_ms = tot;
+      times.update_launches = nT - 1;
+      times.update_flop = upd_flop;
+      times.update_bytes = update_bytes();
+    }
+    return NL_OK;
+  }
+
   nl_status enqueue_factor(int* status, const int* active) {
     if (sizeof(T) == 4 && use_tc) return enqueue_factor_groups(status, active);
+    if (sizeof(T) == 8 && precision_ == NL_PREC_FP64 && cublas_) return enqueue_factor64(status, active);
     const bool tm = timing && !active;
     if (tm && (int)upd_ev_.size() < 4 * ntiles_) {
       for (size_t i = upd_ev_.size(); i < (size_t)4 * ntiles_; i++) {
@@ -701,15 +804,7 @@ class SchurCoreT final : public SchurCore {
       times.update_ms = tot;
       times.update_launches = nupd;
       times.update_flop = upd_flop;
-      // tiles read and written per panel: block column k+1 and the triangle
-      // below it, both cut at the envelope (launch_update's clipping)
-      double tiles = 0;
-      for (int k = 0; k + 1 < ntiles_; k++) {
-        const int last = env_end(k);
-        const double na = std::max(0, last - k), nb = std::max(0, last - k - 1);
-        tiles += na + nb * (nb + 1) / 2;
-      }
-      times.update_bytes = tiles * (double)NB * NB * sizeof(T) * 2;
+      times.update_bytes = update_bytes();
     }
     return NL_OK;
   }

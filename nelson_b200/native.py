@@ -433,12 +433,12 @@ class BAProblemGPU:
         self._c(self.L.nl_set_timing_detail(self.h, C.c_int(1 if detail else 0)), "nl_set_timing_detail")
 
     def set_wait_limit(self, polls: int):
-        """Bound of the triangular solves' flag waits, in polls (<= 0: the
+        """Bound of the triangular solves' waits, in polls (<= 0: the
         default); nl_set_wait_limit."""
         self._c(self.L.nl_set_wait_limit(self.h, C.c_longlong(int(polls))), "nl_set_wait_limit")
 
     def check_wait_timeout(self) -> int:
-        """nl_check_wait_timeout: the forward solve with one tile's flag
+        """nl_check_wait_timeout: the forward solve with one tile's values
         withheld; returns the status code (7 = NL_ERR_TIMEOUT when every wait
         gave up as designed)."""
         return int(self.L.nl_check_wait_timeout(self.h))

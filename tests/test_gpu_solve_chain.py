@@ -66,3 +66,35 @@ def test_residual(prec, bu, nu, kind):
         assert ok
         assert np.abs(H @ x + mu * x + b).max() <= tol * np.abs(b).max()
     g.close()
+
+
+@pytest.mark.parametrize("prec", [N.PREC_FP64, N.PREC_MIXED])
+@pytest.mark.parametrize("links", [(), ((63, 64),), ((0, 191),), ((63, 64), (64, 191), (130, 255))])
+def test_separate_tiles(prec, links):
+    """Envelope order where tile rows have no neighbour below, the next one only, or
+    one further down: four tiles of 64 independent 2 x 2 blocks and a few couplings.
+    The Schur complement is known exactly: same tolerances."""
+    bu, nu = 2, 256
+    r = np.random.default_rng(len(links))
+    u_rc = sorted([(i, i) for i in range(nu)] + list(links), key=lambda t: (t[1], t[0]))
+    U = np.array([8.0 * np.eye(2) if i == j else r.uniform(-1, 1, (2, 2)) for i, j in u_rc])
+    v_rc = w_rc = np.stack([np.arange(nu)] * 2, 1).astype(np.int32)
+    V, W = np.tile(8.0 * np.eye(3), (nu, 1, 1)), r.uniform(-1, 1, (nu, 2, 3))
+    H = np.zeros((5 * nu, 5 * nu))
+    for q, (i, j) in enumerate(u_rc):
+        H[2 * i:2 * i + 2, 2 * j:2 * j + 2] = U[q]
+        H[2 * j:2 * j + 2, 2 * i:2 * i + 2] = U[q].T
+    for p in range(nu):
+        s = slice(2 * nu + 3 * p, 2 * nu + 3 * p + 3)
+        H[s, s] = V[p]
+        H[2 * p:2 * p + 2, s] = W[p]
+        H[s, 2 * p:2 * p + 2] = W[p].T
+    b = r.normal(size=5 * nu)
+    g = N.SchurSolverGPU(bu, nu, nu, np.array(u_rc, np.int32), v_rc, w_rc, precision=prec)
+    g.set_solver_kind(N.SOLVER_ENVELOPE)
+    g.set_hessian(U, V, W, b[:2 * nu], b[2 * nu:])
+    for _ in range(2):
+        ok, du, dv = g.compute_increment(0.0, 0.0)
+        assert ok
+        assert np.abs(H @ np.r_[du, dv] + b).max() <= (1e-11 if prec == N.PREC_FP64 else 2e-5) * np.abs(b).max()
+    g.close()
