@@ -657,7 +657,7 @@ class SchurCoreT final : public SchurCore {
   //         column k+1 below its diagonal tile
   //   side  B(k): the triangle of tiles >= k+2 [waits for both TRSMs]
   // The column update of k+1 ends 35 us after potrf(k), just before the chain needs
-  // it.  200 cameras: 55 -> 38 us per panel.
+  // it.  200 cameras: 55 -> 40 us per panel.
   nl_status enqueue_factor64(int* status, const int* active) {
     const bool tm = timing && !active;
     const int nT = ntiles_;
