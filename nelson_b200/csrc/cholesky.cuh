@@ -928,8 +928,8 @@ static __global__ void __launch_bounds__(256) diag_update_kernel(float* __restri
 
 // ---------------------------------------------------------------------------
 // CUDA-core trailing update (FP32 or FP64), one CTA per 128 x 128 lower tile:
-// C_IJ -= X_I X_J' with X = columns [k NB, (k+1) NB).  Used as the portable
-// reference of the tensor-core kernel and for small problems.
+// C_IJ -= X_I X_J' with X = columns [k NB, (k+1) NB).  The reference of the
+// tensor-core kernel's self-test.
 template <typename T>
 __device__ inline void syrk_cc_tile(T* __restrict__ S, int ld, int k, int gI, int gJ);
 
@@ -943,14 +943,6 @@ static __global__ void __launch_bounds__(256) syrk_cc_kernel(T* __restrict__ S, 
   while (I * (I + 1) / 2 > q) I--;
   const int J = q - I * (I + 1) / 2;
   syrk_cc_tile<T>(S, ld, k, t0 + I, t0 + J);
-}
-
-// one output tile (gI, gJ), gI >= gJ
-template <typename T>
-static __global__ void __launch_bounds__(256) syrk_cc_tile_kernel(T* __restrict__ S, int ld, int k, int gI, int gJ,
-                                                                  const int* __restrict__ active) {
-  if (active && !*active) return;
-  syrk_cc_tile<T>(S, ld, k, gI, gJ);
 }
 
 template <typename T>

@@ -23,7 +23,7 @@ inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 template <typename T, int BC>
 class SchurCoreT final : public SchurCore {
  public:
-  explicit SchurCoreT(cublasHandle_t cb, int precision) : cublas_(cb), precision_(precision) {}
+  explicit SchurCoreT(cublasHandle_t cb) : cublas_(cb) {}
 
   int n() const override { return n_; }
   int ld() const override { return ld_; }
@@ -267,8 +267,6 @@ class SchurCoreT final : public SchurCore {
                                  2 * (int)kDiagUpdSmem));
     if (!ev_[0]) {
       for (auto& e : ev_) NL_CUDA(cudaEventCreate(&e));
-      NL_CUDA(cudaEventCreateWithFlags(&ev_panel_, cudaEventDisableTiming));
-      NL_CUDA(cudaEventCreateWithFlags(&ev_b_, cudaEventDisableTiming));
       {
         // the side stream (bulk trailing updates) yields SMs to the critical path
         int lo = 0, hi = 0;
@@ -345,49 +343,6 @@ class SchurCoreT final : public SchurCore {
     return NL_OK;
   }
 
-  // Right-looking blocked Cholesky with look-ahead.  After panel k is
-  // factored (diagonal tile + TRSM below it), its trailing update is split:
-  //   update A(k): block column k+1 (tiles (I, k+1), I >= k+1), main stream;
-  //   update B(k): the triangle of tiles >= k+2, side stream,
-  // so the factorisation of panel k+1 (which needs only A(k)) overlaps B(k).
-  // A(k) waits for B(k-1) (both touch block column k+1); B(k) follows B(k-1)
-  // on the side stream and waits for panel k.  The BF16 pack of panel k is
-  // double-buffered.
-  nl_status launch_update(int k, int t0, int nt, bool col_only, cudaStream_t st, int* status, const int* active) {
-    nt = std::min(nt, env_end(k) - t0 + 1);  // tile rows past the envelope get zero updates
-    if (nt <= 0) return NL_OK;
-    if (sizeof(T) == 8 && precision_ == NL_PREC_FP64 && cublas_ && !col_only) {
-      // Row-major lower storage = column-major upper.  X = rows >= r0 of
-      // panel k; the column-major view of S is M(a, b) = S[b][a].
-      double* Sd = reinterpret_cast<double*>(S_.p);
-      const double alpha = -1.0, beta = 1.0;
-      const size_t r0 = (size_t)t0 * NB, kc = (size_t)k * NB;
-      const int n_rem = nt * NB;  // ld_ - r0 without the envelope
-      // each stream has its own handle (and workspace)
-      cublasHandle_t hb = (st == st_) ? cublas_ : cublas2_;
-      if (cublasSetStream(hb, st) != CUBLAS_STATUS_SUCCESS) return NL_ERR_CUDA;
-      if (cublasDsyrk(hb, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, n_rem, NB, &alpha, Sd + r0 * ld_ + kc, ld_, &beta,
-                      Sd + r0 * ld_ + r0, ld_) != CUBLAS_STATUS_SUCCESS)
-        return NL_ERR_CUDA;
-    } else if (sizeof(T) == 4 && use_tc) {
-      TcPacks pk{{pack_slot(k), nullptr, nullptr, nullptr}, 1};
-      NL_CUDA(tc_update_f32(reinterpret_cast<float*>(S_.p), ld_, k, t0, nt, col_only ? 1 : 0, 0, pk, active, status,
-                            st));
-      launches++;
-    } else {
-      if (col_only) {
-        // column block as a triangle of 1 plus rows below: reuse the tile kernel per row tile
-        for (int I = 0; I < nt; I++)
-          syrk_cc_tile_kernel<T><<<1, 256, 0, st>>>(S_.as<T>(), ld_, k, t0 + I, t0, active);
-        launches += nt;
-      } else {
-        syrk_cc_kernel<T><<<nt * (nt + 1) / 2, 256, 0, st>>>(S_.as<T>(), ld_, k, t0, nt, active);
-        launches++;
-      }
-    }
-    return NL_OK;
-  }
-
   // Rows [r0, r0 + nrows) of panel k.  One row per thread while that leaves
   // SMs idle, else two: the staging of L_kk is then shared by twice the rows.
   void launch_trsm(int k, int r0, int nrows, uint8_t* pack, const int* active, cudaStream_t st) {
@@ -398,20 +353,6 @@ class SchurCoreT final : public SchurCore {
       trsm_kernel<T, 2><<<cdiv(nrows, 32), 256, trsm_smem<T, 2>(), st>>>(S_.as<T>(), ld_, k, r0, nrows, Linv_.as<T>(),
                                                                          pack, active);
     launches++;
-  }
-
-  nl_status factor_panel(int k, int* status, const int* active) {
-    potrf_diag_kernel<T><<<1, PT, potrf_smem<T>(), st_>>>(S_.as<T>(), ld_, k, Linv_.as<T>(), status, active);
-    launches++;
-    const int below = std::min(ld_, (env_end(k) + 1) * NB) - (k + 1) * NB;  // rows past the envelope are zero
-    if (below > 0) {
-      launch_trsm(k, (k + 1) * NB, below, nullptr, active, st_);
-      if (sizeof(T) == 4 && use_tc) {
-        NL_CUDA(tc_pack_f32(reinterpret_cast<const float*>(S_.p), ld_, k, 0, below, pack_slot(k), active, st_));
-        launches++;
-      }
-    }
-    return NL_OK;
   }
 
   // A kernel on the main stream (launch_next)
@@ -639,7 +580,7 @@ class SchurCoreT final : public SchurCore {
   }
 
   // tiles read and written per panel: block column k+1 and the triangle below it,
-  // both cut at the envelope (launch_update's clipping)
+  // both cut at the envelope
   double update_bytes() const {
     double tiles = 0;
     for (int k = 0; k + 1 < ntiles_; k++) {
@@ -716,8 +657,16 @@ class SchurCoreT final : public SchurCore {
       NL_CUDA(wait(st2_, EV_PACKF));
       NL_CUDA(wait(st2_, EV_PACKR));
       if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 2], st2_));
-      nl_status r = launch_update(k, k + 2, nT - k - 2, false, st2_, status, active);
-      if (r != NL_OK) return r;
+      {
+        // row-major lower storage = column-major upper; the side stream has its own
+        // handle (and workspace)
+        const double alpha = -1.0, beta = 1.0;
+        const size_t kc = (size_t)k * NB, r0 = (size_t)(k + 2) * NB;
+        if (cublasSetStream(cublas2_, st2_) != CUBLAS_STATUS_SUCCESS ||
+            cublasDsyrk(cublas2_, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, rows, NB, &alpha, S + r0 * ld_ + kc, ld_, &beta,
+                        S + r0 * ld_ + r0, ld_) != CUBLAS_STATUS_SUCCESS)
+          return NL_ERR_CUDA;
+      }
       if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 3], st2_));
       timed[4 * k + 2] = tm;
       NL_CUDA(rec(EV_B, st2_));
@@ -748,65 +697,10 @@ class SchurCoreT final : public SchurCore {
   }
 
   nl_status enqueue_factor(int* status, const int* active) {
-    if (sizeof(T) == 4 && use_tc) return enqueue_factor_groups(status, active);
-    if (sizeof(T) == 8 && precision_ == NL_PREC_FP64 && cublas_) return enqueue_factor64(status, active);
-    const bool tm = timing && !active;
-    if (tm && (int)upd_ev_.size() < 4 * ntiles_) {
-      for (size_t i = upd_ev_.size(); i < (size_t)4 * ntiles_; i++) {
-        cudaEvent_t e;
-        NL_CUDA(cudaEventCreate(&e));
-        upd_ev_.push_back(e);
-      }
-    }
-    double upd_flop = 0;
-    nl_status r;
-    if ((r = factor_panel(0, status, active)) != NL_OK) return r;
-    bool pending_b = false;
-    for (int k = 0; k + 1 < ntiles_; k++) {
-      const int below = ld_ - (k + 1) * NB;
-      upd_flop += (double)NB * below * (below + 1);
-      // panel k is factored and packed
-      NL_CUDA(cudaEventRecord(ev_panel_, st_));
-      // A(k): block column k+1, after B(k-1)
-      if (pending_b) NL_CUDA(cudaStreamWaitEvent(st_, ev_b_, 0));
-      if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k], st_));
-      if ((r = launch_update(k, k + 1, ntiles_ - k - 1, true, st_, status, active)) != NL_OK) return r;
-      if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 1], st_));
-      // B(k): tiles >= k+2 on the side stream
-      if (k + 2 < ntiles_) {
-        NL_CUDA(cudaStreamWaitEvent(st2_, ev_panel_, 0));
-        if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 2], st2_));
-        if ((r = launch_update(k, k + 2, ntiles_ - k - 2, false, st2_, status, active)) != NL_OK) return r;
-        if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 3], st2_));
-        NL_CUDA(cudaEventRecord(ev_b_, st2_));
-        pending_b = true;
-      } else {
-        pending_b = false;
-      }
-      if ((r = factor_panel(k + 1, status, active)) != NL_OK) return r;
-    }
-    if (pending_b) NL_CUDA(cudaStreamWaitEvent(st_, ev_b_, 0));
-    if (cublas_) cublasSetStream(cublas_, st_);
-    if (tm) {
-      NL_CUDA(cudaStreamSynchronize(st_));
-      float tot = 0;
-      int nupd = 0;
-      for (int k = 0; k + 1 < ntiles_; k++) {
-        float ms = 0;
-        cudaEventElapsedTime(&ms, upd_ev_[4 * k], upd_ev_[4 * k + 1]);
-        tot += ms;
-        if (k + 2 < ntiles_) {
-          cudaEventElapsedTime(&ms, upd_ev_[4 * k + 2], upd_ev_[4 * k + 3]);
-          tot += ms;
-        }
-        nupd++;
-      }
-      times.update_ms = tot;
-      times.update_launches = nupd;
-      times.update_flop = upd_flop;
-      times.update_bytes = update_bytes();
-    }
-    return NL_OK;
+    if constexpr (sizeof(T) == 4)
+      return use_tc ? enqueue_factor_groups(status, active) : NL_ERR_STATE;
+    else
+      return cublas_ ? enqueue_factor64(status, active) : NL_ERR_STATE;
   }
 
   nl_status enqueue_increment(const double* lam, int* status, const int* active) override {
@@ -996,7 +890,6 @@ class SchurCoreT final : public SchurCore {
 
  private:
   cublasHandle_t cublas_;
-  int precision_;
   cudaStream_t st_ = nullptr;
   int nci_ = 0, np_ = 0, nU_ = 0, nV_ = 0, nW_ = 0, nS_ = 0, n_ = 0, ld_ = 0, ntiles_ = 0;
   long long npairs_ = 0;
@@ -1013,7 +906,6 @@ class SchurCoreT final : public SchurCore {
   DevBuf v_uid_, w_row_ptr_, w_col_, w_row_, w_col_ptr_, w_col_uid_, u_diag_, s_i_, s_j_, s_uuid_, s_ptr_, pa_, pb_, s_items_,
       s_slot_, s_part_, sched_;
   cudaEvent_t ev_[7] = {};
-  cudaEvent_t ev_panel_ = nullptr, ev_b_ = nullptr;
   cudaStream_t st2_ = nullptr;  // side stream of the look-ahead factorisation
   cudaStream_t st3_ = nullptr;  // auxiliary stream of the tensor-core schedule
   cudaEvent_t dev_[8] = {};     // dependency events of the tensor-core schedule
@@ -1039,8 +931,6 @@ class SchurCoreT final : public SchurCore {
       if (e) cudaEventDestroy(e);
     for (auto e : ev_)
       if (e) cudaEventDestroy(e);
-    if (ev_panel_) cudaEventDestroy(ev_panel_);
-    if (ev_b_) cudaEventDestroy(ev_b_);
     for (auto e : upd_ev_) cudaEventDestroy(e);
   }
 };
@@ -1049,10 +939,10 @@ class SchurCoreT final : public SchurCore {
 
 std::unique_ptr<SchurCore> make_schur_core(int precision, int bc, cublasHandle_t cublas) {
   const bool f64 = precision == NL_PREC_FP64;
-#define NL_MK(B)                                                          \
-  case B:                                                                 \
-    if (f64) return std::unique_ptr<SchurCore>(new SchurCoreT<double, B>(cublas, precision)); \
-    return std::unique_ptr<SchurCore>(new SchurCoreT<float, B>(cublas, precision));
+#define NL_MK(B)                                                                   \
+  case B:                                                                          \
+    if (f64) return std::unique_ptr<SchurCore>(new SchurCoreT<double, B>(cublas)); \
+    return std::unique_ptr<SchurCore>(new SchurCoreT<float, B>(cublas));
   switch (bc) {
     NL_MK(2)
     NL_MK(3)
