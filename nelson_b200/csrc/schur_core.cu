@@ -9,8 +9,8 @@ namespace {
 
 constexpr int kNT = 256, kWvNT = 256;
 // Programmatic dependent launches up to this many W blocks: small systems are bound
-// by the 1.8 us between two kernels (20 cameras, 867 -> 718 us per solve; 64
-// cameras 1,590 -> 1,373 us); on large ones the CTAs that wait on the chip cost the
+// by the 1.8 us between two kernels (20 cameras, 867 -> 691 us per solve; 64
+// cameras 1,590 -> 1,322 us); on large ones the CTAs that wait on the chip cost the
 // running kernels as much as is saved (200 cameras, 375k blocks: 8.85 / 8.87 ms,
 // FP64 12.8 / 13.0 ms).
 constexpr int kPdlBlocks = 1 << 16;
