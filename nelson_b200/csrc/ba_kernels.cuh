@@ -309,10 +309,10 @@ static __global__ void __launch_bounds__(NT) pt_pass_kernel(BaDev d, T* __restri
   constexpr int LV = Layout<T, BC>::V;
   chain_start(active);
   if (active && !*active) return;
-  const int t = blockIdx.x * NT + threadIdx.x, l = threadIdx.x & 3;
-  if ((t & ~31) >> 2 >= d.np_var) return;  // whole warps leave
-  const bool valid = t >> 2 < d.np_var;
-  const int p = valid ? t >> 2 : 0;
+  const int t = group_item(blockIdx.x, NT, threadIdx.x, 4), l = threadIdx.x & 3;
+  if (group_item(blockIdx.x, NT, threadIdx.x & ~31, 4) >= d.np_var) return;  // whole warps leave
+  const bool valid = t < d.np_var;
+  const int p = valid ? t : 0;
   const double X[3] = {d.pt[3 * (size_t)p], d.pt[3 * (size_t)p + 1], d.pt[3 * (size_t)p + 2]};
   T v[6] = {0, 0, 0, 0, 0, 0}, b[3] = {0, 0, 0};
   const int e1 = valid ? d.pt_edge_ptr[p + 1] : 0;

@@ -147,6 +147,13 @@ __device__ inline bool item_total(T* sum, T* __restrict__ part, int* __restrict_
   return true;
 }
 
+// Item of a thread where groups of `lanes` threads share one, `nt` threads per CTA
+// (lanes divides nt).  Formed from the CTA's first item: the thread's number in the
+// grid is lanes times as large and passes 2^31 where the items are far from it.
+__host__ __device__ inline int group_item(unsigned block, int nt, int thread, int lanes) {
+  return (int)(block * (unsigned)(nt / lanes)) + thread / lanes;
+}
+
 // CTAs per camera for a pass over a camera's observations with nt threads: four
 // CTAs per SM over the chip, two rounds of work at least for each.
 inline int ctas_per_camera(int nc, long long observations, int nt) {

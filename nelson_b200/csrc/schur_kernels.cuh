@@ -465,15 +465,16 @@ static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T
   constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV, LP = kBackLanes<T>, NP = (PW + LP - 1) / LP;
   chain_start(W, Vinv, bV, ok_flag, active);
   if (active && !*active) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, l = threadIdx.x & (LP - 1);
+  const int l = threadIdx.x & (LP - 1);
   const bool failed = ok_flag && *ok_flag != 0;  // zero increment
   if (failed) {
-    for (int i = t; i < nxu; i += gridDim.x * blockDim.x) xU[i] = 0.0;
-    for (int i = t; i < 3 * d.np; i += gridDim.x * blockDim.x) xV[i] = 0.0;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    for (long long i = t; i < nxu; i += nt) xU[i] = 0.0;
+    for (long long i = t; i < 3LL * d.np; i += nt) xV[i] = 0.0;
     return;
   }
-  const int p = t / LP;
-  if ((t & ~31) / LP >= d.np) return;  // whole warps leave
+  const int p = group_item(blockIdx.x, 128, threadIdx.x, LP);
+  if (group_item(blockIdx.x, 128, threadIdx.x & ~31, LP) >= d.np) return;  // whole warps leave
   const bool valid = p < d.np;
   const int s0 = valid ? d.w_col_ptr[p] : 0, s1 = valid ? d.w_col_ptr[p + 1] : 0;
   // piece i of this lane: elements m0 = (l + LP i) EPV .., rows from m0 / 3 on; sum[i][r]
