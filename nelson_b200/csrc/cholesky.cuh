@@ -1091,11 +1091,17 @@ __device__ __forceinline__ ulonglong2 look_packet(const ulonglong2* p) {
   return v;
 }
 
+// The values of a tile in shared memory, read as double2 (load4)
+struct __align__(16) TileValues {
+  double v[NB];
+};
+static_assert(alignof(TileValues) == 16 && sizeof(TileValues) % 16 == 0, "load4 reads 16-byte pieces");
+
 // Fetches the 128 values at pk into dst (shared), one per thread; every thread of
 // the CTA calls it.  `seen`: what a look at the thread's packet gave earlier.
 // False after a wait that ran out.
 __device__ inline bool fetch_tile(const ulonglong2* __restrict__ pk, ulonglong2 seen, unsigned long long tag,
-                                  double* __restrict__ dst, int* __restrict__ status, long long limit) {
+                                  TileValues& dst, int* __restrict__ status, long long limit) {
   long long it = 0;
   while (seen.y != tag && ++it <= limit) {
     if (it > 4096) __nanosleep(100);
@@ -1103,7 +1109,7 @@ __device__ inline bool fetch_tile(const ulonglong2* __restrict__ pk, ulonglong2 
   }
   const bool bad = seen.y != tag;
   if (bad) atomicOr(status, ST_SPIN_TIMEOUT);
-  dst[threadIdx.x] = __longlong_as_double(seen.x);
+  dst.v[threadIdx.x] = __longlong_as_double(seen.x);
   return !__syncthreads_or(bad);
 }
 
@@ -1376,7 +1382,7 @@ static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
     int* __restrict__ ticket, ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub,
     int* __restrict__ status, long long spin_limit, const int* __restrict__ env, const int* __restrict__ active) {
   extern __shared__ float4 own4[];
-  __shared__ double got[2][NB];
+  __shared__ TileValues got[2];
   __shared__ int t_s;
   chain_start(L, Linv, hop, b, part, call, active);
   if (active && !*active) return;
@@ -1403,7 +1409,7 @@ static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
   double x4[4];
   auto fetch = [&](const ulonglong2* p, ulonglong2 seen) -> bool {  // uniform
     const bool ok = fetch_tile(p, seen, tag, got[par], status, spin_limit);
-    load4(got[par] + 4 * lane, x4);
+    load4(got[par].v + 4 * lane, x4);
     par ^= 1;  // the other buffer is written only after the next barrier
     return ok;
   };
@@ -1462,7 +1468,8 @@ static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
     ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub, int* __restrict__ status,
     long long spin_limit, const int* __restrict__ env, const int* __restrict__ active) {
   extern __shared__ float4 own4[];
-  __shared__ double got[2][NB], red[SVT / 32][SVR];
+  __shared__ TileValues got[2];
+  __shared__ double red[SVT / 32][SVR];
   __shared__ int t_s;
   chain_start(L, Linv, hop, yv, call, active);
   if (active && !*active) return;
@@ -1487,7 +1494,7 @@ static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
   const double* v = nullptr;
   auto fetch = [&](const ulonglong2* p, ulonglong2 seen) -> bool {  // uniform
     const bool ok = fetch_tile(p, seen, tag, got[par], status, spin_limit);
-    v = got[par];
+    v = got[par].v;
     par ^= 1;
     return ok;
   };
