@@ -1411,6 +1411,7 @@ static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
     const bool ok = fetch_tile(p, seen, tag, got[par], status, spin_limit);
     load4(got[par].v + 4 * lane, x4);
     par ^= 1;  // the other buffer is written only after the next barrier
+    if (!ok) cp_async_wait<0>();  // the CTA gives up: no copy stays in flight
     return ok;
   };
   const ulonglong2 none = make_ulonglong2(0, 0);  // call numbers start at 1
@@ -1496,6 +1497,7 @@ static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
     const bool ok = fetch_tile(p, seen, tag, got[par], status, spin_limit);
     v = got[par].v;
     par ^= 1;
+    if (!ok) cp_async_wait<0>();  // the CTA gives up: no copy stays in flight
     return ok;
   };
   // the sum over a column's rows: the lanes of a column, then the warps (thread < SVR)
