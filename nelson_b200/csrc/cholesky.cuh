@@ -1061,9 +1061,13 @@ static __global__ void __launch_bounds__(128) diag_update64_kernel(double* __res
 // kSolveCtas CTAs per tile, 32 rows (backward: columns) each: a hop is bounded by
 // the product with a 128 x 128 matrix, which in FP64 arithmetic on one SM takes
 // 1 us (16 conversions and 38 FMAs per clock), and by the way of the result to
-// the next tile.  CTAs take tickets in tile order (forward) or reverse order
-// (backward); a CTA waits on tiles of earlier tickets and on its own tile's, so
-// with four CTAs on the chip every wait ends; each is also bounded.
+// the next tile.  A CTA waits for earlier tiles (forward; later ones backward) and for
+// the other CTAs of its own tile.  The launch is in clusters of kSolveCtas, whose CTAs
+// are on the chip together, and CTA r of each cluster takes its tile from ticket r: with
+// m clusters placed, the tickets hand out tiles 0 .. m - 1 and each of them has all of
+// its CTAs on the chip, however many other solves share it.  So every wait ends; each
+// is also bounded.  (Without clusters, partly placed tiles of about a hundred FP64 solves
+// at once could fill the chip.)
 //
 // A value is passed on with the tag of its solve as one 16-byte store and load:
 // the reader that finds the tag has the value, without barrier, release, flag and
@@ -1075,6 +1079,8 @@ static __global__ void __launch_bounds__(128) diag_update64_kernel(double* __res
 // hop, of which 0.7 us are the packet's way through L2; three hop matrices instead
 // of two change nothing).
 constexpr int kSolveCtas = 4, SVR = NB / kSolveCtas, SVT = 128;
+// rank of the CTA in its cluster (clusters of kSolveCtas consecutive CTAs)
+__device__ __forceinline__ int solve_rank() { return (int)(blockIdx.x % kSolveCtas); }
 static_assert(SVT == NB && SVR == 8 * (SVT / 32), "a thread fetches one row, a warp finishes eight");
 
 __device__ inline void put_packet(ulonglong2* p, double v, unsigned long long tag) {
@@ -1114,9 +1120,9 @@ __device__ inline bool fetch_tile(const ulonglong2* __restrict__ pk, ulonglong2 
 }
 
 // Start of a call that solves without forming S: clears the solves' tickets (the
-// first forward solve hands out CTAs from `first` on) and numbers the call.
+// first forward solve hands out tiles from `first` on) and numbers the call.
 static __global__ void solve_begin_kernel(int* tickets, int n, int first, unsigned long long* call) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) tickets[i] = i == 0 ? first : 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) tickets[i] = i < kSolveCtas ? first : 0;
   if (threadIdx.x == 0) (*call)++;
 }
 
@@ -1376,7 +1382,7 @@ static __global__ void __launch_bounds__(256) hop_mat_kernel(const T* __restrict
 // `part` of a refinement residual.  Warp w, lane l: rows 8 w .. 8 w + 7 of the
 // CTA's, columns 4 l .. 4 l + 3.  pk: 2 x 128 ntiles packets (y, b - partial).
 template <typename T>
-static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
+static __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(SVT) trsv_fwd_kernel(
     const T* __restrict__ L, int ld, int ntiles, const T* __restrict__ Linv, const T* __restrict__ hop,
     const double* __restrict__ b, const double* __restrict__ part, int nch, double* __restrict__ y,
     int* __restrict__ ticket, ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub,
@@ -1388,9 +1394,9 @@ static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
   if (active && !*active) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned long long tag = (*call << 32) | (unsigned)sub;
-  if (tid == 0) t_s = atomicAdd(ticket, 1);
+  if (tid == 0) t_s = atomicAdd(ticket + solve_rank(), 1);
   __syncthreads();
-  const int I = t_s / kSolveCtas, r0 = (t_s % kSolveCtas) * SVR + warp * 8;
+  const int I = t_s, r0 = solve_rank() * SVR + warp * 8;
   const size_t own = (size_t)r0 * NB + 4 * lane;
   OwnBlock<T>(own4, 0).stage(Linv + (size_t)I * NB * NB + own, NB);
 #pragma unroll
@@ -1463,7 +1469,7 @@ static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
 // thread holds rows 32 w + (l >> 3) + 4 i, columns 4 (l & 7) .. + 3 of the CTA's.
 // `sum`, if given, gets x added (a refinement step).
 template <typename T>
-static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
+static __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(SVT) trsv_bwd_kernel(
     const T* __restrict__ L, int ld, int ntiles, const T* __restrict__ Linv, const T* __restrict__ hop,
     const double* __restrict__ yv, double* __restrict__ x, double* __restrict__ sum, int* __restrict__ ticket,
     ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub, int* __restrict__ status,
@@ -1476,9 +1482,9 @@ static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
   if (active && !*active) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned long long tag = (*call << 32) | (unsigned)sub;
-  if (tid == 0) t_s = atomicAdd(ticket, 1);
+  if (tid == 0) t_s = atomicAdd(ticket + solve_rank(), 1);
   __syncthreads();
-  const int I = ntiles - 1 - t_s / kSolveCtas, q0 = (t_s % kSolveCtas) * SVR;
+  const int I = ntiles - 1 - t_s, q0 = solve_rank() * SVR;
   const int tr = 32 * warp + (lane >> 3), tc = q0 + 4 * (lane & 7);  // transposed blocks: first row, first column
   OwnBlock<T>(own4, 0).stage(Linv + (size_t)I * NB * NB + (size_t)tr * NB + tc, 4 * NB);
 #pragma unroll

@@ -185,7 +185,7 @@ class SchurCoreT final : public SchurCore {
     NL_CUDA(cudaMemcpyAsync(env_dev_.p, env_first_.data(), sizeof(int) * ntiles_, cudaMemcpyHostToDevice, st_));
     NL_CUDA(cudaMemcpyAsync(env_dev_.as<int>() + ntiles_, env_last_.data(), sizeof(int) * ntiles_,
                             cudaMemcpyHostToDevice, st_));
-    NL_TRY(tickets_.alloc(sizeof(int) * 2 * (size_t)solve_slots()));
+    NL_TRY(tickets_.alloc(sizeof(int) * (size_t)tickets()));
     NL_TRY(packets_.alloc(16 * (2 * (size_t)ld_ + 1)));
     NL_CUDA(cudaMemsetAsync(packets_.p, 0, packets_.bytes, st_));
     NL_TRY(S_.alloc(sizeof(T) * (size_t)ld_ * ld_));
@@ -294,8 +294,8 @@ class SchurCoreT final : public SchurCore {
   // later refinement sweeps clear and use them again.
   nl_status enqueue_solve(int k, int* status, const int* active) {
     const int* env = envelope ? env_dev_.as<int>() : nullptr;
-    int* tk = tickets_.as<int>() + 2 * (k % solve_slots());
-    if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(tk, 0, 2 * sizeof(int), st_));
+    int* tk = tickets_.as<int>() + 2 * kSolveCtas * (k % solve_slots());
+    if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(tk, 0, 2 * kSolveCtas * sizeof(int), st_));
     const int grid = kSolveCtas * ntiles_;
     NL_CUDA(launch_next(trsv_fwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl && !timing, S_.as<T>(), ld_,
                         ntiles_,
@@ -304,7 +304,7 @@ class SchurCoreT final : public SchurCore {
     NL_CUDA(launch_next(trsv_bwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl && !timing, S_.as<T>(), ld_,
                         ntiles_,
                         Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
-                        k > 0 ? incU : nullptr, tk + 1, packets(), call(), 2 * k + 1, status, wait_limit, env,
+                        k > 0 ? incU : nullptr, tk + kSolveCtas, packets(), call(), 2 * k + 1, status, wait_limit, env,
                         active));
     launches += 2;
     return NL_OK;
@@ -324,17 +324,19 @@ class SchurCoreT final : public SchurCore {
   // [0] the call's number, then two packets per row
   unsigned long long* call() const { return packets_.as<unsigned long long>(); }
   ulonglong2* packets() const { return packets_.as<ulonglong2>() + 1; }
+  // per solve: one ticket per rank of a cluster, forward and backward
+  int tickets() const { return 2 * kSolveCtas * solve_slots(); }
   int solve_slots() const { return 1 + std::max(0, std::min(refine_sweeps, 3)); }
 
-  // The forward solve with tile 0 left out: the ticket counter starts at
-  // kSolveCtas, so the CTAs take tiles 1 .. ntiles - 1 and each waits for tile 0's
+  // The forward solve with tile 0 left out: the tickets start at 1, so the
+  // clusters take tiles 1 .. ntiles - 1 and each CTA waits for tile 0's
   // packets, which nothing publishes.  Every CTA's wait runs out after wait_limit
   // polls, records ST_SPIN_TIMEOUT and returns before it writes anything but
   // packets of this call; no access leaves the buffers (tiles 1 .. ntiles - 1 of
   // L and Linv).
   nl_status enqueue_solve_withheld(int* status) override {
     if (ntiles_ < 2) return NL_ERR_STATE;
-    solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), 2 * solve_slots(), kSolveCtas, call());
+    solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), tickets(), 1, call());
     trsv_fwd_kernel<T><<<kSolveCtas*(ntiles_ - 1), SVT, trsv_smem<T>(), st_>>>(
         S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), nullptr, 0, y_.as<double>(),
         tickets_.as<int>(), packets(), call(), 0, status, wait_limit, nullptr, nullptr);
@@ -709,7 +711,7 @@ class SchurCoreT final : public SchurCore {
     if (tm) NL_CUDA(cudaEventRecord(ev_[0], st_));
     nvtxRangePushA("nl:vinv+wvinv_bs");
     NL_CUDA(launch_next(vinv_kernel<T, BC>, dim3(cdiv(std::max(np_, 1), 128)), 128, 0, st_, pdl && !tm, d_, V_.as<T>(),
-                        Vinv_.as<T>(), lam, status, sched_.as<int>(), tickets_.as<int>(), 2 * solve_slots(), call(),
+                        Vinv_.as<T>(), lam, status, sched_.as<int>(), tickets_.as<int>(), tickets(), call(),
                         active));
     if (tm) NL_CUDA(cudaEventRecord(ev_[1], st_));
     if (nci_ > 0)
@@ -790,7 +792,7 @@ class SchurCoreT final : public SchurCore {
       NL_CUDA(launch_next(wvinv_bs_kernel<T, BC, kWvNT>, dim3(nci_), kWvNT, wvinv_smem<T, BC, kWvNT>(), st_, pdl, d_,
                           W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(), bV_.as<T>(), bS_.as<double>(), nullptr));
     launches++;
-    solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), 2 * solve_slots(), 0, call());
+    solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), tickets(), 0, call());
     launches++;
     nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
