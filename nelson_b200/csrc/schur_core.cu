@@ -189,7 +189,8 @@ class SchurCoreT final : public SchurCore {
     NL_TRY(packets_.alloc(16 * (2 * (size_t)ld_ + 1)));
     NL_CUDA(cudaMemsetAsync(packets_.p, 0, packets_.bytes, st_));
     NL_TRY(S_.alloc(sizeof(T) * (size_t)ld_ * ld_));
-    s_cleared_ = false;
+    NL_TRY(s_dirty_.alloc(sizeof(int)));
+    NL_CUDA(cudaMemsetAsync(s_dirty_.p, 1, s_dirty_.bytes, st_));
     need_s0_ = refine_sweeps > 0 || keep_schur;
     if (need_s0_) NL_TRY(S0_.alloc(sizeof(T) * (size_t)ld_ * ld_));
     if (sizeof(T) == 4 && use_tc) {
@@ -721,19 +722,18 @@ class SchurCoreT final : public SchurCore {
     if (tm) NL_CUDA(cudaEventRecord(ev_[2], st_));
     nvtxRangePop();
     nvtxRangePushA("nl:schur");
-    // The first time the whole of S (and S0); afterwards only the envelope,
-    // whose outside stays exactly zero -- but only where every kernel that
-    // writes S honours `active`.  The FP64 path's cuBLAS trailing updates
+    // The first time the whole of S (and S0); afterwards only the envelope
+    // (s_dirty_), whose outside stays exactly zero -- but only where every kernel
+    // that writes S honours `active`.  The FP64 path's cuBLAS trailing updates
     // cannot: the sub-iterations that a device-side LM loop leaves in flight
     // after it has finished still subtract L L' from the stale factor, and the
     // overflow that builds up there reaches tiles outside the envelope
     // (0 * inf).  That path clears all of S every time.
     const bool unpredicated_writes = sizeof(T) == 8 && cublas_ != nullptr;
-    const bool full = !s_cleared_ || unpredicated_writes;  // not predicated
     NL_CUDA(launch_next(clear_kernel<T>, dim3(ld_), 128, 0, st_, pdl && !tm, S_.as<T>(),
                         need_s0_ ? S0_.as<T>() : nullptr, n_,
-                        ld_, NB, full ? nullptr : env_dev_.as<int>(), full ? nullptr : active));
-    s_cleared_ = true;
+                        ld_, NB, unpredicated_writes ? nullptr : env_dev_.as<int>(), s_dirty_.as<int>(),
+                        unpredicated_writes ? nullptr : active));
     launches++;
     {
       using Cfg = SchurCfg<T, BC>;
@@ -768,7 +768,8 @@ class SchurCoreT final : public SchurCore {
     if ((s = enqueue_solves(status, active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[5], st_));
     NL_CUDA(launch_next(backsub_kernel<T, BC>, dim3(cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128)), 128, 0,
-                        st_, pdl && !tm, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status, active));
+                        st_, pdl && !tm, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status,
+                        s_dirty_.as<int>(), active));
     launches++;
     if (tm) NL_CUDA(cudaEventRecord(ev_[6], st_));
     NL_CUDA(cudaGetLastError());
@@ -797,7 +798,8 @@ class SchurCoreT final : public SchurCore {
     nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
     NL_CUDA(launch_next(backsub_kernel<T, BC>, dim3(cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128)), 128, 0,
-                        st_, pdl, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status, nullptr));
+                        st_, pdl, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status,
+                        nullptr, nullptr));
     launches++;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
@@ -902,7 +904,7 @@ class SchurCoreT final : public SchurCore {
   // envelope of S (host) and its first / last arrays on the device (solves)
   std::vector<int> env_first_, env_last_, env_run_;
   DevBuf env_dev_;
-  bool s_cleared_ = false;  // S / S0 have had their one full clear (enqueue_increment)
+  DevBuf s_dirty_;  // int: tiles of S / S0 outside the envelope may hold other values than zero (clear_kernel)
   // last tile row that panel k's TRSM and updates must cover
   int env_end(int k) const { return envelope ? env_run_[std::min(k, ntiles_ - 1)] : ntiles_ - 1; }
   DevBuf v_uid_, w_row_ptr_, w_col_, w_row_, w_col_ptr_, w_col_uid_, u_diag_, s_i_, s_j_, s_uuid_, s_ptr_, pa_, pb_, s_items_,

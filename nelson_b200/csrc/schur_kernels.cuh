@@ -421,18 +421,22 @@ static __global__ void __launch_bounds__(SchurCfg<T, BC>::kWarps * 32)
 }
 
 // Zero S (and S0), with the identity on the padded rows n .. ld - 1.  With
-// env_first only the tiles that can hold nonzeros: row r of tile row I over
-// columns [env_first[I] NB, (I + 1) NB), the Cholesky envelope.  The other tiles
-// are zero after the first full clear and stay exactly zero: the Schur blocks
+// env_first and *dirty zero only the tiles that can hold nonzeros: row r of tile
+// row I over columns [env_first[I] NB, (I + 1) NB), the Cholesky envelope.  The
+// other tiles are zero after a full clear and stay exactly zero: the Schur blocks
 // lie inside the envelope, and the factorisation writes only zeros there (TRSM
-// and trailing updates of zero tiles).  One CTA per row.
+// and trailing updates of zero tiles).  *dirty says on the device whether that holds
+// (set from the start, cleared by backsub_kernel), so that it is right for
+// launches that are captured, replayed or skipped by `active` as well.  One CTA per row.
 template <typename T>
 static __global__ void clear_kernel(T* __restrict__ S, T* __restrict__ S0, int n, int ld, int nb,
-                                    const int* __restrict__ env_first, const int* __restrict__ active) {
-  chain_start(active);
+                                    const int* __restrict__ env_first, const int* __restrict__ dirty,
+                                    const int* __restrict__ active) {
+  chain_start(dirty, active);
   if (active && !*active) return;
   const int r = blockIdx.x, I = r / nb;
-  const size_t c0 = env_first ? (size_t)env_first[I] * nb : 0, c1 = env_first ? (size_t)(I + 1) * nb : (size_t)ld;
+  const bool full = !env_first || *dirty != 0;
+  const size_t c0 = full ? 0 : (size_t)env_first[I] * nb, c1 = full ? (size_t)ld : (size_t)(I + 1) * nb;
   constexpr int EPV = 16 / (int)sizeof(T);  // elements per 16-byte store
   using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
   for (size_t c = c0 + (size_t)threadIdx.x * EPV; c < c1; c += (size_t)blockDim.x * EPV) {
@@ -457,7 +461,7 @@ template <typename T, int BC>
 static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T* __restrict__ W,
                                                              const T* __restrict__ Vinv, const T* __restrict__ bV,
                                                              double* xU, int nxu, double* __restrict__ xV,
-                                                             const int* __restrict__ ok_flag,
+                                                             const int* __restrict__ ok_flag, int* __restrict__ dirty,
                                                              const int* __restrict__ active) {
   constexpr int LW = Layout<T, BC>::W;
   constexpr int LV = Layout<T, BC>::V;
@@ -467,6 +471,8 @@ static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T
   if (active && !*active) return;
   const int l = threadIdx.x & (LP - 1);
   const bool failed = ok_flag && *ok_flag != 0;  // zero increment
+  // last kernel of a call that formed S (dirty given): its clear has run (clear_kernel)
+  if (dirty && blockIdx.x == 0 && threadIdx.x == 0) *dirty = 0;
   if (failed) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
     for (long long i = t; i < nxu; i += nt) xU[i] = 0.0;
