@@ -425,9 +425,10 @@ static __global__ void __launch_bounds__(SchurCfg<T, BC>::kWarps * 32)
 // row I over columns [env_first[I] NB, (I + 1) NB), the Cholesky envelope.  The
 // other tiles are zero after a full clear and stay exactly zero: the Schur blocks
 // lie inside the envelope, and the factorisation writes only zeros there (TRSM
-// and trailing updates of zero tiles).  *dirty says on the device whether that holds
-// (set from the start, cleared by backsub_kernel), so that it is right for
-// launches that are captured, replayed or skipped by `active` as well.  One CTA per row.
+// and trailing updates of zero tiles) as long as it does not fail.  *dirty says on the
+// device whether that holds (set from the start and by a failed call, cleared by
+// any other, in backsub_kernel), so that it is right for launches that are captured,
+// replayed or skipped by `active` as well.  One CTA per row.
 template <typename T>
 static __global__ void clear_kernel(T* __restrict__ S, T* __restrict__ S0, int n, int ld, int nb,
                                     const int* __restrict__ env_first, const int* __restrict__ dirty,
@@ -471,8 +472,9 @@ static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T
   if (active && !*active) return;
   const int l = threadIdx.x & (LP - 1);
   const bool failed = ok_flag && *ok_flag != 0;  // zero increment
-  // last kernel of a call that formed S (dirty given): its clear has run (clear_kernel)
-  if (dirty && blockIdx.x == 0 && threadIdx.x == 0) *dirty = 0;
+  // last kernel of a call that formed S (dirty given): its clear has run; a failed
+  // factorisation overflows, and 0 * inf is not zero outside the envelope (clear_kernel)
+  if (dirty && blockIdx.x == 0 && threadIdx.x == 0) *dirty = failed ? 1 : 0;
   if (failed) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
     for (long long i = t; i < nxu; i += nt) xU[i] = 0.0;
