@@ -77,6 +77,12 @@ struct nl_problem {
   std::vector<double> unr_mu;              // damping of the recorded steps
   int unr_n = -1;                          // recorded steps (-1: none)
   cudaGraphExec_t sub_exec = nullptr;       // captured LM sub-iteration without trace (batched solves)
+  // A setting that the launches carry (solver kind, wait bound) has changed: the
+  // next batched solve captures again.
+  void drop_capture() {
+    if (sub_exec) cudaGraphExecDestroy(sub_exec);
+    sub_exec = nullptr;
+  }
   cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
   float eval_ms = 0;
   int have_jac = 0;
@@ -1126,8 +1132,11 @@ nl_status nl_lm_solve_batch(nl_problem** hs, int n, const nl_lm_settings* st, nl
     q.reason = NL_MAX_ITERATION_REACHED;
     lm_begin(&q);
     NL_CUDA(cudaMemcpyAsync(h->lm, &q, sizeof(LmDev), cudaMemcpyHostToDevice, h->st));
-    if (q.done) finished[i] = 1;
-    // one LM sub-iteration as a CUDA graph, captured once per handle
+    if (q.done) {
+      finished[i] = 1;
+      continue;
+    }
+    // one LM sub-iteration as a CUDA graph, captured once per handle and settings
     if (!h->sub_exec) {
       nl_status r = capture_subiteration(h, nullptr, &h->sub_exec);
       if (r != NL_OK) return r;
@@ -1648,7 +1657,9 @@ nl_status nl_set_solver_kind(nl_problem* h, int kind) {
   NL_CHECK_H(h);
   if (kind != NL_SOLVER_DENSE && kind != NL_SOLVER_ENVELOPE) return NL_ERR_ARG;
   if (!h->core) return NL_ERR_STATE;
-  h->core->envelope = kind == NL_SOLVER_ENVELOPE ? 1 : 0;
+  const int envelope = kind == NL_SOLVER_ENVELOPE ? 1 : 0;
+  if (h->core->envelope != envelope) h->drop_capture();
+  h->core->envelope = envelope;
   return NL_OK;
 }
 
@@ -1661,7 +1672,9 @@ nl_status nl_set_timing_detail(nl_problem* h, int detail) {
 nl_status nl_set_wait_limit(nl_problem* h, long long polls) {
   NL_CHECK_H(h);
   if (!h->core) return NL_ERR_STATE;
-  h->core->wait_limit = polls > 0 ? polls : kSpinLimit;
+  const long long limit = polls > 0 ? polls : kSpinLimit;
+  if (h->core->wait_limit != limit) h->drop_capture();
+  h->core->wait_limit = limit;
   return NL_OK;
 }
 

@@ -9,6 +9,35 @@ from nelson_b200.problems import make_config, problem_from_pairs
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("prec", [N.PREC_FP64, N.PREC_MIXED])
+def test_settings_after_the_capture(prec):
+    """A wait bound of one poll makes every solve of several tiles give up, so each
+    sub-iteration is rejected; with the default bound the first result comes back.
+    The solver kind, set after the capture, gives the same parameters (the envelope
+    solver skips zero tiles only)."""
+    p = make_config(1, 0.3)  # 60 cameras x 9: five tiles
+    g = N.BAProblemGPU.from_ba(p, precision=prec)
+    s = N.LMSettings(maxNumIt=3, maxNumSubIt=4)
+
+    def solve():
+        g.set_params(p.cams, p.pts)
+        reason, chi2, its, _ = N.lm_solve_batch([g], s)
+        return reason[0], float(chi2[0]), int(its[0]), g.get_params()[1]
+
+    first = solve()
+    assert first[2] == 3
+    g.set_wait_limit(1)
+    limited = solve()
+    assert limited[2] == 0 and limited[0] == "MaxSubIterationReached"
+    g.set_wait_limit(0)
+    again = solve()
+    assert again[:3] == first[:3] and np.array_equal(again[3], first[3])
+    g.set_solver_kind(N.SOLVER_ENVELOPE)
+    env = solve()
+    assert env[2] == 3 and env[1] == pytest.approx(first[1], rel=1e-12)
+    g.close()
+
+
 @pytest.mark.parametrize("kind", [N.SOLVER_DENSE, N.SOLVER_ENVELOPE])
 def test_no_iteration_then_increment(kind):
     """A batch that may not iterate captures nothing that the next call relies on: the
