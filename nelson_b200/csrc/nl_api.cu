@@ -13,6 +13,7 @@
 
 #include "ba_kernels.cuh"
 #include "adjoint.cuh"
+#include "pinned.h"
 #include "problem_view.h"
 #include "schur_core.cuh"
 #include "unroll.cuh"
@@ -69,6 +70,7 @@ struct nl_problem {
   int* status = nullptr;  // solver status (inside LmDev)
   static constexpr size_t kPinBytes = 4096, kPinParams = 2 << 20;
   double* host_pin = nullptr;  // kPinBytes, then the parameters up to kPinParams
+  size_t pin_params = 0;       // bytes for the parameters: all of them or none
   double lam_host[2] = {0, 0};
   DevBuf d_lam;
   long long launches = 0;
@@ -101,7 +103,7 @@ struct nl_problem {
   int nc_all() const { return desc.nc_var + desc.nc_fix; }
   int np_all() const { return desc.np_var + desc.np_fix; }
   size_t param_bytes() const { return sizeof(double) * ((size_t)nc_all() * desc.bc + (size_t)3 * np_all()); }
-  bool params_pinned() const { return param_bytes() <= kPinParams; }
+  bool params_pinned() const { return pin_params >= param_bytes(); }
   double* param_pin() const { return host_pin + kPinBytes / sizeof(double); }
 };
 
@@ -613,7 +615,16 @@ nl_status nl_create(const nl_problem_desc* d, nl_problem** out) {
   h->scal = h->d_scal.as<double>();
   h->lm = h->d_lm.as<LmDev>();
   h->status = reinterpret_cast<int*>(h->d_lam.as<double>() + 2);
-  NL_CUDA(cudaMallocHost(&h->host_pin, nl_problem::kPinBytes + (h->params_pinned() ? h->param_bytes() : 0)));
+  auto host_alloc = [](void** p, size_t bytes) {
+    const bool ok = cudaMallocHost(p, bytes) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+  };
+  void* pin = nullptr;
+  if (!alloc_pinned(host_alloc, &pin, nl_problem::kPinBytes,
+                    h->param_bytes() <= nl_problem::kPinParams ? h->param_bytes() : 0, &h->pin_params))
+    return NL_ERR_CUDA;
+  h->host_pin = static_cast<double*>(pin);
   if ((s = upload_params(h.get())) != NL_OK) return s;  // identity cameras, origin points
   *out = h.release();
   return NL_OK;
