@@ -151,10 +151,11 @@ __device__ inline void cp_async_wait() {
 }
 
 // 1 / d and 1 / sqrt(d) of a pivot, clamped away from zero (a non-positive
-// pivot is flagged separately)
+// pivot is flagged separately).  Above 2^126 the reciprocal is subnormal and must not be
+// flushed to zero: the elimination would leave the column out.
 __device__ __forceinline__ void pivot_inv(float d, float& ri, float& rs) {
   d = fmaxf(d, 1e-30f);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(d));
+  asm("rcp.approx.f32 %0, %1;" : "=f"(ri) : "f"(d));
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(d));
 }
 __device__ __forceinline__ void pivot_inv(double d, double& ri, double& rs) {
