@@ -418,6 +418,10 @@ class SchurCoreT final : public SchurCore {
       for (int j = 0; j < ncols && j < nt; j++) t += std::max(0, nt - std::max(j, rb));
       return t;
     };
+    // diagonal tiles among them (lower half only)
+    auto diag_tiles_of = [](int nt, int ncols, int rb) {
+      return (double)(ncols <= 0 ? nt : std::max(0, std::min(ncols, nt) - rb));
+    };
     // update with panels k .. k + npan - 1
     auto upd = [&](int k, int npan, int t0, int nt, int ncols, int rb, cudaStream_t st) -> nl_status {
       nt = std::min(nt, env_end(k + npan - 1) - t0 + 1);  // tile rows past the envelope get zero updates
@@ -430,7 +434,9 @@ class SchurCoreT final : public SchurCore {
       nev += 2;
       nupd++;
       launches++;
-      upd_bytes += tiles_of(nt, ncols, rb) * (double)NB * NB * sizeof(float) * 2;
+      const double tiles = tiles_of(nt, ncols, rb), dt = diag_tiles_of(nt, ncols, rb);
+      upd_bytes += tiles * (double)NB * NB * sizeof(float) * 2;
+      upd_flop += npan * (double)NB * NB * (2.0 * NB * (tiles - dt) + (NB + 1) * dt);
       return NL_OK;
     };
     // TRSM + pack of panel j's rows [r0, r0 + nrows) (absolute rows, tile aligned)
@@ -478,10 +484,6 @@ class SchurCoreT final : public SchurCore {
     };
     auto rec = [&](int e, cudaStream_t st) { return cudaEventRecord(dev_[e], st); };
     auto wait = [&](cudaStream_t st, int e) { return cudaStreamWaitEvent(st, dev_[e], 0); };
-    for (int k = 0; k + 1 < nT; k++) {
-      const double below = (double)ld_ - (double)(k + 1) * NB;
-      upd_flop += (double)NB * below * (below + 1);
-    }
     nl_status r;
     // panel 0
     if ((r = potrf(0)) != NL_OK) return r;
@@ -582,18 +584,6 @@ class SchurCoreT final : public SchurCore {
     return NL_OK;
   }
 
-  // tiles read and written per panel: block column k+1 and the triangle below it,
-  // both cut at the envelope
-  double update_bytes() const {
-    double tiles = 0;
-    for (int k = 0; k + 1 < ntiles_; k++) {
-      const int last = env_end(k);
-      const double na = std::max(0, last - k), nb = std::max(0, last - k - 1);
-      tiles += na + nb * (nb + 1) / 2;
-    }
-    return tiles * (double)NB * NB * sizeof(T) * 2;
-  }
-
   // The FP64 schedule (cuBLAS trailing updates).  Per panel k:
   //   main  potrf(k); [wait the column update of k] TRSM of row tile k+1; [wait
   //         B(k-1)] tile (k+1, k+1)
@@ -615,7 +605,14 @@ class SchurCoreT final : public SchurCore {
     double* S = reinterpret_cast<double*>(S_.p);
     auto rec = [&](int e, cudaStream_t st) { return cudaEventRecord(dev_[e], st); };
     auto wait = [&](cudaStream_t st, int e) { return cudaStreamWaitEvent(st, dev_[e], 0); };
-    double upd_flop = 0;
+    double upd_flop = 0, upd_bytes = 0;
+    int nupd = 0;
+    // a cuBLAS update, in flops and in tiles
+    auto count = [&](double flop, double tiles) {
+      upd_flop += flop;
+      upd_bytes += tiles * (double)NB * NB * sizeof(double) * 2;
+      nupd++;
+    };
     std::vector<char> timed(4 * (size_t)nT, 0);
     bool pending_b = false, pending_col = false, early = pdl;
     for (int k = 0; k < nT; k++) {
@@ -623,8 +620,7 @@ class SchurCoreT final : public SchurCore {
                            Linv_.as<T>(), status, active));
       launches++;
       if (k + 1 >= nT) break;
-      const int below = ld_ - (k + 1) * NB, last = std::min(nT - 1, env_end(k));  // last tile row with nonzeros
-      upd_flop += (double)NB * below * (below + 1);
+      const int last = std::min(nT - 1, env_end(k));  // last tile row with nonzeros
       early = false;
       if (last <= k) continue;  // nothing below the diagonal tile
       NL_CUDA(rec(EV_POTRF, st_));
@@ -655,6 +651,7 @@ class SchurCoreT final : public SchurCore {
       }
       if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 1], st3_));
       timed[4 * k] = tm;
+      count(2.0 * NB * NB * rows, rows / NB);
       NL_CUDA(rec(EV_A1R, st3_));
       pending_col = true;
       NL_CUDA(wait(st2_, EV_PACKF));
@@ -672,6 +669,7 @@ class SchurCoreT final : public SchurCore {
       }
       if (tm) NL_CUDA(cudaEventRecord(upd_ev_[4 * k + 3], st2_));
       timed[4 * k + 2] = tm;
+      count((double)NB * rows * (rows + 1.0), 0.5 * (rows / NB) * (rows / NB + 1));
       NL_CUDA(rec(EV_B, st2_));
       pending_b = true;
     }
@@ -692,9 +690,9 @@ class SchurCoreT final : public SchurCore {
           tot += ms;
         }
       times.update_ms = tot;
-      times.update_launches = nT - 1;
+      times.update_launches = nupd;
       times.update_flop = upd_flop;
-      times.update_bytes = update_bytes();
+      times.update_bytes = upd_bytes;
     }
     return NL_OK;
   }
