@@ -322,6 +322,14 @@ class SchurCoreT final : public SchurCore {
     }
     return s;
   }
+  nl_status enqueue_backsub(bool early, int* status, int* dirty, const int* active) {
+    const int lanes = backsub_lanes<T>(np_, W_.bytes);
+    auto kern = lanes == 1 ? backsub_kernel<T, BC, 1> : backsub_kernel<T, BC, kBackLanes<T>>;
+    NL_CUDA(launch_next(kern, dim3(cdiv((long long)lanes * std::max(np_, 1), 128)), 128, 0, st_, early, d_, W_.as<T>(),
+                        Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status, dirty, active));
+    launches++;
+    return NL_OK;
+  }
   // [0] the call's number, then two packets per row
   unsigned long long* call() const { return packets_.as<unsigned long long>(); }
   ulonglong2* packets() const { return packets_.as<ulonglong2>() + 1; }
@@ -765,10 +773,7 @@ class SchurCoreT final : public SchurCore {
     NvtxRange rs("nl:solve+backsub");
     if ((s = enqueue_solves(status, active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[5], st_));
-    NL_CUDA(launch_next(backsub_kernel<T, BC>, dim3(cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128)), 128, 0,
-                        st_, pdl && !tm, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status,
-                        s_dirty_.as<int>(), active));
-    launches++;
+    if ((s = enqueue_backsub(pdl && !tm, status, s_dirty_.as<int>(), active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[6], st_));
     NL_CUDA(cudaGetLastError());
     if (tm) {
@@ -795,10 +800,7 @@ class SchurCoreT final : public SchurCore {
     launches++;
     nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
-    NL_CUDA(launch_next(backsub_kernel<T, BC>, dim3(cdiv((long long)kBackLanes<T> * std::max(np_, 1), 128)), 128, 0,
-                        st_, pdl, d_, W_.as<T>(), Vinv_.as<T>(), bV_.as<T>(), incU, ld_, incV, status,
-                        nullptr, nullptr));
-    launches++;
+    if ((s = enqueue_backsub(pdl, status, nullptr, nullptr)) != NL_OK) return s;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
   }

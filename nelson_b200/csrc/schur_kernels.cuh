@@ -450,15 +450,25 @@ static __global__ void clear_kernel(T* __restrict__ S, T* __restrict__ S0, int n
 }
 
 // ---------------------------------------------------------------------------
-// Eight lanes per point: lane l holds the 16-byte piece l of each of
-// the point's W blocks, so a block is read as one run.  FP64 sixteen lanes.  Bound
-// by the latency of the index chain (point -> W block -> camera).  375k blocks of
-// 9x3, a lane per point -> now: FP32 30 -> 22 us, FP64 49 -> 35 us; 1,500 cameras,
-// where W exceeds L2, 314 -> 178 us; 432 cameras, where it does not, 51 -> 63 us.
-// Half as many lanes: 33, 58, 190, 71 us.
+// Lanes == kBackLanes: eight lanes per point, lane l holds the 16-byte piece l of each
+// of the point's W blocks, so a block is read as one run; FP64 sixteen lanes.  Bound
+// by the latency of the index chain (point -> W block -> camera).
+// Lanes == 1: a thread per point, its block in registers.  The lanes of a point repeat
+// its index chain and add up at the end; where the points alone fill the chip and
+// W is not far larger than L2, a thread each is the faster one (backsub_lanes).
+// us, thread / lanes (9x3 blocks, W in MB): FP32 30k points, 23 MB 21 / 15; 50k, 42 MB
+// 30 / 22; 100k, 34 MB 17 / 22; 150k, 59 MB 27 / 38; 150k, 117 MB 50 / 62; 270k, 212 MB
+// 89 / 99; 500k, 392 MB 311 / 177.  FP64 50k, 84 MB 47 / 41; 100k, 67 MB 26 / 41; 150k,
+// 235 MB 76 / 100; 270k, 424 MB 293 / 168.
 template <typename T>
 constexpr int kBackLanes = sizeof(T) == 4 ? 8 : 16;
-template <typename T, int BC>
+// Lanes for np points and w_bytes of W.  75,000 points are even (FP32 34 / 33 us, FP64
+// 54 / 56); between 235 and 392 MB of W the lanes begin to win.
+template <typename T>
+inline int backsub_lanes(int np, size_t w_bytes) {
+  return np >= (1 << 16) && w_bytes <= ((size_t)256 << 20) ? 1 : kBackLanes<T>;
+}
+template <typename T, int BC, int LANES>
 static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T* __restrict__ W,
                                                              const T* __restrict__ Vinv, const T* __restrict__ bV,
                                                              double* xU, int nxu, double* __restrict__ xV,
@@ -467,7 +477,7 @@ static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T
   constexpr int LW = Layout<T, BC>::W;
   constexpr int LV = Layout<T, BC>::V;
   using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV, LP = kBackLanes<T>, NP = (PW + LP - 1) / LP;
+  constexpr int EPV = 16 / (int)sizeof(T), PW = LW / EPV, LP = LANES, NP = (PW + LP - 1) / LP;
   chain_start(W, Vinv, bV, ok_flag, active);
   if (active && !*active) return;
   const int l = threadIdx.x & (LP - 1);
@@ -482,6 +492,30 @@ static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T
     return;
   }
   const int p = group_item(blockIdx.x, 128, threadIdx.x, LP);
+  if constexpr (LANES == 1) {
+    if (p >= d.np) return;
+    double t[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) t[k] = -(double)bV[3 * (size_t)p + k];
+    const int s1 = d.w_col_ptr[p + 1];
+    for (int s = d.w_col_ptr[p]; s < s1; s++) {
+      const int q = d.w_col_uid[s];
+      const double* x = xU + (size_t)d.w_row[q] * BC;
+      __align__(16) T w[LW];
+#pragma unroll
+      for (int i = 0; i < PW; i++)
+        reinterpret_cast<V16*>(w)[i] = reinterpret_cast<const V16*>(W + (size_t)q * LW)[i];
+#pragma unroll
+      for (int i = 0; i < BC; i++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) t[k] -= (double)w[3 * i + k] * x[i];
+    }
+    const T* v = Vinv + (size_t)p * LV;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      xV[3 * (size_t)p + k] = (double)v[3 * k] * t[0] + (double)v[3 * k + 1] * t[1] + (double)v[3 * k + 2] * t[2];
+    return;
+  }
   if (group_item(blockIdx.x, 128, threadIdx.x & ~31, LP) >= d.np) return;  // whole warps leave
   const bool valid = p < d.np;
   const int s0 = valid ? d.w_col_ptr[p] : 0, s1 = valid ? d.w_col_ptr[p + 1] : 0;
