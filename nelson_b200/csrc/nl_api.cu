@@ -310,17 +310,18 @@ template <typename T, int BC>
 nl_status enqueue_eval_t(nl_problem* h, bool hessian, double* chi2_out, double* maxb_out, const int* active) {
   if (chi2_out) {
     NL_CUDA(launch_next(cost_kernel<BC, kCostNT>, dim3(std::max(1, std::min(kCostCTAs, cdiv(h->ba.ne, kCostNT)))),
-                        kCostNT, 0, h->st, h->core->pdl, h->ba, h->d_part.as<double>(), h->d_cnt.as<int>(), chi2_out, active));
+                        kCostNT, 0, h->st, h->core->pdl(), h->ba, h->d_part.as<double>(), h->d_cnt.as<int>(), chi2_out,
+                        active));
     h->launches++;
   }
   if (hessian) {
     if (h->nci > 0)
       NL_CUDA(launch_next(cam_pass_kernel<T, BC, kCamNT>, dim3(h->nci, h->cam_ctas), kCamNT,
-                          cam_pass_smem<T, BC, kCamNT>(), h->st, h->core->pdl, h->ba, (T*)h->core->dU(), (T*)h->core->dW(),
-                          (T*)h->core->dbU(), h->d_cam_part.as<T>(), h->d_cam_count.as<int>(), active));
+                          cam_pass_smem<T, BC, kCamNT>(), h->st, h->core->pdl(), h->ba, (T*)h->core->dU(),
+                          (T*)h->core->dW(), (T*)h->core->dbU(), h->d_cam_part.as<T>(), h->d_cam_count.as<int>(), active));
     if (h->desc.np_var > 0)
       NL_CUDA(launch_next(pt_pass_kernel<T, BC, 128>, dim3(cdiv(4LL * h->desc.np_var, 128)), 128, 0, h->st,
-                          h->core->pdl,
+                          h->core->pdl(),
                           h->ba, (T*)h->core->dV(), (T*)h->core->dbV(), active));
     h->launches += 2;
     nl_status s = h->core->enqueue_maxabs_b(maxb_out, active);
@@ -344,11 +345,11 @@ nl_status enqueue_oplus(nl_problem* h, const int* active) {
   const int cb = cdiv(h->nci, 256), grid = cb + cdiv(3LL * h->desc.np_var, 256);
   if (grid > 0) {
     if (h->desc.bc == 9)
-      NL_CUDA(launch_next(oplus_kernel<9>, dim3(grid), 256, 0, h->st, h->core->pdl, h->cam.as<double>(), h->ba.cam_slot,
-                          h->nci, h->core->incU, cb, h->pt.as<double>(), h->desc.np_var, h->core->incV, active));
+      NL_CUDA(launch_next(oplus_kernel<9>, dim3(grid), 256, 0, h->st, h->core->pdl(), h->cam.as<double>(),
+                          h->ba.cam_slot, h->nci, h->core->incU, cb, h->pt.as<double>(), h->desc.np_var, h->core->incV, active));
     else
-      NL_CUDA(launch_next(oplus_kernel<6>, dim3(grid), 256, 0, h->st, h->core->pdl, h->cam.as<double>(), h->ba.cam_slot,
-                          h->nci, h->core->incU, cb, h->pt.as<double>(), h->desc.np_var, h->core->incV, active));
+      NL_CUDA(launch_next(oplus_kernel<6>, dim3(grid), 256, 0, h->st, h->core->pdl(), h->cam.as<double>(),
+                          h->ba.cam_slot, h->nci, h->core->incU, cb, h->pt.as<double>(), h->desc.np_var, h->core->incV, active));
   }
   h->launches++;
   NL_CUDA(cudaGetLastError());
@@ -376,12 +377,12 @@ nl_status enqueue_subiteration(nl_problem* h, double* trace) {
   if ((r = h->core->enqueue_inc_dot(s, h->d_part.as<double>() + 4096, trace)) != NL_OK) return r;
   if ((r = enqueue_oplus(h, &s->apply)) != NL_OK) return r;
   if ((r = enqueue_eval(h, false, &s->chi2_new, nullptr, &s->apply)) != NL_OK) return r;
-  NL_CUDA(launch_next(lm_decide_kernel, dim3(1), 1, 0, h->st, h->core->pdl, s, trace));
+  NL_CUDA(launch_next(lm_decide_kernel, dim3(1), 1, 0, h->st, h->core->pdl(), s, trace));
   if ((r = enqueue_copy_params(h, false, &s->rollback)) != NL_OK) return r;
   // update(true) at the accepted point (GN: after every step), then backup
   if ((r = enqueue_eval(h, true, nullptr, &s->maxAbsB, &s->do_jac)) != NL_OK) return r;
   if ((r = enqueue_copy_params(h, true, &s->do_jac)) != NL_OK) return r;
-  NL_CUDA(launch_next(lm_after_jac_kernel, dim3(1), 1, 0, h->st, h->core->pdl, s, h->scal, trace));
+  NL_CUDA(launch_next(lm_after_jac_kernel, dim3(1), 1, 0, h->st, h->core->pdl(), s, h->scal, trace));
   h->launches += 2;
   NL_CUDA(cudaGetLastError());
   return NL_OK;

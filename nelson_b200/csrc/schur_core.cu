@@ -8,12 +8,17 @@ namespace nl {
 namespace {
 
 constexpr int kNT = 256, kWvNT = 256;
-// Programmatic dependent launches up to this many W blocks: small systems are bound
-// by the 1.8 us between two kernels (20 cameras, 867 -> 691 us per solve; 64
-// cameras 1,590 -> 1,322 us); on large ones the CTAs that wait on the chip cost the
-// running kernels as much as is saved (200 cameras, 375k blocks: 8.85 / 8.87 ms,
-// FP64 12.8 / 13.0 ms).
-constexpr int kPdlBlocks = 1 << 16;
+// Programmatic dependent launches (launch_next) up to this many W blocks, and in dense
+// systems up to this many tiles.  They save the 1.2 us between two kernels: LM solves
+// without / with them, 2,800 W blocks 771 / 653 us (mixed 810 / 669), 27,500 1,337 / 1,159,
+// 63,500 (900 rows) 2,528 / 2,395.  A kernel that waits on the chip holds shared memory
+// that the running one has less L1 for.  With many W blocks that costs the passes more
+// than is saved: the saving is 6 % at 105k blocks (2,605 / 2,457), 2 % at 375k (5,475 /
+// 5,361), and at 1.05 M they lose 6 % (9,118 / 9,681, mixed 7,236 / 7,647).  So does the
+// refinement residual of many dense tiles: 31 tiles 6,720 / 6,517, 57 tiles 13,177 /
+// 13,226, 106 tiles 33,542 / 33,864; within an envelope it does not (pose graphs of 47
+// tiles 6,850 / 6,809, of 141 tiles 19,740 / 19,508).
+constexpr int kPdlBlocks = 1 << 16, kPdlTiles = 48;
 constexpr int kRedCTAs = 296;  // 2 x 148 SMs for grid-stride reductions
 constexpr int kSymvChunks = 8;
 constexpr int kSchurMinChunk = 48, kSchurMaxChunk = 480;  // pairs of a Schur work item
@@ -27,6 +32,7 @@ class SchurCoreT final : public SchurCore {
 
   int n() const override { return n_; }
   int ld() const override { return ld_; }
+  bool pdl() const override { return small_w_ && (envelope || ntiles_ <= kPdlTiles); }
   void* dU() override { return U_.p; }
   void* dV() override { return V_.p; }
   void* dW() override { return W_.p; }
@@ -164,7 +170,7 @@ class SchurCoreT final : public SchurCore {
   } while (0)
     NL_TRY(U_.alloc(sizeof(T) * (size_t)std::max(nU_, 1) * Layout<T, BC>::U));
     NL_TRY(V_.alloc(sizeof(T) * (size_t)std::max(nV_, 1) * Layout<T, BC>::V));
-    pdl = nW_ <= kPdlBlocks;
+    small_w_ = nW_ <= kPdlBlocks;
     NL_TRY(W_.alloc(sizeof(T) * (size_t)std::max(nW_, 1) * Layout<T, BC>::W));
     NL_TRY(Y_.alloc(sizeof(T) * (size_t)std::max(nW_, 1) * Layout<T, BC>::W));
     NL_TRY(Vinv_.alloc(sizeof(T) * (size_t)std::max(np_, 1) * Layout<T, BC>::V));
@@ -298,11 +304,11 @@ class SchurCoreT final : public SchurCore {
     int* tk = tickets_.as<int>() + 2 * kSolveCtas * (k % solve_slots());
     if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(tk, 0, 2 * kSolveCtas * sizeof(int), st_));
     const int grid = kSolveCtas * ntiles_;
-    NL_CUDA(launch_next(trsv_fwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl && !timing, S_.as<T>(), ld_,
+    NL_CUDA(launch_next(trsv_fwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl() && !timing, S_.as<T>(), ld_,
                         ntiles_,
                         Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), k > 0 ? part_.as<double>() : nullptr,
                         kSymvChunks, y_.as<double>(), tk, packets(), call(), 2 * k, status, wait_limit, env, active));
-    NL_CUDA(launch_next(trsv_bwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl && !timing, S_.as<T>(), ld_,
+    NL_CUDA(launch_next(trsv_bwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl() && !timing, S_.as<T>(), ld_,
                         ntiles_,
                         Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
                         k > 0 ? incU : nullptr, tk + kSolveCtas, packets(), call(), 2 * k + 1, status, wait_limit, env,
@@ -315,7 +321,7 @@ class SchurCoreT final : public SchurCore {
     nl_status s = enqueue_solve(0, status, active);
     for (int it = 0; it < refine_sweeps && need_s0_ && s == NL_OK; it++) {
       auto symv = envelope ? symv_partial_kernel<T, kSymvChunks, true> : symv_partial_kernel<T, kSymvChunks, false>;
-      NL_CUDA(launch_next(symv, dim3(ntiles_, kSymvChunks), SV, 0, st_, pdl && !timing, S0_.as<T>(), ld_, ntiles_, incU,
+      NL_CUDA(launch_next(symv, dim3(ntiles_, kSymvChunks), SV, 0, st_, pdl() && !timing, S0_.as<T>(), ld_, ntiles_, incU,
                           part_.as<double>(), env_dev_.as<int>(), active));
       launches++;
       s = enqueue_solve(1 + it, status, active);
@@ -483,7 +489,7 @@ class SchurCoreT final : public SchurCore {
       const int e = 8 * nT + 2 * j;  // timing events after the update events
       if (tmc) cudaEventRecord(upd_ev_[e], st_);
       // a programmatic dependent of the Schur formation or the diagonal update before it
-      NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, potrf_smem<T>(), (j > 0 || pdl) && !tmc, S_.as<T>(), ld_, j,
+      NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, potrf_smem<T>(), (j > 0 || pdl()) && !tmc, S_.as<T>(), ld_, j,
                            Linv_.as<T>(), status, active));
       if (tmc) cudaEventRecord(upd_ev_[e + 1], st_);
       npev = j + 1;
@@ -622,7 +628,7 @@ class SchurCoreT final : public SchurCore {
       nupd++;
     };
     std::vector<char> timed(4 * (size_t)nT, 0);
-    bool pending_b = false, pending_col = false, early = pdl;
+    bool pending_b = false, pending_col = false, early = pdl();
     for (int k = 0; k < nT; k++) {
       NL_CUDA(launch_chain(potrf_diag_kernel<T>, 1, PT, potrf_smem<T>(), early && !tm, S_.as<T>(), ld_, k,
                            Linv_.as<T>(), status, active));
@@ -717,13 +723,13 @@ class SchurCoreT final : public SchurCore {
     NvtxRange rg("nl:computeIncrement");
     if (tm) NL_CUDA(cudaEventRecord(ev_[0], st_));
     nvtxRangePushA("nl:vinv+wvinv_bs");
-    NL_CUDA(launch_next(vinv_kernel<T, BC>, dim3(cdiv(std::max(np_, 1), 128)), 128, 0, st_, pdl && !tm, d_, V_.as<T>(),
+    NL_CUDA(launch_next(vinv_kernel<T, BC>, dim3(cdiv(std::max(np_, 1), 128)), 128, 0, st_, pdl() && !tm, d_, V_.as<T>(),
                         Vinv_.as<T>(), lam, status, sched_.as<int>(), tickets_.as<int>(), tickets(), call(),
                         active));
     if (tm) NL_CUDA(cudaEventRecord(ev_[1], st_));
     if (nci_ > 0)
       NL_CUDA(launch_next(wvinv_bs_kernel<T, BC, kWvNT>, dim3(nci_), kWvNT, wvinv_smem<T, BC, kWvNT>(), st_,
-                          pdl && !tm, d_,
+                          pdl() && !tm, d_,
                           W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(), bV_.as<T>(), bS_.as<double>(), active));
     if (tm) NL_CUDA(cudaEventRecord(ev_[2], st_));
     nvtxRangePop();
@@ -736,7 +742,7 @@ class SchurCoreT final : public SchurCore {
     // overflow that builds up there reaches tiles outside the envelope
     // (0 * inf).  That path clears all of S every time.
     const bool unpredicated_writes = sizeof(T) == 8 && cublas_ != nullptr;
-    NL_CUDA(launch_next(clear_kernel<T>, dim3(ld_), 128, 0, st_, pdl && !tm, S_.as<T>(),
+    NL_CUDA(launch_next(clear_kernel<T>, dim3(ld_), 128, 0, st_, pdl() && !tm, S_.as<T>(),
                         need_s0_ ? S0_.as<T>() : nullptr, n_,
                         ld_, NB, unpredicated_writes ? nullptr : env_dev_.as<int>(), s_dirty_.as<int>(),
                         unpredicated_writes ? nullptr : active));
@@ -744,7 +750,7 @@ class SchurCoreT final : public SchurCore {
     {
       using Cfg = SchurCfg<T, BC>;
       const int grid = std::max(1, std::min(cdiv(nitems_, Cfg::kWarps), 148 * schur_occ_));
-      NL_CUDA(launch_next(schur_kernel<T, BC>, dim3(grid), Cfg::kWarps * 32, Cfg::kSmem, st_, pdl && !tm, d_,
+      NL_CUDA(launch_next(schur_kernel<T, BC>, dim3(grid), Cfg::kWarps * 32, Cfg::kSmem, st_, pdl() && !tm, d_,
                           U_.as<T>(),
                           Y_.as<T>(), W_.as<T>(), lam, S_.as<T>(), need_s0_ ? S0_.as<T>() : nullptr,
                           s_items_.as<SchurItem>(), nitems_, chunk_, s_slot_.as<int>(), s_part_.as<T>(),
@@ -763,7 +769,7 @@ class SchurCoreT final : public SchurCore {
         launches++;
       }
       if (s == NL_OK && ntiles_ > 1) {
-        NL_CUDA(launch_next(hop_mat_kernel<T>, dim3(ntiles_ - 1, 2 * kHopDepth, 4), 256, hop_smem<T>(), st_, pdl && !tm,
+        NL_CUDA(launch_next(hop_mat_kernel<T>, dim3(ntiles_ - 1, 2 * kHopDepth, 4), 256, hop_smem<T>(), st_, pdl() && !tm,
                             S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), active));
         launches++;
       }
@@ -773,7 +779,7 @@ class SchurCoreT final : public SchurCore {
     NvtxRange rs("nl:solve+backsub");
     if ((s = enqueue_solves(status, active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[5], st_));
-    if ((s = enqueue_backsub(pdl && !tm, status, s_dirty_.as<int>(), active)) != NL_OK) return s;
+    if ((s = enqueue_backsub(pdl() && !tm, status, s_dirty_.as<int>(), active)) != NL_OK) return s;
     if (tm) NL_CUDA(cudaEventRecord(ev_[6], st_));
     NL_CUDA(cudaGetLastError());
     if (tm) {
@@ -793,14 +799,14 @@ class SchurCoreT final : public SchurCore {
 
   nl_status enqueue_resolve(int* status) override {
     if (nci_ > 0)
-      NL_CUDA(launch_next(wvinv_bs_kernel<T, BC, kWvNT>, dim3(nci_), kWvNT, wvinv_smem<T, BC, kWvNT>(), st_, pdl, d_,
+      NL_CUDA(launch_next(wvinv_bs_kernel<T, BC, kWvNT>, dim3(nci_), kWvNT, wvinv_smem<T, BC, kWvNT>(), st_, pdl(), d_,
                           W_.as<T>(), Vinv_.as<T>(), Y_.as<T>(), bU_.as<T>(), bV_.as<T>(), bS_.as<double>(), nullptr));
     launches++;
     solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), tickets(), 0, call());
     launches++;
     nl_status s = enqueue_solves(status, nullptr);
     if (s != NL_OK) return s;
-    if ((s = enqueue_backsub(pdl, status, nullptr, nullptr)) != NL_OK) return s;
+    if ((s = enqueue_backsub(pdl(), status, nullptr, nullptr)) != NL_OK) return s;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
   }
@@ -818,7 +824,7 @@ class SchurCoreT final : public SchurCore {
 
   nl_status enqueue_maxabs_b(double* out, const int* active) override {
     const int grid = std::max(1, std::min(kRedCTAs, cdiv(n_ + 3 * np_, kNT)));
-    NL_CUDA(launch_next(maxabs_kernel<T, kNT>, dim3(grid), kNT, 0, st_, pdl, bU_.as<T>(), n_, bV_.as<T>(), 3 * np_,
+    NL_CUDA(launch_next(maxabs_kernel<T, kNT>, dim3(grid), kNT, 0, st_, pdl(), bU_.as<T>(), n_, bV_.as<T>(), 3 * np_,
                         part_.as<double>(), sched_.as<int>() + 2, out, active));
     launches++;
     NL_CUDA(cudaGetLastError());
@@ -827,7 +833,7 @@ class SchurCoreT final : public SchurCore {
 
   nl_status enqueue_inc_dot(LmDev* s, double* part, double* trace) override {
     const int grid = std::max(1, std::min(kRedCTAs, cdiv(n_ + 3 * np_, kNT)));
-    NL_CUDA(launch_next(inc_dot_kernel<T, kNT>, dim3(grid), kNT, 0, st_, pdl, incU, bU_.as<T>(), n_, incV,
+    NL_CUDA(launch_next(inc_dot_kernel<T, kNT>, dim3(grid), kNT, 0, st_, pdl(), incU, bU_.as<T>(), n_, incV,
                         bV_.as<T>(), 3 * np_, s, part, sched_.as<int>() + 3, trace));
     launches++;
     NL_CUDA(cudaGetLastError());
@@ -898,6 +904,7 @@ class SchurCoreT final : public SchurCore {
   int nci_ = 0, np_ = 0, nU_ = 0, nV_ = 0, nW_ = 0, nS_ = 0, n_ = 0, ld_ = 0, ntiles_ = 0;
   long long npairs_ = 0;
   int nitems_ = 0, chunk_ = 0, schur_occ_ = 1;  // work items of the Schur formation
+  bool small_w_ = false;  // at most kPdlBlocks W blocks
   bool need_s0_ = false;
   SchurDev d_{};
   DevBuf U_, V_, W_, Y_, Vinv_, bU_, bV_, bS_, incU_, incV_, y_, dx_, part_, Linv_, hop_, tickets_, packets_, S_, S0_, tcs_;

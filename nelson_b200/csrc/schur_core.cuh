@@ -92,6 +92,7 @@ class SchurCore {
   virtual nl_status enqueue_inc_dot(LmDev* s, double* part, double* trace) = 0;
   virtual int n() const = 0;
   virtual int ld() const = 0;
+  virtual bool pdl() const = 0;  // launch_next as programmatic dependents
   virtual nl_status get_hessian(double* U, double* V, double* W, double* bU, double* bV) = 0;
   virtual nl_status set_hessian(const double* U, const double* V, const double* W, const double* bU,
                                 const double* bV) = 0;
@@ -106,7 +107,6 @@ class SchurCore {
   double* incV = nullptr;  // device, 3 np
   int keep_schur = 0;      // keep an undamaged copy of S for nl_get_schur
   int refine_sweeps = 0;
-  bool pdl = false;  // launch_next as programmatic dependents (setup)
   int use_tc = 1;          // tensor-core trailing update (mixed)
   nl_phase_times times{};
   long long launches = 0;
