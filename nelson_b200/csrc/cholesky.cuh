@@ -1063,12 +1063,18 @@ static __global__ void __launch_bounds__(128) diag_update64_kernel(double* __res
 // the product with a 128 x 128 matrix, which in FP64 arithmetic on one SM takes
 // 1 us (16 conversions and 38 FMAs per clock), and by the way of the result to
 // the next tile.  A CTA waits for earlier tiles (forward; later ones backward) and for
-// the other CTAs of its own tile.  The launch is in clusters of kSolveCtas, whose CTAs
-// are on the chip together, and CTA r of each cluster takes its tile from ticket r: with
-// m clusters placed, the tickets hand out tiles 0 .. m - 1 and each of them has all of
-// its CTAs on the chip, however many other solves share it.  So every wait ends; each
-// is also bounded.  (Without clusters, partly placed tiles of about a hundred FP64 solves
-// at once could fill the chip.)
+// the other CTAs of its own tile.  CTA r of each kSolveCtas consecutive ones takes its
+// tile from ticket r, so that tiles are handed out in order, and every wait ends if
+// the CTAs of a tile do get onto the chip, however many other solves share it:
+// - in clusters of kSolveCtas they are there together (with m clusters placed, the
+//   tickets hand out tiles 0 .. m - 1, each complete);
+// - without, a launch holds at most kSolveCtas - 1 CTAs that wait for an unplaced one
+//   (those of complete tiles end, by induction over the tiles), and the device at most
+//   kMaxGrids launches: where the chip has room for many more CTAs than these, the
+//   unplaced ones find it.
+// solve_cluster takes clusters unless there is room for twice as many: systems of one
+// tile (FP32 two) stage less and go without.  A cluster launch costs the host 1.4 us (scan
+// alignment, one tile, 943 -> 959 us a solve).  Each wait is also bounded.
 //
 // A value is passed on with the tag of its solve as one 16-byte store and load:
 // the reader that finds the tag has the value, without barrier, release, flag and
@@ -1080,7 +1086,7 @@ static __global__ void __launch_bounds__(128) diag_update64_kernel(double* __res
 // hop, of which 0.7 us are the packet's way through L2; three hop matrices instead
 // of two change nothing).
 constexpr int kSolveCtas = 4, SVR = NB / kSolveCtas, SVT = 128;
-// rank of the CTA in its cluster (clusters of kSolveCtas consecutive CTAs)
+// rank of the CTA among the kSolveCtas consecutive ones of a cluster
 __device__ __forceinline__ int solve_rank() { return (int)(blockIdx.x % kSolveCtas); }
 static_assert(SVT == NB && SVR == 8 * (SVT / 32), "a thread fetches one row, a warp finishes eight");
 
@@ -1246,9 +1252,12 @@ struct OwnBlock {
   }
 };
 template <typename T>
-constexpr size_t trsv_smem() {  // Linv_I and the hop matrices
-  return (size_t)(1 + kHopDepth) * OwnBlock<T>::kBytes;
+constexpr size_t trsv_smem(int ntiles) {  // Linv_I and the hop matrices
+  return (size_t)(ntiles > kHopDepth ? 1 + kHopDepth : ntiles) * OwnBlock<T>::kBytes;
 }
+constexpr int kMaxGrids = 128;  // grids resident on a device at once, at most
+// CTAs per cluster of a solve where `slots` of its CTAs fit on the chip
+inline int solve_cluster(int slots) { return slots > 2 * (kSolveCtas - 1) * kMaxGrids ? 1 : kSolveCtas; }
 constexpr int kHopB = 64, kHopLd = kHopB + 4;  // output block, row length of a staged block
 template <typename T>
 constexpr size_t hop_smem() {
@@ -1383,7 +1392,7 @@ static __global__ void __launch_bounds__(256) hop_mat_kernel(const T* __restrict
 // `part` of a refinement residual.  Warp w, lane l: rows 8 w .. 8 w + 7 of the
 // CTA's, columns 4 l .. 4 l + 3.  pk: 2 x 128 ntiles packets (y, b - partial).
 template <typename T>
-static __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(SVT) trsv_fwd_kernel(
+static __global__ void __launch_bounds__(SVT) trsv_fwd_kernel(
     const T* __restrict__ L, int ld, int ntiles, const T* __restrict__ Linv, const T* __restrict__ hop,
     const double* __restrict__ b, const double* __restrict__ part, int nch, double* __restrict__ y,
     int* __restrict__ ticket, ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub,
@@ -1470,7 +1479,7 @@ static __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(SVT)
 // thread holds rows 32 w + (l >> 3) + 4 i, columns 4 (l & 7) .. + 3 of the CTA's.
 // `sum`, if given, gets x added (a refinement step).
 template <typename T>
-static __global__ void __cluster_dims__(kSolveCtas, 1, 1) __launch_bounds__(SVT) trsv_bwd_kernel(
+static __global__ void __launch_bounds__(SVT) trsv_bwd_kernel(
     const T* __restrict__ L, int ld, int ntiles, const T* __restrict__ Linv, const T* __restrict__ hop,
     const double* __restrict__ yv, double* __restrict__ x, double* __restrict__ sum, int* __restrict__ ticket,
     ulonglong2* __restrict__ pk, const unsigned long long* __restrict__ call, int sub, int* __restrict__ status,

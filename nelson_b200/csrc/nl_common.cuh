@@ -86,21 +86,35 @@ __device__ __forceinline__ void chain_start(P&... p) {
 
 // Launches `kern`, which begins with chain_start(); with pdl as a programmatic
 // dependent of the stream's preceding kernel (0.6 us from one small kernel's end to
-// the next one's start, 1.8 us without).
+// the next one's start, 1.8 us without), in clusters of `cluster` CTAs.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, bool pdl,
-                               Args... args) {
+inline cudaError_t launch_cluster(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, bool pdl,
+                                  int cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (pdl) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster;
+    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+    n++;
+  }
   cfg.attrs = at;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_next(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, bool pdl,
+                               Args... args) {
+  return launch_cluster(kern, grid, block, smem, st, pdl, 1, args...);
 }
 
 // True for all threads of the block of a launch that finishes last (`count`

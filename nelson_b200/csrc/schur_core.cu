@@ -268,8 +268,18 @@ class SchurCoreT final : public SchurCore {
     NL_CUDA(cudaFuncSetAttribute(wvinv_bs_kernel<T, BC, kWvNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)wvinv_smem<T, BC, kWvNT>()));
     NL_CUDA(cudaFuncSetAttribute(hop_mat_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hop_smem<T>()));
-    NL_CUDA(cudaFuncSetAttribute(trsv_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
-    NL_CUDA(cudaFuncSetAttribute(trsv_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem<T>()));
+    NL_CUDA(cudaFuncSetAttribute(trsv_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)trsv_smem<T>(1 + kHopDepth)));
+    NL_CUDA(cudaFuncSetAttribute(trsv_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)trsv_smem<T>(1 + kHopDepth)));
+    {
+      int dev = 0, sms = 0, fwd = 0, bwd = 0;
+      NL_CUDA(cudaGetDevice(&dev));
+      NL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      NL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fwd, trsv_fwd_kernel<T>, SVT, trsv_smem<T>(ntiles_)));
+      NL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bwd, trsv_bwd_kernel<T>, SVT, trsv_smem<T>(ntiles_)));
+      solve_cluster_ = solve_cluster(sms * std::min(fwd, bwd));
+    }
     NL_CUDA(cudaFuncSetAttribute(diag_update_kernel<kChainRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  2 * (int)kDiagUpdSmem));
     if (!ev_[0]) {
@@ -304,15 +314,16 @@ class SchurCoreT final : public SchurCore {
     int* tk = tickets_.as<int>() + 2 * kSolveCtas * (k % solve_slots());
     if (k >= solve_slots()) NL_CUDA(cudaMemsetAsync(tk, 0, 2 * kSolveCtas * sizeof(int), st_));
     const int grid = kSolveCtas * ntiles_;
-    NL_CUDA(launch_next(trsv_fwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl() && !timing, S_.as<T>(), ld_,
-                        ntiles_,
-                        Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), k > 0 ? part_.as<double>() : nullptr,
-                        kSymvChunks, y_.as<double>(), tk, packets(), call(), 2 * k, status, wait_limit, env, active));
-    NL_CUDA(launch_next(trsv_bwd_kernel<T>, dim3(grid), SVT, trsv_smem<T>(), st_, pdl() && !timing, S_.as<T>(), ld_,
-                        ntiles_,
-                        Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
-                        k > 0 ? incU : nullptr, tk + kSolveCtas, packets(), call(), 2 * k + 1, status, wait_limit, env,
-                        active));
+    const size_t smem = trsv_smem<T>(ntiles_);
+    const bool early = pdl() && !timing;
+    NL_CUDA(launch_cluster(trsv_fwd_kernel<T>, dim3(grid), SVT, smem, st_, early, solve_cluster_, S_.as<T>(), ld_,
+                           ntiles_, Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(),
+                           k > 0 ? part_.as<double>() : nullptr, kSymvChunks, y_.as<double>(), tk, packets(), call(),
+                           2 * k, status, wait_limit, env, active));
+    NL_CUDA(launch_cluster(trsv_bwd_kernel<T>, dim3(grid), SVT, smem, st_, early, solve_cluster_, S_.as<T>(), ld_,
+                           ntiles_, Linv_.as<T>(), hop_.as<T>(), y_.as<double>(), k > 0 ? dx_.as<double>() : incU,
+                           k > 0 ? incU : nullptr, tk + kSolveCtas, packets(), call(), 2 * k + 1, status, wait_limit,
+                           env, active));
     launches += 2;
     return NL_OK;
   }
@@ -352,9 +363,10 @@ class SchurCoreT final : public SchurCore {
   nl_status enqueue_solve_withheld(int* status) override {
     if (ntiles_ < 2) return NL_ERR_STATE;
     solve_begin_kernel<<<1, 32, 0, st_>>>(tickets_.as<int>(), tickets(), 1, call());
-    trsv_fwd_kernel<T><<<kSolveCtas*(ntiles_ - 1), SVT, trsv_smem<T>(), st_>>>(
-        S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(), bS_.as<double>(), nullptr, 0, y_.as<double>(),
-        tickets_.as<int>(), packets(), call(), 0, status, wait_limit, nullptr, nullptr);
+    NL_CUDA(launch_cluster(trsv_fwd_kernel<T>, dim3(kSolveCtas * (ntiles_ - 1)), SVT, trsv_smem<T>(ntiles_), st_,
+                           false, solve_cluster_, S_.as<T>(), ld_, ntiles_, Linv_.as<T>(), hop_.as<T>(),
+                           bS_.as<double>(), nullptr, 0, y_.as<double>(), tickets_.as<int>(), packets(), call(), 0,
+                           status, wait_limit, nullptr, nullptr));
     launches += 2;
     NL_CUDA(cudaGetLastError());
     return NL_OK;
@@ -904,6 +916,7 @@ class SchurCoreT final : public SchurCore {
   int nci_ = 0, np_ = 0, nU_ = 0, nV_ = 0, nW_ = 0, nS_ = 0, n_ = 0, ld_ = 0, ntiles_ = 0;
   long long npairs_ = 0;
   int nitems_ = 0, chunk_ = 0, schur_occ_ = 1;  // work items of the Schur formation
+  int solve_cluster_ = kSolveCtas;  // CTAs per cluster of the triangular solves
   bool small_w_ = false;  // at most kPdlBlocks W blocks
   bool need_s0_ = false;
   SchurDev d_{};
