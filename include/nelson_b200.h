@@ -115,7 +115,7 @@ typedef struct {
                           and the start of the next row-tile TRSM (waiting for
                           the auxiliary stream's column updates) */
   float first_ms;      /* main-stream time of the row-tile TRSMs and the
-                          diagonal-tile updates (8-CTA kernels), incl. launch gaps */
+                          diagonal-tile updates (32-CTA kernels), incl. launch gaps */
 } nl_phase_times;
 
 /* ---- problem: device-resident BA section -------------------------------- */

@@ -29,7 +29,9 @@
 // 11.2 ms against 23.2 ms for 512 threads (27.5 ms for 256), of which per
 // increment S 0.65 ms (0.80 before), Y, bS and V^-1 0.14 (0.73), Cholesky 0.28
 // (0.86), solves 0.06 (0.15), back-substitution 0.11 (0.14) and the Jacobian pass
-// 0.22 (0.42).  What bounds it now is the L1 again: the pairs' blocks are 2.3 KB
+// 0.22 (0.42).  Another draw of 128 problems, 6 and 9 parameters: 24.9 -> 10.4 and
+// 52.5 -> 20.1 ms (the 9-parameter kernel spills 1,756 bytes at its 128 registers).
+// What bounds it now is the L1 again: the pairs' blocks are 2.3 KB
 // of gathered lines per 8 pairs.
 // Every sum has a fixed order that does not depend on the CTA size or on which
 // CTA takes the problem (per-thread loops, warp butterflies, 32-element chunk
@@ -1317,8 +1319,8 @@ nl_status nl_batch_lm_solve(nl_batch* b, const nl_lm_settings* st, int threads, 
   NL_CUDA(cudaSetDevice(b->device));
   BSettings s{st->maxNumIt, st->maxNumSubIt, st->minNumIt, 0, st->epsBVector, st->epsIncSquare, st->epsChi2,
               st->tau, st->penaltyV, st->initV, st->maxScaleFactor, st->minScaleFactor};
-  // untuned: 512 threads (128 problems of 8 .. 64 cameras, 6 iterations: 14.4 ms
-  // against 22.4 ms with 256)
+  // untuned: 512 threads (128 problems of 8 .. 64 cameras, 6 iterations: 10.4 ms against
+  // 17.5 ms with 256 and 30.4 with 128; 9 parameters 20.1, 27.9, 47.7)
   const int nt = threads ? threads : (b->tuned_nt ? b->tuned_nt : 512);
   const int cps = ctas_per_sm ? ctas_per_sm : (b->tuned_cps ? b->tuned_cps : 1);
   nl_status r = batch_params(b, true);

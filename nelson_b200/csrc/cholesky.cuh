@@ -52,7 +52,7 @@ constexpr long long kSpinLimit = 1LL << 24;  // default bound of the solves' wai
 // Between two block columns only the last update of the next diagonal block is
 // left on the chain.  Blocks of 16 keep the unrolled code of the roles that run
 // side by side within the instruction cache (blocks of 32 did not: about 3
-// cycles an instruction).  One tile after another on an idle B200: FP32 14.4 us
+// cycles an instruction).  One tile after another on an idle B200: FP32 15.4 us
 // against 30.0 us, FP64 22.6 against 67.5, for 32 rank-4 super-steps that
 // formed the whole inverse as well (forming it here too: 20.5 and 28.7 us).
 constexpr int PB = 16;
@@ -1082,9 +1082,10 @@ static __global__ void __launch_bounds__(128) diag_update64_kernel(double* __res
 // it), so the packets are not cleared between calls.
 //
 // Per solve, one CTA per tile with flags -> now: 15 tiles FP32 33 -> 21.5 us, FP64
-// 42 -> 22 us, band of 47 tiles 92 -> 53 us, 106 tiles 240 -> 200 us (1.3 us per
-// hop, of which 0.7 us are the packet's way through L2; three hop matrices instead
-// of two change nothing).
+// 42 -> 22 us, band of 47 tiles 92 -> 53 us, 106 tiles 240 -> 205 us (1.4 us per
+// hop at 15 and 31 tiles, of which 0.7 us are the packet's way through L2; 1.9 us at 106
+// tiles, where a CTA also streams L's rows; three hop matrices instead of two
+// change nothing).
 constexpr int kSolveCtas = 4, SVR = NB / kSolveCtas, SVT = 128;
 // rank of the CTA among the kSolveCtas consecutive ones of a cluster
 __device__ __forceinline__ int solve_rank() { return (int)(blockIdx.x % kSolveCtas); }

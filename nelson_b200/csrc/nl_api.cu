@@ -491,8 +491,8 @@ nl_status run_solver(nl_problem* h, LmDev& init, nl_solve_report* rep, double* t
   NL_CUDA(cudaMemcpyAsync(h->lm, &init, sizeof(LmDev), cudaMemcpyHostToDevice, h->st));
   // launch loop: (iter, subiter, nsub, done) read one launch behind; where that
   // shows that the latest launch can reach maxNumIt, it is waited for as well,
-  // so that no sub-iteration is enqueued with nothing to do (its launches cost
-  // 38 x 2.2 us on a small scene, the wait 10 us)
+  // so that no sub-iteration is enqueued with nothing to do (twenty launches and those of
+  // the factorisation, each a kernel that returns at once; the wait takes 10 us)
   int(*pin)[4] = reinterpret_cast<int(*)[4]>(h->host_pin + 8);
   int launched = 0, iters = 0;  // sub-iterations enqueued; accepted steps seen
   auto finished = [&](int k, bool* out) {  // sub-iteration k

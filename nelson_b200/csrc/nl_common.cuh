@@ -168,8 +168,9 @@ __host__ __device__ inline int group_item(unsigned block, int nt, int thread, in
   return (int)(block * (unsigned)(nt / lanes)) + thread / lanes;
 }
 
-// CTAs per camera for a pass over a camera's observations with nt threads: four
-// CTAs per SM over the chip, two rounds of work at least for each.
+// CTAs per camera for a pass over a camera's observations with nt threads: enough for
+// four CTAs per SM in all (three of the camera pass are resident, FP64 two; the
+// rest start as those end), two rounds of work at least for each.
 inline int ctas_per_camera(int nc, long long observations, int nt) {
   const long long avg = observations / (nc > 0 ? nc : 1), want = (4 * 148 + nc - 1) / (nc > 0 ? nc : 1);
   const long long n = want < avg / (2 * nt) ? want : avg / (2 * nt);

@@ -372,8 +372,8 @@ class SchurCoreT final : public SchurCore {
     return NL_OK;
   }
 
-  // Rows [r0, r0 + nrows) of panel k.  One row per thread while that leaves
-  // SMs idle, else two: the staging of L_kk is then shared by twice the rows.
+  // Rows [r0, r0 + nrows) of panel k.  CTAs of 16 rows while they leave SMs idle, else
+  // of 32: L_kk is then staged once for twice the rows.
   void launch_trsm(int k, int r0, int nrows, uint8_t* pack, const int* active, cudaStream_t st) {
     if (nrows <= 16 * 148)
       trsm_kernel<T, 1><<<cdiv(nrows, 16), 256, trsm_smem<T, 1>(), st>>>(S_.as<T>(), ld_, k, r0, nrows, Linv_.as<T>(),

@@ -103,7 +103,7 @@ static __global__ void vinv_kernel(SchurDev d, const T* __restrict__ V, T* __res
 // consecutive: they pass through shared memory so that every access to W and Y is
 // to whole lines (a lane reading its own 112 bytes takes 32 lines per access).
 // Bound by the L1 lines of the Vinv / bV gather.  375k blocks of 9x3 FP32 33 -> 24
-// us, FP64 65 -> 50 us, 1,500 cameras 338 -> 179 us; several CTAs per camera were
+// us, FP64 67 -> 55 us, 1,500 cameras 338 -> 184 us; several CTAs per camera were
 // slower (28 us: the sums wait for the stores).
 template <typename T, int BC, int NT>
 constexpr size_t wvinv_smem() {
