@@ -468,12 +468,13 @@ template <typename T>
 inline int backsub_lanes(int np, size_t w_bytes) {
   return np >= (1 << 16) && w_bytes <= ((size_t)256 << 20) ? 1 : kBackLanes<T>;
 }
+// Sixteen lanes keep to 32 registers, every warp of an SM resident: 200 cameras FP64 35 us
+// against 41 with 36 registers.
 template <typename T, int BC, int LANES>
-static __global__ void __launch_bounds__(128) backsub_kernel(SchurDev d, const T* __restrict__ W,
-                                                             const T* __restrict__ Vinv, const T* __restrict__ bV,
-                                                             double* xU, int nxu, double* __restrict__ xV,
-                                                             const int* __restrict__ ok_flag, int* __restrict__ dirty,
-                                                             const int* __restrict__ active) {
+static __global__ void __launch_bounds__(128, LANES == 16 ? 16 : 0)
+    backsub_kernel(SchurDev d, const T* __restrict__ W, const T* __restrict__ Vinv, const T* __restrict__ bV,
+                   double* xU, int nxu, double* __restrict__ xV, const int* __restrict__ ok_flag,
+                   int* __restrict__ dirty, const int* __restrict__ active) {
   constexpr int LW = Layout<T, BC>::W;
   constexpr int LV = Layout<T, BC>::V;
   using V16 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
