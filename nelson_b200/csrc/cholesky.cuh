@@ -36,7 +36,8 @@ constexpr long long kSpinLimit = 1LL << 24;  // default bound of the solves' wai
 // around that chain, in eight block columns of 16:
 //   pivot warp    the diagonal block, a lane holding one row of 16 columns in
 //       registers (lanes 16 .. 31 repeat lanes 0 .. 15).  With u = the unscaled
-//       column, d its pivot and r = 1 / d, an entry becomes a_c -= (a_j r) u_c.
+//       column, d its pivot and r = 1 / d, an entry becomes a_c -= (a_j r) u_c
+//       (u and d times kPivScale, r over it).
 //       Every lane carries the next pivot itself (d' = v - u1 (u1 r), u1 and v
 //       fetched by shuffle while r is formed), so a column costs one reciprocal
 //       and a few FMAs of latency; the columns further right are updated one
@@ -150,16 +151,23 @@ __device__ inline void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// 1 / d and 1 / sqrt(d) of a pivot, clamped away from zero (a non-positive
-// pivot is flagged separately).  Above 2^126 the reciprocal is subnormal and must not be
-// flushed to zero: the elimination would leave the column out.
-__device__ __forceinline__ void pivot_inv(float d, float& ri, float& rs) {
-  d = fmaxf(d, 1e-30f);
-  asm("rcp.approx.f32 %0, %1;" : "=f"(ri) : "f"(d));
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(d));
+// A pivot d is carried as kPivScale d, and the published columns have the same
+// factor.  FP32 takes a quarter: its reciprocal 4 / d is then a normal number up to the end
+// of the range, where that of d is subnormal above 2^126 and the flushing rcp.approx
+// would leave the column out of the elimination (the one that does not flush costs
+// 0.6 us a tile in the chain).  A power of two changes no other bit.
+template <typename T>
+constexpr T kPivScale = sizeof(T) == 4 ? (T)0.25 : (T)1;
+// 1 / dq and 1 / sqrt(d) of a pivot, dq = kPivScale d, clamped away from zero (a
+// non-positive pivot is flagged separately)
+__device__ __forceinline__ void pivot_inv(float dq, float& ri, float& rs) {
+  dq = fmaxf(dq, 0.25e-30f);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(dq));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(dq));
+  rs *= 0.5f;
 }
-__device__ __forceinline__ void pivot_inv(double d, double& ri, double& rs) {
-  rs = rsqrt(fmax(d, 1e-300));
+__device__ __forceinline__ void pivot_inv(double dq, double& ri, double& rs) {
+  rs = rsqrt(fmax(dq, 1e-300));
   ri = rs * rs;
 }
 
@@ -172,26 +180,28 @@ __device__ __forceinline__ void named_arrive(int id, int n) {
 
 // Eliminates the 16 x 16 block whose row lane % 16 is a[] (entries right of the
 // diagonal are ignored), leaving the row of L in a[] and publishing every
-// column in uc, (1 / d, 1 / sqrt(d)) in inv_s.  False on a non-positive pivot.
+// column (times kPivScale) in uc, (1 / (kPivScale d), 1 / sqrt(d)) in inv_s.  False
+// on a non-positive pivot.
 // kPaced: named barriers pace the row warps of the same CTA behind it.
 template <typename T, bool kPaced = true>
 __device__ __forceinline__ bool pivot_block(T (&a)[PB], Sh<T> uc, Sh<T> inv_s, int lane) {
   bool ok = true;
-  T d = __shfl_sync(0xffffffffu, a[0], 0);
+  constexpr T kQ = kPivScale<T>;
+  T dq = kQ * __shfl_sync(0xffffffffu, a[0], 0);
   T up[PB];
   T tp = (T)0;
 #pragma unroll
   for (int j = 0; j < PB; j++) {
     T ri, rs;
-    pivot_inv(d, ri, rs);
+    pivot_inv(dq, ri, rs);
     T u1 = (T)0, u2 = (T)0, v = (T)0;
     if (j + 1 < PB) {
-      u1 = __shfl_sync(0xffffffffu, a[j], j + 1);
-      v = __shfl_sync(0xffffffffu, a[j + 1], j + 1);
+      u1 = kQ * __shfl_sync(0xffffffffu, a[j], j + 1);
+      v = kQ * __shfl_sync(0xffffffffu, a[j + 1], j + 1);
     }
-    if (j + 2 < PB) u2 = __shfl_sync(0xffffffffu, a[j], j + 2);
-    if (lane < PB) store_one(uc + (j * PB + lane), a[j]);
-    ok &= d > (T)0 && isfinite(d);
+    if (j + 2 < PB) u2 = kQ * __shfl_sync(0xffffffffu, a[j], j + 2);
+    if (lane < PB) store_one(uc + (j * PB + lane), kQ * a[j]);
+    ok &= dq > (T)0 && isfinite(dq);
     // column j - 1 applied to the columns that its step left out
     if (j > 0) {
 #pragma unroll
@@ -208,7 +218,7 @@ __device__ __forceinline__ bool pivot_block(T (&a)[PB], Sh<T> uc, Sh<T> inv_s, i
     }
     const T t = a[j] * ri;
     if (j + 1 < PB) {
-      d = v - u1 * (u1 * ri);
+      dq = v - u1 * (u1 * ri);
       a[j + 1] -= t * u1;
     }
     if (j + 2 < PB) a[j + 2] -= t * u2;
@@ -384,7 +394,7 @@ static __global__ void __launch_bounds__(PT, 1) potrf_diag_kernel(T* __restrict_
   const Sh<T> sm{(uint32_t)__cvta_generic_to_shared(smf4)};  // L on and below the diagonal 16-blocks
   const Sh<T> dg = sm + NB * kPotLd;     // inverses of the diagonal blocks, transposed
   const Sh<T> uc = dg + NB * kPotDld;    // published columns of the pivot block
-  const Sh<T> inv_s = uc + PB * PB;    // (1 / d, 1 / sqrt(d)) per column
+  const Sh<T> inv_s = uc + PB * PB;    // (1 / (kPivScale d), 1 / sqrt(d)) per column
   chain_release();
   chain_wait();
   if (active && !*active) return;
