@@ -459,15 +459,16 @@ static __global__ void clear_kernel(T* __restrict__ S, T* __restrict__ S0, int n
 // W is not far larger than L2, a thread each is the faster one (backsub_lanes).
 // us, thread / lanes (9x3 blocks, W in MB): FP32 30k points, 23 MB 21 / 15; 50k, 42 MB
 // 30 / 22; 100k, 34 MB 17 / 22; 150k, 59 MB 27 / 38; 150k, 117 MB 50 / 62; 270k, 212 MB
-// 89 / 99; 500k, 392 MB 311 / 177.  FP64 50k, 84 MB 47 / 41; 100k, 67 MB 26 / 41; 150k,
-// 235 MB 76 / 100; 270k, 424 MB 293 / 168.
+// 89 / 99; 500k, 392 MB 311 / 177.  FP64 50k, 84 MB 47 / 35; 75k, 117 MB 54 / 47; 100k,
+// 67 MB 26 / 35; 150k, 117 MB 40 / 53; 150k, 235 MB 76 / 84; 270k, 424 MB 293 / 137.
 template <typename T>
 constexpr int kBackLanes = sizeof(T) == 4 ? 8 : 16;
-// Lanes for np points and w_bytes of W.  75,000 points are even (FP32 34 / 33 us, FP64
-// 54 / 56); between 235 and 392 MB of W the lanes begin to win.
+// Lanes for np points and w_bytes of W.  FP32 is even at 75,000 points of 7 observations
+// (34 / 33 us) and sooner with fewer, FP64 at about 100,000; between 235 and 392 MB of W
+// the lanes begin to win.
 template <typename T>
 inline int backsub_lanes(int np, size_t w_bytes) {
-  return np >= (1 << 16) && w_bytes <= ((size_t)256 << 20) ? 1 : kBackLanes<T>;
+  return np >= (sizeof(T) == 4 ? 1 << 16 : 3 << 15) && w_bytes <= ((size_t)256 << 20) ? 1 : kBackLanes<T>;
 }
 // Sixteen lanes keep to 32 registers, every warp of an SM resident: 200 cameras FP64 35 us
 // against 41 with 36 registers.

@@ -1,6 +1,6 @@
-"""Back-substitution on both sides of its rule (a thread per point from 65,536 points on, up to
-256 MB of W blocks: the last size has 269 MB in FP64): dV = V^-1 (-bV - W' dU) of the returned dU in numpy, on a
-caller-assembled system.
+"""Back-substitution on both sides of its rule (a thread per point from 65,536 points on,
+FP64 98,304, up to 256 MB of W blocks: the last size has 269 MB in FP64):
+dV = V^-1 (-bV - W' dU) of the returned dU in numpy, on a caller-assembled system.
 
 Tolerance per value: the FP32 path rounds V^-1 once (formed and applied in FP64), so
 2^-24 of sum |V^-1| |t| with t = -bV - W' dU, doubled; FP64: the condition of V (below
@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("prec", [N.PREC_FP64, N.PREC_MIXED])
-@pytest.mark.parametrize("bu,nv,k", [(2, 65537, 2), (3, 65535, 3), (6, 65536, 2), (9, 65535, 2), (9, 65536, 3), (9, 150000, 8)])
+@pytest.mark.parametrize("bu,nv,k", [(2, 65537, 2), (3, 65535, 3), (6, 65536, 2), (9, 65535, 2), (9, 65536, 3), (3, 98303, 2), (9, 98304, 2),
+                                     (9, 150000, 8)])
 def test_points(bu, nv, k, prec):
     r = np.random.default_rng(bu * nv + k)
     nu = 12
