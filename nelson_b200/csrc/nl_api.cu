@@ -90,7 +90,7 @@ struct nl_problem {
   int have_jac = 0;
 
   ~nl_problem() {
-    if (sub_exec) cudaGraphExecDestroy(sub_exec);
+    drop_capture();
     if (cublas) cublasDestroy(cublas);
     if (host_pin) cudaFreeHost(host_pin);
     if (ev_a) cudaEventDestroy(ev_a);
