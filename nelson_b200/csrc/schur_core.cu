@@ -15,9 +15,9 @@ constexpr int kNT = 256, kWvNT = 256;
 // that the running one has less L1 for.  With many W blocks that costs the passes more
 // than is saved: the saving is 6 % at 105k blocks (2,605 / 2,457), 2 % at 375k (5,475 /
 // 5,361), and at 1.05 M they lose 6 % (9,118 / 9,681, mixed 7,236 / 7,647); the line is on
-// the safe side.  The refinement residual of many dense tiles loses as well: 31 tiles 6,720 / 6,517, 57 tiles 13,177 /
-// 13,226, 106 tiles 33,542 / 33,864; within an envelope it does not (pose graphs of 47
-// tiles 6,850 / 6,809, of 141 tiles 19,740 / 19,508).
+// the safe side.  The refinement residual of many dense tiles loses as well: 31 tiles
+// 6,720 / 6,517, 57 tiles 13,177 / 13,226, 106 tiles 33,542 / 33,864; within an envelope
+// it does not (pose graphs of 47 tiles 6,850 / 6,809, of 141 tiles 19,740 / 19,508).
 constexpr int kPdlBlocks = 1 << 16, kPdlTiles = 48;
 constexpr int kRedCTAs = 296;  // 2 x 148 SMs for grid-stride reductions
 constexpr int kSymvChunks = 8;
